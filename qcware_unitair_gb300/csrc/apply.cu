@@ -1762,6 +1762,9 @@ extern "C" int gbsv_apply_all_qubits(const void* state_in, void* state_out,
     return set_error(GBSV_ERR_INVALID_ARG, "negative operator qubit stride");
   if (num_states == 0) return GBSV_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == GBSV_C64 && num_qubits >= 4)
+    return apply_all_fused(state_in, state_out, num_qubits, num_states,
+                           in_stride, ops, op_stride, op_qubit_stride, st);
   const int amp = dtype_bytes(dtype);
   const int64_t N = int64_t(1) << num_qubits;
   for (int q = 0; q < num_qubits; ++q) {

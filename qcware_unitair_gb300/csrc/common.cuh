@@ -164,6 +164,10 @@ int after_launch(const char* what);
 int set_error(int status, const char* fmt, ...);
 // GBSV_C128_PAIRS or GBSV_C128_FP64 (gbsv_set_c128_arith)
 int c128_arith();
+// apply_all_qubits for complex64 states of n >= 4 qubits (allq.cu)
+int apply_all_fused(const void* in, void* out, int n, int64_t num_states,
+                    int64_t in_stride, const void* ops, int64_t op_stride,
+                    int64_t op_qstride, cudaStream_t st);
 inline int dtype_bytes(int dtype) {
   switch (dtype) {
     case GBSV_C64: return 8;
