@@ -123,6 +123,43 @@ int gbsv_apply_all_qubits(const void* state_in, void* state_out, int dtype,
                           int64_t op_stride, int64_t op_qubit_stride,
                           void* stream);
 
+/* Passes over the state that gbsv_apply_all_qubits makes for complex64
+ * states of num_qubits >= 9; 0 for what the two functions below do not
+ * take (complex128, fewer qubits). */
+int gbsv_all_qubits_passes(int dtype, int num_qubits);
+
+/* gbsv_apply_all_qubits with the state after each pass kept: pass i reads
+ * state_in (i = 0) or pass_out[i - 1] and writes pass_out[i] (a HOST array
+ * of gbsv_all_qubits_passes device pointers, the last the result). */
+int gbsv_apply_all_qubits_passes(const void* state_in, void* const* pass_out,
+                                 int dtype, int num_qubits,
+                                 int64_t num_states, int64_t in_stride,
+                                 const void* ops, int64_t op_stride,
+                                 int64_t op_qubit_stride, void* stream);
+
+/* Scratch bytes gbsv_apply_all_qubits_grad needs. */
+size_t gbsv_all_qubits_grad_scratch_bytes(int64_t num_states, int num_qubits,
+                                          int shared, int each);
+
+/* Gradients of gbsv_apply_all_qubits (torch's convention, as
+ * gbsv_operator_grad): from grad_out and the states that entered each pass
+ * (pass_in, a HOST array; pass_in[0] with in_stride), dL/d(state) into
+ * grad_state (num_states dense states; may be NULL when need_state == 0 and
+ * there is one pass; it is overwritten as scratch when there are more) and
+ * dL/d(operators) into grad_ops: with op_qubit_stride != 0 one 2x2 per
+ * qubit, (num_states or, with shared != 0, 1) x num_qubits x 2 x 2, else
+ * summed over the qubits, (num_states or 1) x 2 x 2.  Deterministic.  The
+ * autograd backward that unitair gets from torch through its loop of einsums
+ * (src/unitair/simulation/operations.py:332-413). */
+int gbsv_apply_all_qubits_grad(const void* grad_out,
+                               const void* const* pass_in, int dtype,
+                               int num_qubits, int64_t num_states,
+                               int64_t in_stride, const void* ops,
+                               int64_t op_stride, int64_t op_qubit_stride,
+                               void* grad_state, int need_state,
+                               void* grad_ops, int shared, void* scratch,
+                               size_t scratch_bytes, void* stream);
+
 /* out = exp(-i * angles) * state with broadcasting.  Replaces
  * unitair.simulation.apply_phase (operations.py:15-42).  bc describes the
  * output shape; operand a is the real angle tensor (angle_dtype GBSV_F32 or

@@ -88,6 +88,13 @@ SIGNATURES = {
                                  ctypes.POINTER(_I32), _I, _P]),
     "gbsv_apply_all_qubits": (_I, [_P, _P, _I, _I, _I64, _I64, _P, _I64,
                                    _I64, _P]),
+    "gbsv_all_qubits_passes": (_I, [_I, _I]),
+    "gbsv_apply_all_qubits_passes": (_I, [_P, ctypes.POINTER(_P), _I, _I,
+                                          _I64, _I64, _P, _I64, _I64, _P]),
+    "gbsv_all_qubits_grad_scratch_bytes": (_SZ, [_I64, _I, _I, _I]),
+    "gbsv_apply_all_qubits_grad": (_I, [_P, ctypes.POINTER(_P), _I, _I, _I64,
+                                        _I64, _P, _I64, _I64, _P, _I, _P, _I,
+                                        _P, _SZ, _P]),
     "gbsv_apply_phase": (_I, [_P, _I, _P, _I, _P, _I, _BC, _P]),
     "gbsv_fused_max_tile_qubits": (_I, [_I]),
     "gbsv_run_stage": (_I, [_P, _P, _I, _I, _I64, _I64, _I, _I,
@@ -199,3 +206,7 @@ def complex128_arithmetic() -> str:
 def qubit_array(qubits):
     arr = (_I32 * max(len(qubits), 1))(*[int(q) for q in qubits])
     return arr
+
+
+def pointer_array(tensors):
+    return (_P * len(tensors))(*[t.data_ptr() for t in tensors])

@@ -7,6 +7,7 @@
 // write of the state: a pass takes a tile of 2^12 amplitudes, applies the
 // operators of up to 12 of its index bits, and writes it back.
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 
@@ -349,4 +350,530 @@ int apply_all_fused(const void* in, void* out, int n, int64_t num_states,
   return GBSV_OK;
 }
 
+
+// ------------------------------------------------------------- gradient --
+// Gradient of a pass: for out = (prod_q U_q) psi and g = dL/d(out),
+//   dL/dU_q[a, c] = sum_rest g_q[rest | a] * conj(psi_q[rest | c])
+// where, because the U commute, psi_q may be psi with any of the other
+// operators applied as long as g_q has the adjoints of the rest.  A CTA
+// runs the layouts upwards on psi, keeping psi before each in shared
+// memory, and downwards on g; inside a layout it takes the bits from the
+// top, with the lower bits' operators applied to a fresh copy of psi and
+// the upper bits' adjoints already applied to g.  One read of psi and g and
+// one write of dL/dpsi per pass, where a loop over the qubits would save or
+// recompute a state per qubit.
+//
+// Sums: a thread's products enter a float pair exactly (Acc<float>), pairs
+// meet across a warp with TwoSum and everything beyond a warp is FP64, in a
+// fixed order.  That accumulation bounds the kernel (about 10 FP32
+// operations per real product, 16 products per pair and operator).
+//
+// One autograd node and three or four launches take the place of a node,
+// an adjoint gate, a gradient kernel, its sum and an accumulation per
+// qubit: a QAOA step (16 states of 14 qubits, 3 layers, forward and
+// backward) went from 9.3 to 3.2 ms, most of it host time before and after.
+struct AllqGradArgs {
+  AllqArgs f;
+  int chunk_log;   // log2 tiles of one state that a CTA walks (12 tile bits)
+  int store;       // write dL/dpsi
+  double* partial; // [state][qubit][chunk][8]: re, im of the four entries
+};
+
+__device__ __forceinline__ AqOp aq_dagger(const AqOp& o) {
+  AqOp d;
+  d.m[0] = make_float2(o.m[0].x, -o.m[0].y);
+  d.m[1] = make_float2(o.m[2].x, -o.m[2].y);
+  d.m[2] = make_float2(o.m[1].x, -o.m[1].y);
+  d.m[3] = make_float2(o.m[3].x, -o.m[3].y);
+  d.kind = o.kind;
+  return d;
+}
+
+__device__ __forceinline__ void aq_pair_add(float& hi, float& lo, float oh,
+                                            float ol) {
+  const float s = hi + oh;
+  const float bp = s - hi;
+  lo += ol + ((hi - (s - bp)) + (oh - bp));
+  hi = s;
+}
+
+// Sums eight pairs over the warp by halving: after three exchanges a lane
+// keeps one value, two more finish it.  Lane 4 k holds value k's bits in
+// reverse order of the exchanges; *v is the value this lane ends with.
+__device__ __forceinline__ float2 aq_warp_sum8(Acc<float>* acc, int* v) {
+  const int lane = threadIdx.x & 31;
+  float h[8], l[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    h[j] = acc[j].hi;
+    l[j] = acc[j].lo;
+  }
+#pragma unroll
+  for (int w = 4, o = 16; w > 0; w >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (j >= w) continue;
+      const float sh = up ? h[j] : h[j + w], sl = up ? l[j] : l[j + w];
+      h[j] = up ? h[j + w] : h[j];
+      l[j] = up ? l[j + w] : l[j];
+      aq_pair_add(h[j], l[j], __shfl_xor_sync(0xffffffffu, sh, o),
+                  __shfl_xor_sync(0xffffffffu, sl, o));
+    }
+  }
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1)
+    aq_pair_add(h[0], l[0], __shfl_xor_sync(0xffffffffu, h[0], o),
+                __shfl_xor_sync(0xffffffffu, l[0], o));
+  *v = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+  return make_float2(h[0], l[0]);
+}
+
+// g0 conj(x0), g0 conj(x1), g1 conj(x0), g1 conj(x1) over the pairs of
+// register bit B
+template <int B>
+__device__ __forceinline__ void aq_outer(const float2* g, const float2* x,
+                                         Acc<float>* acc) {
+  constexpr int H = 1 << B;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    if (i & H) continue;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 u = g[i | (e & 2 ? H : 0)], v = x[i | (e & 1 ? H : 0)];
+      acc[2 * e].add_prod(u.x, v.x);
+      acc[2 * e].add_prod(u.y, v.y);
+      acc[2 * e + 1].add_prod(u.y, v.x);
+      acc[2 * e + 1].add_prod(-u.x, v.y);
+    }
+  }
+}
+
+// One layout of the gradient: registers RB .. RB + 3, tile bits LO .. HI,
+// psi before the layout in S (this thread's slots are its own).
+template <int RB, int LO, int HI>
+__device__ __forceinline__ void aq_grad_round(float2* g, const float2* S,
+                                              int u, const float2* ops,
+                                              const AllqArgs& a,
+                                              float2* wred) {
+#pragma unroll 1
+  for (int b = HI; b >= LO; --b) {
+    if (!((a.mask >> b) & 1)) continue;
+    float2 x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = S[aq_swz(aq_index<RB>(u, i))];
+    const bool xfin = aq_finite(x);
+#pragma unroll
+    for (int c = LO; c < HI; ++c) {
+      if (c >= b || !((a.mask >> c) & 1)) continue;
+      const AqOp o = aq_load_op(ops, a, c);
+      const int kind = xfin ? o.kind : AQ_FULL;
+      if (c - RB == 0) aq_apply<0>(x, o, kind);
+      else if (c - RB == 1) aq_apply<1>(x, o, kind);
+      else aq_apply<2>(x, o, kind);
+    }
+    const AqOp d = aq_dagger(aq_load_op(ops, a, b));
+    const int kind = aq_finite(g) ? d.kind : AQ_FULL;
+    Acc<float> acc[8];
+    switch (b - RB) {
+      case 0: aq_outer<0>(g, x, acc); aq_apply<0>(g, d, kind); break;
+      case 1: aq_outer<1>(g, x, acc); aq_apply<1>(g, d, kind); break;
+      case 2: aq_outer<2>(g, x, acc); aq_apply<2>(g, d, kind); break;
+      default: aq_outer<3>(g, x, acc); aq_apply<3>(g, d, kind); break;
+    }
+    int v;
+    const float2 sum = aq_warp_sum8(acc, &v);
+    if ((threadIdx.x & 3) == 0)
+      wred[(b * (AQ_THREADS / 32) + (threadIdx.x >> 5)) * 8 + v] = sum;
+  }
+}
+
+constexpr size_t AQ_GRAD_SMEM =
+    (3 * (size_t(1) << AQ_TILE) + AQ_TILE * (AQ_THREADS / 32) * 8) *
+    sizeof(float2);
+
+// M = min(n, 12) >= 9, so that a warp's amplitudes belong to one state.
+template <int M>
+__global__ void __launch_bounds__(AQ_THREADS, 2)
+    allq_grad_kernel(const float2* psi, const float2* gin, float2* gout,
+                     const float2* ops, AllqGradArgs ga) {
+  using W = AqRounds<M>;
+  const AllqArgs& a = ga.f;
+  constexpr int R0 = W::R0, R1 = W::R1;
+  extern __shared__ __align__(16) float2 aq_sm[];
+  float2* const wred = aq_sm + 3 * (1 << AQ_TILE);
+  const int sub = threadIdx.x >> (M - 4);
+  const int u = threadIdx.x & ((1 << (M - 4)) - 1);
+  float2* const SA = aq_sm + (sub << M);
+  float2* const SB = SA + (1 << AQ_TILE);
+  float2* const SC = SB + (1 << AQ_TILE);
+  const bool act1 = aq_any<R1, R0 - 1>(a.mask);
+  bool act2 = false;
+  if constexpr (M > 8) act2 = R1 > 0 && aq_any<0, (R1 > 0 ? R1 - 1 : 0)>(a.mask);
+
+#define AQ_PUT(S, r, A)                                              \
+  _Pragma("unroll") for (int i = 0; i < 16; ++i)                     \
+      S[aq_swz(aq_index<A>(u, i))] = r[i];                           \
+  __syncthreads();
+#define AQ_GET(S, r, B)                                              \
+  _Pragma("unroll") for (int i = 0; i < 16; ++i) r[i] =              \
+      S[aq_swz(aq_index<B>(u, i))];
+
+  const int walk = M == AQ_TILE ? 1 << ga.chunk_log : 1;
+  double total = 0.0;  // M = 12: value threadIdx.x & 7 of bit threadIdx.x / 8
+  uint64_t s = 0;
+  for (int w = 0; w < walk; ++w) {
+    uint64_t base;
+    s = aq_place<M>(a, (uint64_t)blockIdx.x * walk + w, sub, &base);
+    const bool live = M == AQ_TILE || s < (uint64_t)a.num_states;
+    const float2* const xs = psi + (int64_t)s * a.in_stride + base;
+    const float2* const gs = gin + (s << a.n) + base;
+    const float2* const so = ops + (live ? (int64_t)s * a.op_stride : 0);
+    {
+      float2 r[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        r[i] = make_float2(0.f, 0.f);
+        if (live) r[i] = __ldcs(xs + aq_offset(a, aq_index<R0>(u, i)));
+      }
+      float2* const first = act2 ? SA : act1 ? SB : SC;
+      AQ_PUT(first, r, R0)
+      if (act2) {
+        if constexpr (W::R2 >= 0) {
+          AQ_GET(SA, r, 0)
+          aq_round<0, 0, (R1 > 0 ? R1 - 1 : 0)>(r, so, a);
+          float2* const to = act1 ? SB : SC;
+          AQ_PUT(to, r, 0)
+        }
+      }
+      if (act1) {
+        AQ_GET(SB, r, R1)
+        aq_round<R1, R1, R0 - 1>(r, so, a);
+        AQ_PUT(SC, r, R1)
+      }
+    }
+    float2 g[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      g[i] = make_float2(0.f, 0.f);
+      if (live) g[i] = __ldcs(gs + aq_offset(a, aq_index<R0>(u, i)));
+    }
+    aq_grad_round<R0, R0, M - 1>(g, SC, u, so, a, wred);
+    int at = 0;
+    if (act1) {
+      AQ_PUT(SC, g, R0)
+      AQ_GET(SC, g, R1)
+      aq_grad_round<R1, R1, R0 - 1>(g, SB, u, so, a, wred);
+      at = 1;
+    }
+    if (act2) {
+      if constexpr (W::R2 >= 0) {
+        if (act1) {
+          AQ_PUT(SB, g, R1)
+          AQ_GET(SB, g, 0)
+        } else {
+          AQ_PUT(SC, g, R0)
+          AQ_GET(SC, g, 0)
+        }
+        aq_grad_round<0, 0, (R1 > 0 ? R1 - 1 : 0)>(g, SA, u, so, a, wred);
+        at = 2;
+      }
+    }
+    if (ga.store) {
+      float2* const dst = gout + (s << a.n) + base;
+      if (at == 2) {
+        AQ_PUT(SA, g, 0)
+        AQ_GET(SA, g, R0)
+      } else if (at == 1) {
+        AQ_PUT(SB, g, R1)
+        AQ_GET(SB, g, R0)
+      }
+      if (live) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          __stcs(dst + aq_offset(a, aq_index<R0>(u, i)), g[i]);
+      }
+    }
+    __syncthreads();  // wred complete, and the slots free for the next tile
+    if constexpr (M == AQ_TILE) {
+      const int b = threadIdx.x >> 3, v = threadIdx.x & 7;
+      if (b < M && ((a.mask >> b) & 1))
+        for (int k = 0; k < AQ_THREADS / 32; ++k) {
+          const float2 p = wred[(b * (AQ_THREADS / 32) + k) * 8 + v];
+          total += (double)p.x + (double)p.y;
+        }
+      if (w + 1 < walk) __syncthreads();
+    }
+  }
+#undef AQ_PUT
+#undef AQ_GET
+  if constexpr (M == AQ_TILE) {
+    const int b = threadIdx.x >> 3, v = threadIdx.x & 7;
+    if (b < M && ((a.mask >> b) & 1)) {
+      const int pos = b < a.cl ? b : a.p + (b - a.cl);
+      const int nch = a.n - AQ_TILE - ga.chunk_log;  // log2 chunks
+      const uint64_t ch = blockIdx.x & ((uint64_t(1) << nch) - 1);
+      ga.partial[((((s * a.n + (a.n - 1 - pos)) << nch) + ch) << 3) + v] =
+          total;
+    }
+  } else {
+    constexpr int SUBS = 1 << (AQ_TILE - M), WPS = (AQ_THREADS / 32) / SUBS;
+    for (int i = threadIdx.x; i < SUBS * M * 8; i += AQ_THREADS) {
+      const int v = i & 7, b = (i >> 3) % M, k = (i >> 3) / M;
+      const uint64_t st = ((uint64_t)blockIdx.x << (AQ_TILE - M)) + k;
+      if (st >= (uint64_t)a.num_states) continue;
+      double t = 0.0;
+      for (int w = 0; w < WPS; ++w) {
+        const float2 p = wred[(b * (AQ_THREADS / 32) + k * WPS + w) * 8 + v];
+        t += (double)p.x + (double)p.y;
+      }
+      ga.partial[((st * a.n + (a.n - 1 - b)) << 3) + v] = t;
+    }
+  }
+}
+
+// Sums runs of `len` items of eight doubles, starting at run * len: block
+// (run, part) sums items part, part + parts, ... ; with out != null (parts
+// == 1) the four complex sums go to out[4 run ..], else to next[run * parts
+// + part].
+__global__ void __launch_bounds__(AQ_THREADS)
+    allq_grad_sum_kernel(const double* items, uint64_t len, int parts,
+                         double* next, float2* out) {
+  const uint64_t run = blockIdx.x / parts;
+  const int part = blockIdx.x % parts;
+  const int v = threadIdx.x & 7, lane = threadIdx.x >> 3;
+  double t = 0.0;
+  for (uint64_t i = part + (uint64_t)lane * parts; i < len;
+       i += (uint64_t)parts * (AQ_THREADS / 8))
+    t += items[((run * len + i) << 3) + v];
+  __shared__ double red[AQ_THREADS];
+  red[threadIdx.x] = t;
+  __syncthreads();
+  if (lane) return;
+  t = 0.0;
+  for (int k = 0; k < AQ_THREADS / 8; ++k) t += red[8 * k + v];
+  if (out)
+    reinterpret_cast<float*>(out)[(run << 3) + v] = (float)t;
+  else
+    next[((run * parts + part) << 3) + v] = t;
+}
+
+struct AqGradPlan {
+  int chunk_log;      // tiles a CTA walks
+  uint64_t items;     // [state][qubit][chunk] partials of eight doubles
+  uint64_t runs, len; // gradients and the items of each
+  int parts;          // second-level partials per gradient (1: none)
+};
+
+// Gradients are per (state, qubit), (state), (qubit) or one; items of one
+// gradient are contiguous except for (qubit) summed over the states, where
+// each state is a run of its own first (see the caller).
+static AqGradPlan aq_grad_plan(int64_t num_states, int n, bool shared,
+                               bool each) {
+  AqGradPlan p{};
+  const int lt = n > AQ_TILE ? n - AQ_TILE : 0;
+  // at most 512 partials per state and qubit
+  p.chunk_log = lt > 9 ? lt - 9 : 0;
+  const uint64_t chunks = uint64_t(1) << (lt - p.chunk_log);
+  p.items = (uint64_t)num_states * n * chunks;
+  if (shared && !each) {
+    p.runs = 1;
+    p.len = p.items;
+  } else if (!shared && !each) {
+    p.runs = (uint64_t)num_states;
+    p.len = n * chunks;
+  } else {
+    p.runs = (uint64_t)num_states * n;
+    p.len = chunks;
+  }
+  const uint64_t parts = (p.len + 4095) / 4096;
+  p.parts = (int)std::min<uint64_t>(parts, 256);
+  return p;
+}
+
+// Sums over states of [state][qubit] gradients: one thread per value.
+__global__ void allq_grad_states_kernel(const double* items,
+                                        uint64_t num_states, int values,
+                                        float* out) {
+  const int v = blockIdx.x;
+  double t = 0.0;
+  for (uint64_t s = threadIdx.x; s < num_states; s += blockDim.x)
+    t += items[s * values + v];
+  __shared__ double red[AQ_THREADS];
+  red[threadIdx.x] = t;
+  __syncthreads();
+  for (int o = AQ_THREADS / 2; o > 0; o >>= 1) {
+    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[v] = (float)red[0];
+}
+
+static size_t aq_grad_scratch(const AqGradPlan& p, int64_t num_states, int n,
+                              bool shared, bool each) {
+  uint64_t items = p.items;
+  if (p.parts > 1) items += p.runs * p.parts;
+  if (shared && each) items += (uint64_t)num_states * n;
+  return items * 8 * sizeof(double);
+}
+
+template <int M>
+static int aq_grad_launch(const float2* psi, const float2* gin, float2* gout,
+                          const float2* ops, const AllqGradArgs& ga,
+                          uint64_t ctas, cudaStream_t st) {
+  // the shared-memory opt-in, once per device (a race only repeats it)
+  static std::atomic<uint64_t> attr_set;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const uint64_t bit = uint64_t(1) << (dev & 63);
+  if (!(attr_set.load(std::memory_order_relaxed) & bit)) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        allq_grad_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (int)AQ_GRAD_SMEM);
+    if (e != cudaSuccess)
+      return set_error(GBSV_ERR_CUDA, "allq_grad_kernel: %s",
+                       cudaGetErrorString(e));
+    attr_set.fetch_or(bit, std::memory_order_relaxed);
+  }
+  allq_grad_kernel<M><<<(unsigned)ctas, AQ_THREADS, AQ_GRAD_SMEM, st>>>(
+      psi, gin, gout, ops, ga);
+  return after_launch("allq_grad_kernel");
+}
+
 }  // namespace gbsv
+
+using namespace gbsv;
+
+extern "C" int gbsv_all_qubits_passes(int dtype, int num_qubits) {
+  return dtype == GBSV_C64 && num_qubits >= 9 && num_qubits <= 62
+             ? aq_passes(num_qubits)
+             : 0;
+}
+
+static int aq_check(int dtype, int n, int64_t num_states, int64_t in_stride,
+                    int64_t op_stride, int64_t op_qubit_stride) {
+  if (gbsv_all_qubits_passes(dtype, n) == 0)
+    return set_error(GBSV_ERR_UNSUPPORTED,
+                     "needs complex64 states of 9 qubits or more");
+  if (num_states < 0 || in_stride < 0 || op_stride < 0 || op_qubit_stride < 0)
+    return set_error(GBSV_ERR_INVALID_ARG, "negative size or stride");
+  return GBSV_OK;
+}
+
+extern "C" int gbsv_apply_all_qubits_passes(
+    const void* state_in, void* const* pass_out, int dtype, int num_qubits,
+    int64_t num_states, int64_t in_stride, const void* ops, int64_t op_stride,
+    int64_t op_qubit_stride, void* stream) {
+  int rc = aq_check(dtype, num_qubits, num_states, in_stride, op_stride,
+                    op_qubit_stride);
+  if (rc || num_states == 0) return rc;
+  const int np = aq_passes(num_qubits);
+  if (!state_in || !ops || !pass_out)
+    return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
+  for (int i = 0; i < np; ++i)
+    if (!pass_out[i]) return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
+  AllqArgs a{};
+  a.n = num_qubits;
+  a.num_states = num_states;
+  a.op_stride = op_stride;
+  a.op_qstride = op_qubit_stride;
+  const void* src = state_in;
+  for (int i = 0; i < np; ++i) {
+    aq_pass(&a, i);
+    a.in_stride = i == 0 ? in_stride : int64_t(1) << num_qubits;
+    rc = aq_launch(static_cast<const float2*>(src),
+                   static_cast<float2*>(pass_out[i]),
+                   static_cast<const float2*>(ops), a,
+                   static_cast<cudaStream_t>(stream));
+    if (rc) return rc;
+    src = pass_out[i];
+  }
+  return GBSV_OK;
+}
+
+extern "C" size_t gbsv_all_qubits_grad_scratch_bytes(int64_t num_states,
+                                                     int num_qubits,
+                                                     int shared, int each) {
+  if (num_states <= 0 || gbsv_all_qubits_passes(GBSV_C64, num_qubits) == 0)
+    return 0;
+  return aq_grad_scratch(
+      aq_grad_plan(num_states, num_qubits, shared != 0, each != 0),
+      num_states, num_qubits, shared != 0, each != 0);
+}
+
+extern "C" int gbsv_apply_all_qubits_grad(
+    const void* grad_out, const void* const* pass_in, int dtype,
+    int num_qubits, int64_t num_states, int64_t in_stride, const void* ops,
+    int64_t op_stride, int64_t op_qubit_stride, void* grad_state,
+    int need_state, void* grad_ops, int shared, void* scratch,
+    size_t scratch_bytes, void* stream) {
+  int rc = aq_check(dtype, num_qubits, num_states, in_stride, op_stride,
+                    op_qubit_stride);
+  if (rc || num_states == 0) return rc;
+  const int n = num_qubits, np = aq_passes(n);
+  const bool each = op_qubit_stride != 0;
+  if (!grad_out || !ops || !grad_ops || !pass_in ||
+      ((need_state || np > 1) && !grad_state))
+    return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
+  for (int i = 0; i < np; ++i)
+    if (!pass_in[i]) return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
+  const AqGradPlan p = aq_grad_plan(num_states, n, shared != 0, each);
+  const size_t need = aq_grad_scratch(p, num_states, n, shared != 0, each);
+  if (!scratch || scratch_bytes < need || (uintptr_t)scratch % 16)
+    return set_error(GBSV_ERR_SCRATCH,
+                     "all-qubit gradient needs %zu aligned scratch bytes",
+                     need);
+  const uint64_t ctas =
+      n >= AQ_TILE
+          ? (uint64_t)num_states << (n - AQ_TILE - p.chunk_log)
+          : ((uint64_t)num_states + (uint64_t(1) << (AQ_TILE - n)) - 1) >>
+                (AQ_TILE - n);
+  if (ctas > 0x7fffffffull || p.runs * p.parts > 0x7fffffffull)
+    return set_error(GBSV_ERR_UNSUPPORTED, "grid too large");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  AllqGradArgs ga{};
+  ga.f.n = n;
+  ga.f.num_states = num_states;
+  ga.f.op_stride = op_stride;
+  ga.f.op_qstride = op_qubit_stride;
+  ga.chunk_log = p.chunk_log;
+  ga.partial = static_cast<double*>(scratch);
+  const float2* m = static_cast<const float2*>(ops);
+  float2* gs = static_cast<float2*>(grad_state);
+  for (int i = np - 1; i >= 0; --i) {
+    aq_pass(&ga.f, i);
+    ga.f.in_stride = i == 0 ? in_stride : int64_t(1) << n;
+    ga.store = i > 0 || need_state;
+    const float2* x = static_cast<const float2*>(pass_in[i]);
+    const float2* gi =
+        i == np - 1 ? static_cast<const float2*>(grad_out) : gs;
+    switch (std::min(n, AQ_TILE)) {
+      case 9: rc = aq_grad_launch<9>(x, gi, gs, m, ga, ctas, st); break;
+      case 10: rc = aq_grad_launch<10>(x, gi, gs, m, ga, ctas, st); break;
+      case 11: rc = aq_grad_launch<11>(x, gi, gs, m, ga, ctas, st); break;
+      default: rc = aq_grad_launch<12>(x, gi, gs, m, ga, ctas, st); break;
+    }
+    if (rc) return rc;
+  }
+  // sums: chunks (and qubits, states) of each gradient, in a fixed order
+  const double* items = ga.partial;
+  double* next = ga.partial + p.items * 8;
+  uint64_t len = p.len;
+  if (p.parts > 1) {
+    allq_grad_sum_kernel<<<(unsigned)(p.runs * p.parts), AQ_THREADS, 0, st>>>(
+        items, len, p.parts, next, nullptr);
+    rc = after_launch("allq_grad_sum_kernel");
+    if (rc) return rc;
+    items = next;
+    len = p.parts;
+    next += p.runs * p.parts * 8;
+  }
+  const bool states = shared && each;
+  allq_grad_sum_kernel<<<(unsigned)p.runs, AQ_THREADS, 0, st>>>(
+      items, len, 1, next, states ? nullptr : static_cast<float2*>(grad_ops));
+  rc = after_launch("allq_grad_sum_kernel");
+  if (rc || !states) return rc;
+  allq_grad_states_kernel<<<(unsigned)(n * 8), AQ_THREADS, 0, st>>>(
+      next, (uint64_t)num_states, n * 8, static_cast<float*>(grad_ops));
+  return after_launch("allq_grad_states_kernel");
+}

@@ -143,6 +143,18 @@ def _validate_apply(operator, qubits, state):
     return num_qubits, [int(q) for q in qubits], op_num_qubits
 
 
+def _op_grad(gop, plan, tail, target):
+    """Operator gradients of a launch, (num_states or 1, *tail), summed to
+    the shape the operator came in."""
+    target = tuple(target)
+    if plan.op_stride == 0:
+        return gop.reshape(target)
+    grad_op = gop.reshape(plan.out_batch + tail)
+    core = target[len(target) - grad_op.dim():] \
+        if len(target) > grad_op.dim() else target
+    return grad_op.sum_to_size(core).reshape(target)
+
+
 def _dagger(ops: torch.Tensor) -> torch.Tensor:
     return ops.conj().transpose(-1, -2).contiguous()
 
@@ -204,14 +216,7 @@ class _ApplyOperator(torch.autograd.Function):
                 int(shared), scratch.data_ptr() if scratch is not None else
                 None, nbytes, _core.stream_of(g.device))
             _lib.check(rc, "operator_grad")
-            target = tuple(ctx.op_shape)
-            if shared:
-                grad_op = gop.reshape(target)
-            else:
-                grad_op = gop.reshape(plan.out_batch + (d, d))
-                core = target[len(target) - grad_op.dim():] \
-                    if len(target) > grad_op.dim() else target
-                grad_op = grad_op.sum_to_size(core).reshape(target)
+            grad_op = _op_grad(gop, plan, (d, d), ctx.op_shape)
         return grad_op, grad_state, None, None, None
 
 
@@ -273,21 +278,25 @@ def act_first_qubits(operator: torch.Tensor,
     return apply_operator(operator, range(k), state)
 
 
-def _apply_all_qubits_kernel(operator, state, n, each):
-    """One launch per qubit; operator is (*b, 2, 2), or (*b, n, 2, 2) with
-    one matrix per qubit when ``each``."""
+def _all_qubits_plan(operator, state, n, each):
+    """(plan, operators, their state stride, their qubit stride); operator
+    is (*b, 2, 2), or (*b, n, 2, 2) with one matrix per qubit when
+    ``each``."""
     plan = _BatchPlan(operator if not each else operator[..., 0, :, :],
                       state, n, 1)
-    if each:
-        if plan.op_stride:
-            ops = operator.expand(plan.out_batch + (n, 2, 2)).contiguous()
-            op_stride = n * 4
-        else:
-            ops = operator.reshape(n, 2, 2).contiguous()
-            op_stride = 0
-        op_qubit_stride = 4
-    else:
-        ops, op_stride, op_qubit_stride = plan.ops, plan.op_stride, 0
+    if not each:
+        return plan, plan.ops, plan.op_stride, 0
+    if plan.op_stride:
+        ops = operator.expand(plan.out_batch + (n, 2, 2)).contiguous()
+        return plan, ops, n * 4, 4
+    return plan, operator.reshape(n, 2, 2).contiguous(), 0, 4
+
+
+def _apply_all_qubits_kernel(operator, state, n, each):
+    """Every qubit's operator, up to 12 qubits per pass over the state
+    (complex64; one launch per qubit otherwise)."""
+    plan, ops, op_stride, op_qubit_stride = _all_qubits_plan(operator, state,
+                                                             n, each)
     state_c = state.contiguous()
     out = torch.empty(plan.out_batch + (2 ** n,), dtype=state.dtype,
                       device=state.device)
@@ -299,6 +308,81 @@ def _apply_all_qubits_kernel(operator, state, n, each):
             _core.stream_of(state.device))
         _lib.check(rc, "apply_all_qubits")
     return out
+
+
+class _ApplyAllQubits(torch.autograd.Function):
+    """apply_all_qubits / apply_each_qubit as one node.  It keeps the states
+    that enter each pass (one per 8 to 12 qubits) instead of one per
+    qubit."""
+
+    @staticmethod
+    def forward(ctx, operator, state, n, each, passes):
+        plan, ops, op_stride, op_qubit_stride = _all_qubits_plan(
+            operator, state, n, each)
+        state_c = state.contiguous()
+        shape = plan.out_batch + (2 ** n,)
+        outs = [torch.empty(shape, dtype=state.dtype, device=state.device)
+                for _ in range(passes)]
+        rc = _lib.load().gbsv_apply_all_qubits_passes(
+            state_c.data_ptr(), _lib.pointer_array(outs),
+            _core.complex_code(state.dtype), n, plan.num_states,
+            plan.in_stride, ops.data_ptr(), op_stride, op_qubit_stride,
+            _core.stream_of(state.device))
+        _lib.check(rc, "apply_all_qubits")
+        ctx.plan, ctx.n, ctx.each = plan, n, each
+        ctx.ops, ctx.strides = ops, (op_stride, op_qubit_stride)
+        ctx.op_shape, ctx.state_shape = operator.shape, state.shape
+        ctx.save_for_backward(state_c, *outs[:-1])
+        return outs[-1]
+
+    @staticmethod
+    def backward(ctx, g):
+        entered = ctx.saved_tensors
+        plan, n, each, ops = ctx.plan, ctx.n, ctx.each, ctx.ops
+        op_stride, op_qubit_stride = ctx.strides
+        g = g.contiguous()
+        need_op, need_state = ctx.needs_input_grad[:2]
+        grad_op = gs = None
+        L = _lib.load()
+        code, stream = _core.complex_code(g.dtype), _core.stream_of(g.device)
+        if need_state or len(entered) > 1:
+            gs = torch.empty_like(g)
+        if need_op:
+            shared = plan.op_stride == 0
+            nbytes = int(L.gbsv_all_qubits_grad_scratch_bytes(
+                plan.num_states, n, int(shared), int(each)))
+            scratch = torch.empty(nbytes, dtype=torch.uint8, device=g.device)
+            tail = (n, 2, 2) if each else (2, 2)
+            gop = torch.empty((1 if shared else plan.num_states,) + tail,
+                              dtype=g.dtype, device=g.device)
+            rc = L.gbsv_apply_all_qubits_grad(
+                g.data_ptr(), _lib.pointer_array(entered), code, n,
+                plan.num_states, plan.in_stride, ops.data_ptr(), op_stride,
+                op_qubit_stride, gs.data_ptr() if gs is not None else None,
+                int(need_state), gop.data_ptr(), int(shared),
+                scratch.data_ptr(), nbytes, stream)
+            _lib.check(rc, "apply_all_qubits_grad")
+            grad_op = _op_grad(gop, plan, tail, ctx.op_shape)
+        elif need_state:
+            rc = L.gbsv_apply_all_qubits(
+                g.data_ptr(), gs.data_ptr(), code, n, plan.num_states,
+                2 ** n, _dagger(ops).data_ptr(), op_stride, op_qubit_stride,
+                stream)
+            _lib.check(rc, "apply_all_qubits")
+        if not need_state:
+            return grad_op, None, None, None, None
+        if plan.state_expanded:
+            gs = gs.reshape(-1, 2 ** n).sum(0)
+        return grad_op, gs.reshape(ctx.state_shape), None, None, None
+
+
+def _all_qubits_passes(operator, state, n) -> int:
+    """Passes of the one-node form, or 0 where the loop over the qubits
+    runs: complex128, fewer than 9 qubits, no states."""
+    if not state.numel() or not operator.numel():
+        return 0
+    return _lib.load().gbsv_all_qubits_passes(
+        _core.complex_code(state.dtype), n)
 
 
 def apply_all_qubits(operator: torch.Tensor,
@@ -317,6 +401,10 @@ def apply_all_qubits(operator: torch.Tensor,
                            "qubit")
     if torch.is_grad_enabled() and (operator.requires_grad
                                     or state.requires_grad):
+        passes = _all_qubits_passes(operator, state, num_qubits)
+        if passes:
+            return _ApplyAllQubits.apply(operator, state, num_qubits, False,
+                                         passes)
         out = state
         for q in range(num_qubits):
             out = apply_operator(operator, [q], out)
@@ -343,6 +431,10 @@ def apply_each_qubit(operators: torch.Tensor,
     _check_dtypes(operators, state)
     if torch.is_grad_enabled() and (operators.requires_grad
                                     or state.requires_grad):
+        passes = _all_qubits_passes(operators, state, num_qubits)
+        if passes:
+            return _ApplyAllQubits.apply(operators, state, num_qubits, True,
+                                         passes)
         out = state
         for q in range(num_qubits):
             out = apply_operator(operators[..., q, :, :], [q], out)

@@ -95,3 +95,59 @@ def test_all_qubits_broadcast_state_and_odd_offset(n):
     got = ug.apply_all_qubits(torch.from_numpy(ops).to(DEV), buf[1:])
     ref = _reference(ops, psi, n, False)
     assert np.abs(got.cpu().numpy() - ref).max() <= _tol(n)
+
+
+# Gradients against complex128 autograd through the per-qubit loop.  Per
+# amplitude the FP32 states differ from complex128 by about 4 sqrt(2 n)
+# 2^-24 of the state's norm (forward and adjoint), sums are exact beside
+# that, and a sum over B states and n qubits grows like the reference's.
+@pytest.mark.parametrize("n,batch", [(9, 9), (10, 4), (11, 3), (12, 2),
+                                     (13, 2), (17, 2), (20, 1), (22, 1)])
+@pytest.mark.parametrize("each", [False, True])
+@pytest.mark.parametrize("form", ["shared", "per_state", "broadcast_state",
+                                  "operator_only"])
+def test_all_qubits_gradients(n, batch, each, form):
+    rng = np.random.default_rng(n)
+    b = (batch,)
+    ops = torch.from_numpy(_unitaries(
+        rng, (b if form in ("per_state", "broadcast_state") else ()) +
+        ((n,) if each else ()))).to(DEV)
+    psi = torch.from_numpy(_states(
+        rng, () if form == "broadcast_state" else b, n)).to(DEV)
+    w = torch.from_numpy(_states(rng, b, n)).to(DEV)
+
+    def loss(m, s, wide):
+        if wide:
+            out = s
+            for q in range(n):
+                out = ug.apply_operator(m[..., q, :, :] if each else m, [q],
+                                        out)
+        else:
+            out = (ug.apply_each_qubit if each else ug.apply_all_qubits)(m, s)
+        return (w.to(out.dtype).conj() * out).sum(-1).abs().square().sum()
+
+    grads = []
+    for dt in (torch.complex64, torch.complex128):
+        m = ops.to(dt, copy=True).requires_grad_()
+        s = psi.to(dt, copy=True).requires_grad_(form != "operator_only")
+        loss(m, s, dt == torch.complex128).backward()
+        grads.append((m.grad, s.grad))
+    tol = 16 * np.sqrt(2 * n) * 2.0 ** -24
+    for got, ref in zip(*grads):
+        if ref is None:
+            assert got is None
+            continue
+        assert got.shape == ref.shape and got.dtype == torch.complex64
+        off = torch.linalg.vector_norm(got.to(ref.dtype) - ref)
+        assert off <= tol * torch.linalg.vector_norm(ref) * n
+
+
+def test_all_qubits_gradient_state_only_and_unused():
+    n, rng = 14, np.random.default_rng(3)
+    m = torch.from_numpy(_unitaries(rng, (2,))).to(DEV)
+    s = torch.from_numpy(_states(rng, (2,), n)).to(DEV).requires_grad_()
+    w = torch.from_numpy(_states(rng, (2,), n)).to(DEV)
+    out = ug.apply_all_qubits(m, s)
+    out.backward(w)
+    ref = ug.apply_all_qubits(m.conj().transpose(-1, -2), w)
+    assert torch.equal(s.grad, ref)
