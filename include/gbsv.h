@@ -446,6 +446,19 @@ int gbsv_operator_grad(const void* grad_out, const void* state_in, int dtype,
                        void* grad_ops, int shared, void* scratch,
                        size_t scratch_bytes, void* stream);
 
+/* gbsv_operator_grad with the state's gradient U^H grad_out (num_states
+ * dense states, not grad_out) from the same read of grad_out: complex64
+ * operators on 1 or 2 qubits, ops and op_stride as for gbsv_apply_operator;
+ * grad_state NULL gives the operator's gradient alone, for every k.
+ * Scratch as for gbsv_operator_grad. */
+int gbsv_apply_operator_grad(const void* grad_out, const void* state_in,
+                             int dtype, int num_qubits, int64_t num_states,
+                             int64_t in_stride, const void* ops,
+                             int64_t op_stride, const int32_t* qubits,
+                             int num_targets, void* grad_state,
+                             void* grad_ops, int shared, void* scratch,
+                             size_t scratch_bytes, void* stream);
+
 /* ---- adjoint differentiation ------------------------------------------ */
 
 /* One term c * P of a Pauli-sum observable (32 bytes, device memory).

@@ -115,6 +115,9 @@ SIGNATURES = {
     "gbsv_operator_grad": (_I, [_P, _P, _I, _I, _I64, _I64,
                                 ctypes.POINTER(_I32), _I, _P, _I, _P, _SZ,
                                 _P]),
+    "gbsv_apply_operator_grad": (_I, [_P, _P, _I, _I, _I64, _I64, _P, _I64,
+                                      ctypes.POINTER(_I32), _I, _P, _P, _I,
+                                      _P, _SZ, _P]),
     "gbsv_pauli_sum_apply": (_I, [_P, _P, _I, _I, _I64, _P, _I, _P]),
     "gbsv_adjoint_scratch_bytes": (_SZ, [_I64, _I]),
     "gbsv_adjoint_rotation_step": (_I, [_P, _P, _I, _I, _I64, _I, _I, _P, _I,

@@ -192,13 +192,13 @@ class _ApplyOperator(torch.autograd.Function):
             return (torch.zeros(ctx.op_shape, dtype=g.dtype, device=g.device),
                     torch.zeros(ctx.state_shape, dtype=g.dtype,
                                 device=g.device), None, None, None)
-        if ctx.needs_input_grad[1]:
-            gs = torch.empty_like(g)
+        gs = torch.empty_like(g) if ctx.needs_input_grad[1] else None
+        # complex64 operators on 1 or 2 qubits: both gradients in one pass
+        both = (all(ctx.needs_input_grad[:2]) and k in (1, 2) and
+                g.dtype == torch.complex64)
+        if gs is not None and not both:
             _launch_apply(_dagger(plan.ops), plan.op_stride, g, 2 ** n, gs, n,
                           qubits, plan.num_states)
-            if plan.state_expanded:
-                gs = gs.reshape(-1, 2 ** n).sum(0)
-            grad_state = gs.reshape(ctx.state_shape)
         if ctx.needs_input_grad[0]:
             shared = plan.op_stride == 0
             d = 2 ** k
@@ -209,14 +209,20 @@ class _ApplyOperator(torch.autograd.Function):
                        if nbytes else None)
             gop = torch.empty((1 if shared else plan.num_states, d, d),
                               dtype=g.dtype, device=g.device)
-            rc = L.gbsv_operator_grad(
+            rc = L.gbsv_apply_operator_grad(
                 g.data_ptr(), state_c.data_ptr(),
                 _core.complex_code(g.dtype), n, plan.num_states,
-                plan.in_stride, _lib.qubit_array(qubits), k, gop.data_ptr(),
+                plan.in_stride, plan.ops.data_ptr(), plan.op_stride,
+                _lib.qubit_array(qubits), k,
+                gs.data_ptr() if both else None, gop.data_ptr(),
                 int(shared), scratch.data_ptr() if scratch is not None else
                 None, nbytes, _core.stream_of(g.device))
             _lib.check(rc, "operator_grad")
             grad_op = _op_grad(gop, plan, (d, d), ctx.op_shape)
+        if gs is not None:
+            if plan.state_expanded:
+                gs = gs.reshape(-1, 2 ** n).sum(0)
+            grad_state = gs.reshape(ctx.state_shape)
         return grad_op, grad_state, None, None, None
 
 
