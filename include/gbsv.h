@@ -169,6 +169,18 @@ int gbsv_apply_phase(const void* angles, int angle_dtype, const void* state,
                      int state_dtype, void* out, int out_dtype,
                      const gbsv_bcast_t* bc, void* stream);
 
+/* Backward of gbsv_apply_phase from grad_out = dL/d(out) (both dense, of
+ * out_dtype): grad_state = exp(i * angles) * grad_out in out_dtype and
+ * grad_angles = Re(i * grad_out * conj(out)) in out_dtype's real type, each
+ * over the whole broadcast output bc (operand a the angles, operand b
+ * unused; the caller sums broadcast dims).  Either may be NULL.  The
+ * autograd backward that unitair gets from torch
+ * (src/unitair/simulation/operations.py:15-42). */
+int gbsv_apply_phase_grad(const void* angles, int angle_dtype,
+                          const void* grad_out, const void* out,
+                          int out_dtype, const gbsv_bcast_t* bc,
+                          void* grad_state, void* grad_angles, void* stream);
+
 /* ---- fused gate stages ------------------------------------------------ */
 
 /* One fused-stage gate record (48 bytes, device memory).  kind:

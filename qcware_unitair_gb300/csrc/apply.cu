@@ -1792,24 +1792,48 @@ struct PhaseArgs {
   int df;  // double angles: double-float pairs (1) or FP64 (0)
 };
 
-// out = (cos t - i sin t) * psi.
+// exp(-i t).  The phase factor is formed in the angle's precision, as torch
+// forms exp(-1j * angles) in complex(angles.dtype); the product is then taken
+// in the promoted output precision.  Double angles within 2^20 use pairs
+// (df_sincos); the angle is kept for amplitudes outside the pair range.
+template <typename RA> struct PhaseFactor;
+template <> struct PhaseFactor<float> {
+  float s, c;
+};
+template <> struct PhaseFactor<double> {
+  double t;
+  DSC sc;
+  bool pairs;
+};
+
+__device__ __forceinline__ PhaseFactor<float> phase_factor(float t, int) {
+  PhaseFactor<float> f;
+  sincosf(t, &f.s, &f.c);
+  return f;
+}
+__device__ __forceinline__ PhaseFactor<double> phase_factor(double t,
+                                                            int df) {
+  PhaseFactor<double> f;
+  f.t = t;
+  f.pairs = df && (df_hiword(t) & 0x7ff00000u) <= ((1023u + 19) << 20);
+  if (f.pairs) f.sc = df_sincos(t);
+  return f;
+}
+
+// (cos t - i sin t) * v
 template <typename RA, typename RS, typename RO>
-__device__ __forceinline__ Cx<RO> phase_one(RA t, Cx<RS> v, int df) {
-  // The phase factor is formed in the angle's precision, as torch forms
-  // exp(-1j * angles) in complex(angles.dtype); the product is then taken
-  // in the promoted output precision.
+__device__ __forceinline__ Cx<RO> phase_times(const PhaseFactor<RA>& f,
+                                              Cx<RS> v) {
+  RA sa, ca;
   if constexpr (sizeof(RA) == 8) {
-    // double angles in pairs (df_sincos) when the angle is within 2^20 and
-    // the amplitude within the pair range; FP64 otherwise
     uint32_t mx = 0;
     if constexpr (sizeof(RS) == 8)
       mx = max(df_hiword(v.x) & 0x7ff00000u, df_hiword(v.y) & 0x7ff00000u);
-    const bool ok = df && (df_hiword(t) & 0x7ff00000u) <= ((1023u + 19) << 20) &&
+    const bool ok = f.pairs &&
                     (sizeof(RS) == 4 ||
                      (mx < ((DF_EMAX + 1) << 20) &&
                       (mx == 0 || mx >= (DF_EMIN << 20))));
     if (ok) {
-      const DSC sc = df_sincos(t);
       DC a;
       if constexpr (sizeof(RS) == 8) {
         a = df_split2(v.x, v.y);
@@ -1817,22 +1841,30 @@ __device__ __forceinline__ Cx<RO> phase_one(RA t, Cx<RS> v, int df) {
         a.re = DF{(float)v.x, 0.f};
         a.im = DF{(float)v.y, 0.f};
       }
-      const DF re = df_sum2(df_prod2(sc.c, a.re), df_prod2(sc.s, a.im));
-      const DF im = df_sum2(df_prod2(sc.c, a.im), df_neg(df_prod2(sc.s, a.re)));
+      const DF re = df_sum2(df_prod2(f.sc.c, a.re), df_prod2(f.sc.s, a.im));
+      const DF im =
+          df_sum2(df_prod2(f.sc.c, a.im), df_neg(df_prod2(f.sc.s, a.re)));
       Cx<RO> o;
       o.x = df_join(re);
       o.y = df_join(im);
       return o;
     }
+    sincos(f.t, &sa, &ca);
+  } else {
+    sa = f.s;
+    ca = f.c;
   }
-  RA sa, ca;
-  sincos(t, &sa, &ca);
   const RO s = (RO)sa, c = (RO)ca;
   const RO x = (RO)v.x, y = (RO)v.y;
   Cx<RO> o;
-  o.x = c * x + s * y;
-  o.y = c * y - s * x;
+  o.x = fma(c, x, s * y);
+  o.y = fma(c, y, -(s * x));
   return o;
+}
+
+template <typename RA, typename RS, typename RO>
+__device__ __forceinline__ Cx<RO> phase_one(RA t, Cx<RS> v, int df) {
+  return phase_times<RA, RS, RO>(phase_factor(t, df), v);
 }
 
 template <typename RA, typename RS, typename RO, int NDIM>
@@ -1875,9 +1907,158 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Element offsets of the angle and the state at row `row` (all dims but the
+// last) of the broadcast.
+__device__ __forceinline__ void phase_row(const PhaseArgs& a, uint64_t row,
+                                          int64_t* oa, int64_t* ob) {
+  *oa = *ob = 0;
+  for (int d = a.ndim - 2; d >= 0; --d) {
+    const uint64_t sz = (uint64_t)a.shape[d];
+    const uint64_t idx = row % sz;
+    row /= sz;
+    *oa += (int64_t)idx * a.sa[d];
+    *ob += (int64_t)idx * a.sb[d];
+  }
+}
+
+constexpr int PHASE_COLS = 1024;  // columns per block: four per thread
+constexpr int PHASE_ROWS = 8;     // rows per block, at most
+
+struct PhaseRowArgs {
+  PhaseArgs p;
+  uint64_t cols, rows;
+  uint64_t col_blocks;
+  int per;     // rows per block
+  int shared;  // the angles are the same in every row
+};
+
+// The broadcast forms: angles over a batch of states, or states over a
+// batch of angles.  A block takes 1024 columns of up to eight rows and finds
+// the row offsets once (one element at a time, their 64-bit divisions cost
+// more than the element); a phase factor is formed once where the rows
+// share the angles.  7 states of 20 qubits, one set of angles: 43 us by
+// element, 17 us here (HBM: 18 us without the L2).
+template <typename RA, typename RS, typename RO>
+__global__ void __launch_bounds__(256)
+    phase_rows_kernel(const RA* ang, const Cx<RS>* psi, Cx<RO>* out,
+                      PhaseRowArgs a) {
+  __shared__ int64_t off_a[PHASE_ROWS], off_b[PHASE_ROWS];
+  const uint64_t cb = blockIdx.x % a.col_blocks;
+  const uint64_t row0 = (blockIdx.x / a.col_blocks) * a.per;
+  const int nrows =
+      a.rows - row0 < (uint64_t)a.per ? (int)(a.rows - row0) : a.per;
+  if ((int)threadIdx.x < nrows)
+    phase_row(a.p, row0 + threadIdx.x, &off_a[threadIdx.x],
+              &off_b[threadIdx.x]);
+  __syncthreads();
+  const int64_t s0 = a.p.sa[a.p.ndim - 1], s1 = a.p.sb[a.p.ndim - 1];
+  const uint64_t c0 = cb * PHASE_COLS + threadIdx.x;
+  PhaseFactor<RA> f[4];
+  for (int r = 0; r < nrows; ++r) {
+    if (r == 0 || !a.shared) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint64_t c = c0 + 256 * k;
+        if (c < a.cols)
+          f[k] = phase_factor(ang[off_a[r] + (int64_t)c * s0], a.p.df);
+      }
+    }
+    Cx<RS> v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint64_t c = c0 + 256 * k;
+      if (c < a.cols) v[k] = psi[off_b[r] + (int64_t)c * s1];
+    }
+    Cx<RO>* dst = out + (row0 + r) * a.cols;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint64_t c = c0 + 256 * k;
+      if (c < a.cols) dst[c] = phase_times<RA, RS, RO>(f[k], v[k]);
+    }
+  }
+}
+
+// Backward of out = exp(-i a) psi from g = dL/d(out), both gradients from
+// one read of g and out: gs = exp(i a) g and ga = Re(i g conj(out)), over
+// the broadcast output (the caller sums broadcast dims).  out and g are
+// dense; ROWS as above, by element otherwise.
+template <typename RA, typename RO, bool ROWS>
+__global__ void __launch_bounds__(256)
+    phase_grad_kernel(const RA* ang, const Cx<RO>* g, const Cx<RO>* out,
+                      Cx<RO>* gs, RO* ga, PhaseRowArgs a) {
+  const uint64_t stride = (uint64_t)gridDim.x * 256;
+  uint64_t i, end, step;
+  int64_t oa = 0, ob;
+  const int64_t s0 = a.p.sa[a.p.ndim - 1];
+  uint64_t row_base = 0;
+  if constexpr (ROWS) {
+    const uint64_t row = blockIdx.x / a.col_blocks;
+    const uint64_t cb = blockIdx.x % a.col_blocks;
+    phase_row(a.p, row, &oa, &ob);
+    row_base = row * a.cols;
+    i = cb * PHASE_COLS + threadIdx.x;
+    end = (cb + 1) * PHASE_COLS < a.cols ? (cb + 1) * PHASE_COLS : a.cols;
+    step = 256;
+  } else {
+    i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+    end = a.p.total;
+    step = stride;
+  }
+#pragma unroll 4
+  for (; i < end; i += step) {
+    int64_t at;
+    if constexpr (ROWS) {
+      at = oa + (int64_t)i * s0;
+    } else {
+      phase_row(a.p, i / a.cols, &oa, &ob);
+      at = oa + (int64_t)(i % a.cols) * s0;
+    }
+    const Cx<RO> gv = g[row_base + i];
+    if (ga) {
+      const Cx<RO> o = out[row_base + i];
+      ga[row_base + i] = fma(gv.x, o.y, -(gv.y * o.x));
+    }
+    if (gs)
+      gs[row_base + i] = phase_times<RA, RO, RO>(
+          phase_factor((RA)-ang[at], a.p.df), gv);
+  }
+}
+
+// Whether rows are long enough for a block of columns each.
+static bool phase_by_rows(const PhaseArgs& a) {
+  return a.shape[a.ndim - 1] >= PHASE_COLS / 4;
+}
+
+static PhaseRowArgs phase_row_args(const PhaseArgs& a, int most_rows) {
+  PhaseRowArgs r{};
+  r.p = a;
+  r.cols = (uint64_t)a.shape[a.ndim - 1];
+  r.rows = a.total / r.cols;
+  r.col_blocks = (r.cols + PHASE_COLS - 1) / PHASE_COLS;
+  r.shared = 1;
+  for (int d = 0; d + 1 < a.ndim; ++d) r.shared &= a.sa[d] == 0;
+  // rows share a block only where they share its angles, and only as far as
+  // the chip still gets a few blocks per SM
+  r.per = 1;
+  while (r.shared && r.per < most_rows && r.per < (int64_t)r.rows &&
+         r.col_blocks * (r.rows / (2 * r.per)) >= (uint64_t)sm_count() * 4)
+    r.per *= 2;
+  return r;
+}
+
 template <typename RA, typename RS, typename RO>
 static int launch_phase(const void* ang, const void* psi, void* out,
                         const PhaseArgs& a, cudaStream_t st) {
+  if (a.ndim > 1 && phase_by_rows(a)) {
+    const PhaseRowArgs r = phase_row_args(a, PHASE_ROWS);
+    const uint64_t grid = r.col_blocks * ((r.rows + r.per - 1) / r.per);
+    if (grid <= 0x7fffffffull) {
+      phase_rows_kernel<RA, RS, RO><<<(unsigned)grid, 256, 0, st>>>(
+          static_cast<const RA*>(ang), static_cast<const Cx<RS>*>(psi),
+          static_cast<Cx<RO>*>(out), r);
+      return after_launch("phase_rows_kernel");
+    }
+  }
   uint64_t blocks = (a.total + 255) / 256;
   const uint64_t cap = (uint64_t)sm_count() * 32;
   if (blocks > cap) blocks = cap;
@@ -1935,4 +2116,58 @@ extern "C" int gbsv_apply_phase(const void* angles, int angle_dtype,
   if (angle_dtype == GBSV_F32 && state_dtype == GBSV_C128)
     return launch_phase<float, double, double>(angles, state, out, a, st);
   return launch_phase<double, double, double>(angles, state, out, a, st);
+}
+
+extern "C" int gbsv_apply_phase_grad(const void* angles, int angle_dtype,
+                                     const void* grad_out, const void* out,
+                                     int out_dtype, const gbsv_bcast_t* bc,
+                                     void* grad_state, void* grad_angles,
+                                     void* stream) {
+  if (!bc || bc->ndim < 1 || bc->ndim > GBSV_MAX_DIMS)
+    return set_error(GBSV_ERR_INVALID_ARG, "bad broadcast descriptor");
+  if ((angle_dtype != GBSV_F32 && angle_dtype != GBSV_F64) ||
+      (out_dtype != GBSV_C64 && out_dtype != GBSV_C128) ||
+      (angle_dtype == GBSV_F64 && out_dtype != GBSV_C128))
+    return set_error(GBSV_ERR_INVALID_ARG, "bad angle or output dtype");
+  PhaseArgs a{};
+  a.df = c128_arith() == GBSV_C128_PAIRS;
+  a.ndim = bc->ndim;
+  a.total = 1;
+  for (int d = 0; d < bc->ndim; ++d) {
+    if (bc->shape[d] < 0)
+      return set_error(GBSV_ERR_INVALID_ARG, "negative extent");
+    a.shape[d] = bc->shape[d];
+    a.sa[d] = bc->stride_a[d];
+    a.sb[d] = bc->stride_b[d];
+    a.total *= (uint64_t)bc->shape[d];
+  }
+  if (a.total == 0 || (!grad_state && !grad_angles)) return GBSV_OK;
+  if (!angles || !grad_out || !out)
+    return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const PhaseRowArgs r = phase_row_args(a, 1);
+  const uint64_t row_grid = r.col_blocks * r.rows;
+  const bool rows = phase_by_rows(a) && row_grid <= 0x7fffffffull;
+  const uint64_t grid =
+      rows ? row_grid
+           : std::min<uint64_t>((a.total + 255) / 256,
+                                (uint64_t)sm_count() * 32);
+#define GBSV_PHASE_GRAD(RA, RO, ROWS)                               \
+  phase_grad_kernel<RA, RO, ROWS><<<(unsigned)grid, 256, 0, st>>>(  \
+      static_cast<const RA*>(angles),                               \
+      static_cast<const Cx<RO>*>(grad_out),                         \
+      static_cast<const Cx<RO>*>(out),                              \
+      static_cast<Cx<RO>*>(grad_state), static_cast<RO*>(grad_angles), r)
+  if (out_dtype == GBSV_C64) {
+    if (rows) GBSV_PHASE_GRAD(float, float, true);
+    else GBSV_PHASE_GRAD(float, float, false);
+  } else if (angle_dtype == GBSV_F32) {
+    if (rows) GBSV_PHASE_GRAD(float, double, true);
+    else GBSV_PHASE_GRAD(float, double, false);
+  } else {
+    if (rows) GBSV_PHASE_GRAD(double, double, true);
+    else GBSV_PHASE_GRAD(double, double, false);
+  }
+#undef GBSV_PHASE_GRAD
+  return after_launch("phase_grad_kernel");
 }

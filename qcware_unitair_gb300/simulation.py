@@ -458,15 +458,36 @@ class _ApplyPhase(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         angles, state, out = ctx.saved_tensors
-        ga = gs = None
-        if ctx.needs_input_grad[1]:
-            gs = _phase_kernel(-angles, g.contiguous())
+        need_angles, need_state = ctx.needs_input_grad[:2]
+        # out = exp(-i a) psi  =>  dL/dpsi = exp(i a) g and
+        # dL/da = Re(i * g * conj(out)), both from one read of g
+        a = _phase_angles(angles).contiguous()
+        g = g.contiguous()
+        gs = torch.empty_like(g) if need_state else None
+        ga = torch.empty(g.shape, dtype=_core.real_of(g.dtype),
+                         device=g.device) if need_angles else None
+        if g.numel():
+            desc = _core.bcast_desc(g.shape,
+                                    _core.broadcast_strides(a, g.shape),
+                                    _core.broadcast_strides(g, g.shape))
+            rc = _lib.load().gbsv_apply_phase_grad(
+                a.data_ptr(), _core.real_code(a.dtype), g.data_ptr(),
+                out.data_ptr(), _core.complex_code(g.dtype), desc,
+                gs.data_ptr() if need_state else None,
+                ga.data_ptr() if need_angles else None,
+                _core.stream_of(g.device))
+            _lib.check(rc, "apply_phase_grad")
+        if need_state:
             gs = gs.to(state.dtype).sum_to_size(state.shape)
-        if ctx.needs_input_grad[0]:
-            # out = exp(-i a) psi  =>  dL/da = Re(i * g * conj(out))
-            ga = (1j * g * out.conj()).real.to(angles.dtype)
-            ga = ga.sum_to_size(angles.shape)
+        if need_angles:
+            ga = ga.to(angles.dtype).sum_to_size(angles.shape)
         return ga, gs
+
+
+def _phase_angles(angles: torch.Tensor) -> torch.Tensor:
+    if angles.dtype in (torch.float32, torch.float64):
+        return angles
+    return angles.to(torch.float32)
 
 
 def _phase_kernel(angles: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
@@ -474,10 +495,7 @@ def _phase_kernel(angles: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
     scode = _core.complex_code(state.dtype)
     if angles.is_complex():
         raise NotImplementedError("apply_phase takes real angles")
-    if not angles.is_floating_point():
-        angles = angles.to(torch.float32)
-    if angles.dtype not in (torch.float32, torch.float64):
-        angles = angles.to(torch.float32)
+    angles = _phase_angles(angles)
     acode = _core.real_code(angles.dtype)
     out_dtype = torch.complex128 if (angles.dtype == torch.float64 or
                                      state.dtype == torch.complex128) \

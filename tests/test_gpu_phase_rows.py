@@ -1,0 +1,51 @@
+"""apply_phase over broadcast rows and its backward, against complex128 torch:
+rows below, at and above a block of columns, several rows per block, angles
+shared or per row, states shared, every dtype pair.
+
+Tolerance: the factor is rounded to the angle's precision (an error of at
+most 2 ulp per component), the product to the output's: 8 * eps of the
+largest amplitude for the coarser of the two; sums over broadcast rows add
+one rounding per row."""
+import numpy as np
+import pytest
+import torch
+
+import qcware_unitair_gb300 as ug
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+@pytest.mark.parametrize("shape_a,shape_s", [
+    ((255,), (3, 255)), ((256,), (3, 256)), ((1024,), (9, 1024)),
+    ((1025,), (1300, 1025)), ((5, 1), (5, 2048)), ((4, 1, 700), (1, 3, 700)),
+    ((6, 512), (512,)), ((2, 1, 64), (2, 5, 64)), ((3, 300), (3, 300)),
+    ((1,), (2, 1000)), ((7,), (2, 7))])
+@pytest.mark.parametrize("da", [torch.float32, torch.float64])
+@pytest.mark.parametrize("ds", [torch.complex64, torch.complex128])
+def test_phase_and_gradients(shape_a, shape_s, da, ds):
+    rng = np.random.default_rng(len(shape_a) + shape_s[-1])
+    a = torch.from_numpy(rng.uniform(-9, 9, shape_a)).to(da).to(DEV)
+    s = torch.from_numpy(rng.normal(size=shape_s) +
+                         1j * rng.normal(size=shape_s)).to(ds).to(DEV)
+    a.requires_grad_()
+    s.requires_grad_()
+    out = ug.apply_phase(a, s)
+    w = torch.from_numpy(rng.normal(size=out.shape) + 1j *
+                         rng.normal(size=out.shape)).to(out.dtype).to(DEV)
+    out.backward(w)
+    a2 = a.detach().double().requires_grad_()
+    s2 = s.detach().to(torch.complex128).requires_grad_()
+    ref = torch.exp(-1j * a2) * s2
+    ref.backward(w.to(torch.complex128))
+    assert out.dtype == torch.promote_types(
+        ds, torch.complex64 if da == torch.float32 else torch.complex128)
+    coarse = da == torch.float32 or ds == torch.complex64
+    eps = 2.0 ** -24 if coarse else 2.0 ** -46
+    for got, want in ((out, ref), (s.grad, s2.grad), (a.grad, a2.grad)):
+        rows = max(1, out.numel() // got.numel())
+        assert got.shape == want.shape
+        off = (got.detach().to(want.dtype) - want.detach()).abs().max()
+        # both factors of dL/da are up to |w| |out|
+        size = want.detach().abs().max() + w.abs().max() * s.abs().max()
+        assert off <= 8 * eps * rows * size
