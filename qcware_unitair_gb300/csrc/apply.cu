@@ -1937,7 +1937,7 @@ struct PhaseRowArgs {
 // the row offsets once (one element at a time, their 64-bit divisions cost
 // more than the element); a phase factor is formed once where the rows
 // share the angles.  7 states of 20 qubits, one set of angles: 43 us by
-// element, 17 us here (HBM: 18 us without the L2).
+// element, 25 us here (HBM: 18 us without the L2).
 template <typename RA, typename RS, typename RO>
 __global__ void __launch_bounds__(256)
     phase_rows_kernel(const RA* ang, const Cx<RS>* psi, Cx<RO>* out,
@@ -1954,7 +1954,17 @@ __global__ void __launch_bounds__(256)
   const int64_t s0 = a.p.sa[a.p.ndim - 1], s1 = a.p.sb[a.p.ndim - 1];
   const uint64_t c0 = cb * PHASE_COLS + threadIdx.x;
   PhaseFactor<RA> f[4];
+  Cx<RS> v[4], next[4];
+  auto load = [&](int r, Cx<RS>* x) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint64_t c = c0 + 256 * k;
+      if (c < a.cols) x[k] = psi[off_b[r] + (int64_t)c * s1];
+    }
+  };
+  load(0, v);
   for (int r = 0; r < nrows; ++r) {
+    if (r + 1 < nrows) load(r + 1, next);  // in flight during this row
     if (r == 0 || !a.shared) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -1963,18 +1973,14 @@ __global__ void __launch_bounds__(256)
           f[k] = phase_factor(ang[off_a[r] + (int64_t)c * s0], a.p.df);
       }
     }
-    Cx<RS> v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint64_t c = c0 + 256 * k;
-      if (c < a.cols) v[k] = psi[off_b[r] + (int64_t)c * s1];
-    }
     Cx<RO>* dst = out + (row0 + r) * a.cols;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint64_t c = c0 + 256 * k;
       if (c < a.cols) dst[c] = phase_times<RA, RS, RO>(f[k], v[k]);
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = next[k];
   }
 }
 
