@@ -489,6 +489,33 @@ int gbsv_pauli_sum_apply(const void* psi, void* out, int dtype,
                          int num_qubits, int64_t num_states,
                          const void* terms, int num_terms, void* stream);
 
+/* gbsv_pauli_sum_apply with the terms in HOST memory: they travel as a
+ * kernel parameter, so nothing waits for a copy. */
+int gbsv_pauli_sum_apply_host(const void* psi, void* out, int dtype,
+                              int num_qubits, int64_t num_states,
+                              const gbsv_pauli_term_t* terms, int num_terms,
+                              void* stream);
+
+/* One parameterised rotation exp(-i theta/2 P) of a program (32 bytes,
+ * device memory): theta = 2 * half * params[b, pidx] for state b; its matrix
+ * (nv = 4 entries, or the 2 of a diagonal; generator 0 X, 1 Y, 2 Z) is at
+ * pool + off + b * nv. */
+typedef struct gbsv_rotation {
+  int32_t gen, nv, pidx, pad_;
+  int64_t off;
+  double half;
+} gbsv_rotation_t;
+
+/* Write the matrices of num_rots rotations for num_states states into a
+ * program's pool (complex, `dtype`), sin and cos in FP64; params is
+ * (num_states, num_params) real.  unitair builds these matrices with a
+ * handful of torch operations per gate
+ * (src/unitair/gates/gates.py:6-91). */
+int gbsv_rotation_values(const void* params, int params_dtype,
+                         int64_t num_params, int64_t num_states,
+                         const void* rots, int64_t num_rots, void* pool,
+                         int dtype, void* stream);
+
 /* Scratch bytes gbsv_adjoint_rotation_step needs. */
 size_t gbsv_adjoint_scratch_bytes(int64_t num_states, int num_qubits);
 

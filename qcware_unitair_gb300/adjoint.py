@@ -66,9 +66,9 @@ class PauliSum:
         dt = np.dtype([("x", "<u8"), ("z", "<u8"), ("re", "<f8"),
                        ("im", "<f8")])
         out = np.zeros(len(self.terms), dtype=dt)
-        for k, (c, ps) in enumerate(self.terms):
-            xm = zm = 0
-            ny = 0
+        xs, zs, res, ims = [], [], [], []
+        for c, ps in self.terms:
+            xm = zm = ny = 0
             for q, p in ps.items():
                 bit = 1 << (n - 1 - q)
                 if p in "XY":
@@ -76,8 +76,12 @@ class PauliSum:
                 if p in "ZY":
                     zm |= bit
                 ny += p == "Y"
-            phase = 1j ** ny
-            out[k] = (xm, zm, c * phase.real, c * phase.imag)
+            # c * i^ny
+            xs.append(xm)
+            zs.append(zm)
+            res.append((c, 0.0, -c, 0.0)[ny & 3])
+            ims.append((0.0, c, 0.0, -c)[ny & 3])
+        out["x"], out["z"], out["re"], out["im"] = xs, zs, res, ims
         return out
 
     def dense(self) -> np.ndarray:
@@ -282,6 +286,36 @@ def _rotation_values(which, params, B, dtype):
 _rotation_values._meta = {}
 
 
+ROT_DTYPE = np.dtype([("gen", "<i4"), ("nv", "<i4"), ("pidx", "<i4"),
+                      ("pad", "<i4"), ("off", "<i8"), ("half", "<f8")])
+
+
+def _real_params(params: torch.Tensor) -> torch.Tensor:
+    """Parameters as the kernels read them: contiguous float32/float64."""
+    p = params.detach().contiguous()
+    if p.dtype not in (torch.float32, torch.float64):
+        p = p.to(torch.float64)
+    return p
+
+
+def _write_rotations(prog, which, p):
+    """Every rotation's matrices written into the program's pool by one
+    kernel (sin and cos in FP64)."""
+    from .fusion import _to_device
+    recs = prog.__dict__.get("_rot_recs")
+    if recs is None:
+        host = np.zeros(len(which), dtype=ROT_DTYPE)
+        for i, (gen, pi, scale, off, nv) in enumerate(which):
+            host[i] = (GEN[gen], nv, pi, 0, off, 0.5 * scale)
+        recs = prog._rot_recs = _to_device(host.view(np.uint8),
+                                           prog.pool.device)
+    rc = _lib.load().gbsv_rotation_values(
+        p.data_ptr(), _core.real_code(p.dtype), p.shape[1], p.shape[0],
+        recs.data_ptr(), len(which), prog.pool.data_ptr(),
+        _core.complex_code(prog.dtype), _core.stream_of(p.device))
+    _lib.check(rc, "rotation_values")
+
+
 def _initial_state(n, B, dtype, device, psi0):
     if psi0 is None:
         s = torch.zeros(B, 2 ** n, dtype=dtype, device=device)
@@ -300,7 +334,7 @@ def _forward(pc: ParamCircuit, params, dtype, psi0, checkpoints: bool,
     dev = params.device
     psi = _initial_state(n, B, dtype, dev, psi0)
     saved = []
-    p = params.detach()
+    p = _real_params(params)
     for a, b in pc.segments():
         if checkpoints:
             saved.append(psi.clone())
@@ -313,25 +347,17 @@ def _forward(pc: ParamCircuit, params, dtype, psi0, checkpoints: bool,
             continue
         prog, which, _ = _forward_program(pc, a, b, B, dtype, dev, fuse)
         if which:
-            # one scatter of every rotation's values into the cached pool
-            idx = prog.__dict__.get("_rot_index")
-            if idx is None:
-                parts = [torch.arange(off, off + B * nv, device=dev)
-                         for _, _, _, off, nv in which]
-                idx = prog._rot_index = torch.cat(parts)
-            prog.pool.index_copy_(0, idx, _rotation_values(which, p, B,
-                                                           dtype))
+            _write_rotations(prog, which, p)
         prog.run(psi, inplace=True)
     return psi, saved
 
 
 def _pauli_apply(H: PauliSum, psi: torch.Tensor, out: torch.Tensor):
-    terms = torch.from_numpy(H.term_array().view(np.uint8).copy()).to(
-        psi.device)
+    terms = H.term_array()
     n = H.num_qubits
-    rc = _lib.load().gbsv_pauli_sum_apply(
+    rc = _lib.load().gbsv_pauli_sum_apply_host(
         psi.data_ptr(), out.data_ptr(), _core.complex_code(psi.dtype), n,
-        psi.numel() >> n, terms.data_ptr(), len(H.terms),
+        psi.numel() >> n, terms.ctypes.data, len(terms),
         _core.stream_of(psi.device))
     _lib.check(rc, "pauli_sum_apply")
     return out
@@ -359,9 +385,7 @@ def _backward_sweep(pc, params, H, psi_L, saved, dtype):
     psi.copy_(psi_L)
     _pauli_apply(H, psi, lam)
     grads = torch.zeros(B, pc.num_params, dtype=torch.float64, device=dev)
-    p = params.detach().contiguous()
-    if p.dtype not in (torch.float32, torch.float64):
-        p = p.to(torch.float64)
+    p = _real_params(params)
     L = _lib.load()
     code = _core.complex_code(dtype)
     acode = _core.real_code(p.dtype)
@@ -613,9 +637,7 @@ def _backward_fused(pc, params, H, psi_L, saved, dtype):
     psi.copy_(psi_L)
     _pauli_apply(H, psi, lam)
     grads = torch.zeros(B, pc.num_params, dtype=torch.float64, device=dev)
-    p = params.detach().contiguous()
-    if p.dtype not in (torch.float32, torch.float64):
-        p = p.to(torch.float64)
+    p = _real_params(params)
     L = _lib.load()
     code = _core.complex_code(dtype)
     pcode = _core.real_code(p.dtype)

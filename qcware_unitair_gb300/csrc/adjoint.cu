@@ -19,6 +19,8 @@
 //   and adds the result to grad[s * grad_stride].
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace gbsv {
 
 constexpr int ADJ_THREADS = 256;
@@ -31,9 +33,10 @@ struct PauliTerm {
 };
 
 template <typename R>
-__global__ void __launch_bounds__(256)
-    pauli_apply_kernel(const Cx<R>* psi, Cx<R>* out, uint64_t total, int n,
-                       const PauliTerm* terms, int num_terms) {
+__device__ __forceinline__ void pauli_body(const Cx<R>* psi, Cx<R>* out,
+                                           uint64_t total, int n,
+                                           const PauliTerm* terms,
+                                           int num_terms) {
   __shared__ PauliTerm st[PAULI_MAX_TERMS];
   for (int k = threadIdx.x; k < num_terms; k += blockDim.x) st[k] = terms[k];
   __syncthreads();
@@ -61,58 +64,145 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+template <typename R>
+__global__ void __launch_bounds__(256)
+    pauli_apply_kernel(const Cx<R>* psi, Cx<R>* out, uint64_t total, int n,
+                       const PauliTerm* terms, int num_terms) {
+  pauli_body<R>(psi, out, total, n, terms, num_terms);
+}
+
+// A term as the block kernel holds it: coefficients in the state's type
+// (converting a double costs as much as an FP64 operation, and was half of
+// the kernel's time when every thread did it).
+template <typename R>
+struct PauliRow {
+  uint64_t xmask, zmask;
+  R re, im;
+  int kind;  // 0 a Z string, 1 an X string, 2 other (or a complex factor)
+  int end;   // the run of neighbouring terms of this kind ends here
+};
+
+template <typename R>
+__device__ __forceinline__ R pauli_sign(R v, int neg);
+template <>
+__device__ __forceinline__ float pauli_sign<float>(float v, int neg) {
+  return __uint_as_float(__float_as_uint(v) ^ ((uint32_t)neg << 31));
+}
+template <>
+__device__ __forceinline__ double pauli_sign<double>(double v, int neg) {
+  return __hiloint2double(__double2hiint(v) ^ (neg << 31),
+                          __double2loint(v));
+}
+
+// Parity of e & (low bits of zm) for the V amplitudes of a block.
+__device__ __forceinline__ int pauli_low(int e, int zm) {
+  return (e & 1 & zm) ^ ((e >> 1) & (zm >> 1) & 1);
+}
+
+// b[e] holds amplitude (block start) + e; afterwards amplitude e ^ xm.
+template <typename C, int V>
+__device__ __forceinline__ void pauli_swap(C* b, int xm) {
+  if (xm & 1) {
+#pragma unroll
+    for (int e = 0; e < V; e += 2) {
+      const C t = b[e];
+      b[e] = b[e + 1];
+      b[e + 1] = t;
+    }
+  }
+  if constexpr (V == 4) {
+    if (xm & 2) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const C t = b[e];
+        b[e] = b[e + 2];
+        b[e + 2] = t;
+      }
+    }
+  }
+}
+
 // The same with V consecutive amplitudes (one 32-byte block) per thread:
 // for each term the partner amplitudes y = x ^ xmask of the block are again
-// one 32-byte block, read with one vector load, their order permuted by the
-// low bits of xmask.
+// one 32-byte block, read with vector loads, their order permuted by the
+// low bits of xmask.  Z strings use the thread's own block, and X strings
+// need no signs; the terms are summed in the order given (products with a
+// zero imaginary part left out, which changes no finite sum).
 template <typename R, int V>
-__global__ void __launch_bounds__(256)
-    pauli_apply_block_kernel(const Cx<R>* psi, Cx<R>* out, uint64_t total,
-                             int n, const PauliTerm* terms, int num_terms) {
+__device__ __forceinline__ void pauli_block_body(const Cx<R>* psi,
+                                                 Cx<R>* out, uint64_t total,
+                                                 int n,
+                                                 const PauliTerm* terms,
+                                                 int num_terms) {
   using C = Cx<R>;
-  __shared__ PauliTerm st[PAULI_MAX_TERMS];
-  for (int k = threadIdx.x; k < num_terms; k += blockDim.x) st[k] = terms[k];
+  __shared__ PauliRow<R> st[PAULI_MAX_TERMS];
+  for (int k = threadIdx.x; k < num_terms; k += blockDim.x) {
+    const PauliTerm t = terms[k];
+    const int kind = t.im != 0.0 ? 2 : t.xmask == 0 ? 0 : t.zmask == 0 ? 1 : 2;
+    st[k] = PauliRow<R>{t.xmask, t.zmask, (R)t.re, (R)t.im, kind, 0};
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < num_terms; k += blockDim.x) {
+    int e = k + 1;
+    while (e < num_terms && st[e].kind == st[k].kind) ++e;
+    st[k].end = e;
+  }
   __syncthreads();
   const uint64_t nmask = (uint64_t(1) << n) - 1;
   for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
        i < total; i += (uint64_t)gridDim.x * blockDim.x * V) {
     const uint64_t x = i & nmask;  // block start, low log2(V) bits zero
     const C* p = psi + (i - x);
+    C own[V];
+    load_chunk<V>(p + x, own);
     R ar[V], ai[V];
 #pragma unroll
     for (int e = 0; e < V; ++e) ar[e] = ai[e] = 0;
-    for (int k = 0; k < num_terms; ++k) {
-      const uint64_t xm = st[k].xmask, zm = st[k].zmask;
-      C b[V];
-      load_chunk<V>(p + ((x ^ xm) & ~uint64_t(V - 1)), b);
-      // b[e] holds amplitude ((x ^ xm) & ~(V-1)) + e; amplitude e of this
-      // thread's block needs partner (x + e) ^ xm, i.e. b[e ^ (xm & (V-1))]
-      if (xm & 1) {
+    for (int k = 0; k < num_terms;) {
+      const int end = st[k].end;
+      if (st[k].kind == 0) {
+#pragma unroll 2
+        for (; k < end; ++k) {
+          const uint64_t zm = st[k].zmask;
+          const int par = __popcll(x & zm) & 1;
 #pragma unroll
-        for (int e = 0; e < V; e += 2) {
-          const C t = b[e];
-          b[e] = b[e + 1];
-          b[e + 1] = t;
+          for (int e = 0; e < V; ++e) {
+            const R cr = pauli_sign(st[k].re, par ^ pauli_low(e, (int)zm));
+            ar[e] = fma(cr, own[e].x, ar[e]);
+            ai[e] = fma(cr, own[e].y, ai[e]);
+          }
         }
-      }
-      if constexpr (V == 4) {
-        if (xm & 2) {
-          C t = b[0];
-          b[0] = b[2];
-          b[2] = t;
-          t = b[1];
-          b[1] = b[3];
-          b[3] = t;
-        }
-      }
-      const R re = (R)st[k].re, im = (R)st[k].im;
+      } else if (st[k].kind == 1) {
+#pragma unroll 4
+        for (; k < end; ++k) {
+          const uint64_t xm = st[k].xmask;
+          C b[V];
+          load_chunk<V>(p + ((x ^ xm) & ~uint64_t(V - 1)), b);
+          pauli_swap<C, V>(b, (int)xm);
+          const R re = st[k].re;
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
-        const uint64_t y = (x + e) ^ xm;
-        const R sgn = (__popcll(y & zm) & 1) ? R(-1) : R(1);
-        const R cr = sgn * re, ci = sgn * im;
-        ar[e] = fma(cr, b[e].x, fma(-ci, b[e].y, ar[e]));
-        ai[e] = fma(cr, b[e].y, fma(ci, b[e].x, ai[e]));
+          for (int e = 0; e < V; ++e) {
+            ar[e] = fma(re, b[e].x, ar[e]);
+            ai[e] = fma(re, b[e].y, ai[e]);
+          }
+        }
+      } else {
+        for (; k < end; ++k) {
+          const uint64_t xm = st[k].xmask, zm = st[k].zmask;
+          C b[V];
+          load_chunk<V>(p + ((x ^ xm) & ~uint64_t(V - 1)), b);
+          pauli_swap<C, V>(b, (int)xm);
+          // the sign of amplitude e's partner y = (x + e) ^ xm
+          const int par = __popcll((x ^ xm) & zm) & 1;
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            const int neg = par ^ pauli_low(e, (int)zm);
+            const R cr = pauli_sign(st[k].re, neg);
+            const R ci = pauli_sign(st[k].im, neg);
+            ar[e] = fma(cr, b[e].x, fma(-ci, b[e].y, ar[e]));
+            ai[e] = fma(cr, b[e].y, fma(ci, b[e].x, ai[e]));
+          }
+        }
       }
     }
     C o[V];
@@ -122,6 +212,81 @@ __global__ void __launch_bounds__(256)
       o[e].y = ai[e];
     }
     store_chunk<V>(out + i, o);
+  }
+}
+
+// 31 terms (16 Z, 15 XX) on 32 states of 16 qubits: 108 us with doubles
+// converted per thread and every term complex, 30 us here (the partners'
+// blocks come from L1 and L2).
+template <typename R, int V>
+__global__ void __launch_bounds__(256)
+    pauli_apply_block_kernel(const Cx<R>* psi, Cx<R>* out, uint64_t total,
+                             int n, const PauliTerm* terms, int num_terms) {
+  pauli_block_body<R, V>(psi, out, total, n, terms, num_terms);
+}
+
+// The terms as a kernel parameter: no copy to the device, which from
+// pageable host memory would wait for the stream.
+struct PauliParam {
+  PauliTerm t[PAULI_MAX_TERMS];
+};
+template <typename R, int V>
+__global__ void __launch_bounds__(256)
+    pauli_apply_param_kernel(const Cx<R>* psi, Cx<R>* out, uint64_t total,
+                             int n, const __grid_constant__ PauliParam terms,
+                             int num_terms) {
+  if constexpr (V > 1)
+    pauli_block_body<R, V>(psi, out, total, n, terms.t, num_terms);
+  else
+    pauli_body<R>(psi, out, total, n, terms.t, num_terms);
+}
+
+// Entries of parameterised rotations, written into a program's matrix pool:
+// rotation k of state b with angle theta = 2 half * params[b, pidx] fills
+// pool[off + b nv ..] with its 2x2 (nv = 4) or diagonal (nv = 2), sin and
+// cos in FP64.
+struct RotRec {
+  int32_t gen;   // 0 X, 1 Y, 2 Z
+  int32_t nv;
+  int32_t pidx;
+  int32_t pad_;
+  int64_t off;
+  double half;
+};
+
+template <typename R, typename P>
+__global__ void __launch_bounds__(256)
+    rotation_values_kernel(const P* params, int64_t num_params,
+                           int64_t num_states, const RotRec* recs,
+                           int64_t num_rots, Cx<R>* pool) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= num_states * num_rots) return;
+  // states fastest: neighbouring threads write neighbouring pool entries
+  const int64_t b = i % num_states;
+  const RotRec r = recs[i / num_states];
+  double sn, cs;
+  sincos((double)params[b * num_params + r.pidx] * r.half, &sn, &cs);
+  const R c = (R)cs, s = (R)sn;
+  Cx<R>* o = pool + r.off + b * r.nv;
+  auto put = [&](int k, R x, R y) {
+    o[k].x = x;
+    o[k].y = y;
+  };
+  if (r.gen == 2) {
+    put(0, c, -s);
+    if (r.nv == 2) {
+      put(1, c, s);
+    } else {
+      put(1, 0, 0);
+      put(2, 0, 0);
+      put(3, c, s);
+    }
+  } else {
+    const bool x = r.gen == 0;
+    put(0, c, 0);
+    put(1, x ? R(0) : -s, x ? -s : R(0));
+    put(2, x ? R(0) : s, x ? -s : R(0));
+    put(3, c, 0);
   }
 }
 
@@ -267,10 +432,10 @@ static int adj_parts(int64_t num_states, int64_t pairs, int64_t* len) {
 
 using namespace gbsv;
 
-extern "C" int gbsv_pauli_sum_apply(const void* psi, void* out, int dtype,
-                                    int num_qubits, int64_t num_states,
-                                    const void* terms, int num_terms,
-                                    void* stream) {
+// terms on the device, or (host != NULL) on the host.
+static int pauli_sum(const void* psi, void* out, int dtype, int num_qubits,
+                     int64_t num_states, const void* terms, const void* host,
+                     int num_terms, void* stream) {
   if (dtype != GBSV_C64 && dtype != GBSV_C128)
     return set_error(GBSV_ERR_INVALID_ARG, "state dtype must be complex");
   if (num_qubits < 0 || num_qubits > 62 || num_states < 0 || num_terms < 0)
@@ -279,45 +444,106 @@ extern "C" int gbsv_pauli_sum_apply(const void* psi, void* out, int dtype,
     return set_error(GBSV_ERR_UNSUPPORTED, "more than %d Pauli terms",
                      PAULI_MAX_TERMS);
   if (num_states == 0) return GBSV_OK;
-  if (!psi || !out || (num_terms > 0 && !terms))
+  if (!psi || !out || (num_terms > 0 && !terms && !host))
     return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
   if (psi == out)
     return set_error(GBSV_ERR_INVALID_ARG, "pauli_sum_apply is not in place");
   const uint64_t total = (uint64_t)num_states << num_qubits;
-  uint64_t blocks = (total + 255) / 256;
   const uint64_t cap = (uint64_t)sm_count() * 16;
-  if (blocks > cap) blocks = cap;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // 32-byte blocks need 4 (complex64) / 2 (complex128) amplitudes per state
   // and 32-byte aligned buffers
   const int V = dtype == GBSV_C64 ? 4 : 2;
-  if ((num_qubits >= 2 || (dtype != GBSV_C64 && num_qubits >= 1)) &&
-      (uintptr_t)psi % 32 == 0 && (uintptr_t)out % 32 == 0) {
-    uint64_t vb = (total / V + 255) / 256;
-    const uint64_t cap = (uint64_t)sm_count() * 32;
-    if (vb > cap) vb = cap;
-    if (vb < 1) vb = 1;
-    if (dtype == GBSV_C64)
-      pauli_apply_block_kernel<float, 4><<<(unsigned)vb, 256, 0, st>>>(
-          static_cast<const float2*>(psi), static_cast<float2*>(out), total,
-          num_qubits, static_cast<const PauliTerm*>(terms), num_terms);
+  const bool block =
+      (num_qubits >= 2 || (dtype != GBSV_C64 && num_qubits >= 1)) &&
+      (uintptr_t)psi % 32 == 0 && (uintptr_t)out % 32 == 0;
+  const uint64_t units = block ? total / V : total;
+  uint64_t grid = (units + 255) / 256;
+  if (grid > cap * (block ? 2 : 1)) grid = cap * (block ? 2 : 1);
+  if (grid < 1) grid = 1;
+  const unsigned g = (unsigned)grid;
+  const float2* pf = static_cast<const float2*>(psi);
+  const double2* pd = static_cast<const double2*>(psi);
+  float2* of = static_cast<float2*>(out);
+  double2* od = static_cast<double2*>(out);
+  if (host) {
+    PauliParam par;
+    const PauliTerm* h = static_cast<const PauliTerm*>(host);
+    std::copy(h, h + num_terms, par.t);
+    if (dtype == GBSV_C64 && block)
+      pauli_apply_param_kernel<float, 4>
+          <<<g, 256, 0, st>>>(pf, of, total, num_qubits, par, num_terms);
+    else if (dtype == GBSV_C64)
+      pauli_apply_param_kernel<float, 1>
+          <<<g, 256, 0, st>>>(pf, of, total, num_qubits, par, num_terms);
+    else if (block)
+      pauli_apply_param_kernel<double, 2>
+          <<<g, 256, 0, st>>>(pd, od, total, num_qubits, par, num_terms);
     else
-      pauli_apply_block_kernel<double, 2><<<(unsigned)vb, 256, 0, st>>>(
-          static_cast<const double2*>(psi), static_cast<double2*>(out),
-          total, num_qubits, static_cast<const PauliTerm*>(terms),
-          num_terms);
-    (void)V;
-    return after_launch("pauli_apply_block_kernel");
+      pauli_apply_param_kernel<double, 1>
+          <<<g, 256, 0, st>>>(pd, od, total, num_qubits, par, num_terms);
+    return after_launch("pauli_apply_param_kernel");
   }
-  if (dtype == GBSV_C64)
-    pauli_apply_kernel<float><<<(unsigned)blocks, 256, 0, st>>>(
-        static_cast<const float2*>(psi), static_cast<float2*>(out), total,
-        num_qubits, static_cast<const PauliTerm*>(terms), num_terms);
+  const PauliTerm* t = static_cast<const PauliTerm*>(terms);
+  if (dtype == GBSV_C64 && block)
+    pauli_apply_block_kernel<float, 4>
+        <<<g, 256, 0, st>>>(pf, of, total, num_qubits, t, num_terms);
+  else if (dtype == GBSV_C64)
+    pauli_apply_kernel<float>
+        <<<g, 256, 0, st>>>(pf, of, total, num_qubits, t, num_terms);
+  else if (block)
+    pauli_apply_block_kernel<double, 2>
+        <<<g, 256, 0, st>>>(pd, od, total, num_qubits, t, num_terms);
   else
-    pauli_apply_kernel<double><<<(unsigned)blocks, 256, 0, st>>>(
-        static_cast<const double2*>(psi), static_cast<double2*>(out), total,
-        num_qubits, static_cast<const PauliTerm*>(terms), num_terms);
+    pauli_apply_kernel<double>
+        <<<g, 256, 0, st>>>(pd, od, total, num_qubits, t, num_terms);
   return after_launch("pauli_apply_kernel");
+}
+
+extern "C" int gbsv_pauli_sum_apply(const void* psi, void* out, int dtype,
+                                    int num_qubits, int64_t num_states,
+                                    const void* terms, int num_terms,
+                                    void* stream) {
+  return pauli_sum(psi, out, dtype, num_qubits, num_states, terms, nullptr,
+                   num_terms, stream);
+}
+
+extern "C" int gbsv_pauli_sum_apply_host(
+    const void* psi, void* out, int dtype, int num_qubits, int64_t num_states,
+    const gbsv_pauli_term_t* terms, int num_terms, void* stream) {
+  return pauli_sum(psi, out, dtype, num_qubits, num_states, nullptr,
+                   num_terms > 0 ? terms : nullptr, num_terms, stream);
+}
+
+extern "C" int gbsv_rotation_values(const void* params, int params_dtype,
+                                    int64_t num_params, int64_t num_states,
+                                    const void* rots, int64_t num_rots,
+                                    void* pool, int dtype, void* stream) {
+  if ((dtype != GBSV_C64 && dtype != GBSV_C128) ||
+      (params_dtype != GBSV_F32 && params_dtype != GBSV_F64))
+    return set_error(GBSV_ERR_INVALID_ARG, "bad dtype");
+  if (num_params < 0 || num_states < 0 || num_rots < 0)
+    return set_error(GBSV_ERR_INVALID_ARG, "negative size");
+  if (num_states == 0 || num_rots == 0) return GBSV_OK;
+  if (!params || !rots || !pool)
+    return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
+  const uint64_t grid = ((uint64_t)num_states * num_rots + 255) / 256;
+  if (grid > 0x7fffffffull)
+    return set_error(GBSV_ERR_UNSUPPORTED, "too many rotations");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define GBSV_ROT(R, P)                                                     \
+  rotation_values_kernel<R, P><<<(unsigned)grid, 256, 0, st>>>(            \
+      static_cast<const P*>(params), num_params, num_states,               \
+      static_cast<const RotRec*>(rots), num_rots, static_cast<Cx<R>*>(pool))
+  if (dtype == GBSV_C64) {
+    if (params_dtype == GBSV_F32) GBSV_ROT(float, float);
+    else GBSV_ROT(float, double);
+  } else {
+    if (params_dtype == GBSV_F32) GBSV_ROT(double, float);
+    else GBSV_ROT(double, double);
+  }
+#undef GBSV_ROT
+  return after_launch("rotation_values_kernel");
 }
 
 extern "C" size_t gbsv_adjoint_scratch_bytes(int64_t num_states,
