@@ -569,6 +569,79 @@ int gbsv_adjoint_stage(void* psi, void* lam, int dtype, int num_qubits,
                        double* grad, void* scratch, size_t scratch_bytes,
                        void* stream);
 
+/* The stages above with the ops in register layouts.  One op (64 bytes):
+ * type 0-11 rotation X / Y / Z (type / 4) on register bit type % 4; 12 a Z
+ * rotation on the tile bit t[0] (a mask), 13 on position o[0] outside the
+ * tile; 14 a sign: -1 on the registers in `signs` where all tile bits of
+ * t[0] are set; 15 a fixed diagonal on nq qubits; 16 a 2x2 on k[0], with
+ * nq == 2 controlled by qubit 1 (entries 10, 11, 14, 15 of its 4x4); 17 a
+ * 4x4 on k[0] (MSB), k[1].  A qubit is a register bit (k >= 0), a tile bit
+ * of the thread index (t != 0) or a position outside the tile (o).  Values
+ * at pool + mat; applied where (base & cmask) == cval. */
+typedef struct gbsv_adjoint_regop {
+  int32_t type, slot, nq, signs;
+  int32_t k[2];
+  uint32_t t[2];
+  int32_t o[2];
+  int64_t mat;
+  uint64_t cmask, cval;
+} gbsv_adjoint_regop_t;
+
+/* A layout (32 bytes): ops [first, first + count) run with tile bits rb on a
+ * thread's registers; thread-index bit j is tile bit tb[j]. */
+typedef struct gbsv_adjoint_layout {
+  int8_t rb[4];
+  int8_t tb[12];
+  int32_t first, count;
+  int32_t pad_[2];
+} gbsv_adjoint_layout_t;
+
+/* Register bits per thread of gbsv_adjoint_stage_regs for this dtype.  It
+ * takes tiles of 5 to 8 bits more. */
+int gbsv_adjoint_register_bits(int dtype);
+
+/* Group a stage's ops (gbsv_adjoint_op_t, HOST) into layouts of
+ * register_bits tile bits: ops keep their order except past ops on other
+ * qubits.  pool (HOST, `dtype`; may be NULL) lets controlled gates and signs
+ * be recognised.  regops has room for 4 * num_ops; GBSV_ERR_SCRATCH when
+ * max_layouts is too small, GBSV_ERR_UNSUPPORTED for per-state gates. */
+int gbsv_adjoint_layouts(const void* ops, int num_ops, int tile_qubits,
+                         int register_bits, const void* pool, int dtype,
+                         gbsv_adjoint_regop_t* regops, int* num_regops,
+                         gbsv_adjoint_layout_t* layouts, int max_layouts,
+                         int* num_layouts);
+
+/* cos and sin of half * params[s, pidx] for the total_slots rotations of a
+ * sweep (rots: 16-byte device records int32 pidx, int32 0, double half) into
+ * angles[num_states][total_slots][2] (FP64). */
+int gbsv_adjoint_angles(const void* params, int params_dtype,
+                        int64_t num_params, int64_t num_states,
+                        const void* rots, int64_t total_slots, double* angles,
+                        void* stream);
+
+/* gbsv_adjoint_stage with ops and layouts (device) from
+ * gbsv_adjoint_layouts; the stage's rotations are slots [slot0, slot0 +
+ * num_slots) of angles, and partial[slot - slot0][tile] receives each one's
+ * Im <lam|P|psi> per tile. */
+int gbsv_adjoint_stage_regs(void* psi, void* lam, int dtype, int num_qubits,
+                            int64_t num_states, int tile_qubits,
+                            int contiguous_qubits,
+                            const int32_t* tile_positions, const void* ops,
+                            int num_ops, const void* layouts, int num_layouts,
+                            const void* pool, const double* angles,
+                            int64_t total_slots, int64_t slot0, int num_slots,
+                            double* partial, void* stream);
+
+/* grad[s * num_params + slot_param[k]] += slot_scale[k] * sum of the state's
+ * partials of slot k, for slots [slot0, slot1) (partial[k - slot0][tile]).
+ * prev / next chain the slots of one parameter (-1 ends), so that it has
+ * one writer.  All arrays on the device. */
+int gbsv_adjoint_grad_sum(const double* partial, int64_t slot0, int64_t slot1,
+                          int64_t num_states, int64_t tiles_per_state,
+                          const int32_t* slot_param, const double* slot_scale,
+                          const int32_t* prev, const int32_t* next,
+                          double* grad, int64_t num_params, void* stream);
+
 /* ---- reductions (FP64 accumulation) ----------------------------------- */
 
 /* Scratch bytes a reduction over num_rows rows of length dim needs; 0 means

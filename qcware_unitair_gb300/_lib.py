@@ -138,6 +138,16 @@ SIGNATURES = {
     "gbsv_adjoint_stage": (_I, [_P, _P, _I, _I, _I64, _I, _I,
                                 ctypes.POINTER(_I32), _P, _I, _P, _P, _I,
                                 _I64, _I, _P, _P, _P, _P, _SZ, _P]),
+    "gbsv_adjoint_register_bits": (_I, [_I]),
+    "gbsv_adjoint_layouts": (_I, [_P, _I, _I, _I, _P, _I, _P,
+                                  ctypes.POINTER(_I), _P, _I,
+                                  ctypes.POINTER(_I)]),
+    "gbsv_adjoint_angles": (_I, [_P, _I, _I64, _I64, _P, _I64, _P, _P]),
+    "gbsv_adjoint_stage_regs": (_I, [_P, _P, _I, _I, _I64, _I, _I,
+                                     ctypes.POINTER(_I32), _P, _I, _P, _I,
+                                     _P, _P, _I64, _I64, _I, _P, _P]),
+    "gbsv_adjoint_grad_sum": (_I, [_P, _I64, _I64, _I64, _I64, _P, _P, _P,
+                                   _P, _P, _I64, _P]),
     "gbsv_reduce_scratch_bytes": (_SZ, [_I64, _I64]),
     "gbsv_norm_squared": (_I, [_P, _I, _I64, _I64, _P, _I, _P, _SZ, _P]),
     "gbsv_norm_squared_noalloc": (_I, [_P, _I, _I64, _I64, _P, _I, _P]),

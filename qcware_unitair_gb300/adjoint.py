@@ -455,7 +455,8 @@ def _adjop_dtype():
     return np.dtype(ADJOP_DTYPE.descr + [("g", FG_DTYPE)])
 
 
-def _plan_backward(pc: ParamCircuit, a: int, b: int, dtype, dev, m: int):
+def _plan_backward(pc: ParamCircuit, a: int, b: int, dtype, dev, m: int,
+                   device_ops: bool = True):
     """Fused backward stages for ops [a, b) walked in reverse: a list of
     ("stage", launch args) / ("rot", op) / ("fixed", op) entries.  Depends
     only on the circuit's structure, so it is cached per circuit."""
@@ -520,25 +521,34 @@ def _plan_backward(pc: ParamCircuit, a: int, b: int, dtype, dev, m: int):
         recs["slot"], recs["pidx"], recs["scale"] = slots, pidxs, scales
         args = {
             "c": c, "positions": (ctypes_int32 * m)(*order),
-            "ops": _to_device(recs.view(np.uint8), dev),
-            "num_ops": G,
+            "records": recs, "host_pool": None,
+            "params": (slot_p, slot_s), "num_ops": G,
             "pool": (torch.cat(pool) if pool else torch.zeros(1, dtype=dtype)
                      ).to(dev),
-            "num_slots": len(slot_p),
-            "slot_param": torch.tensor(slot_p or [0], dtype=torch.int32,
-                                       device=dev),
-            "slot_scale": torch.tensor(slot_s or [0.0], dtype=torch.float64,
-                                       device=dev)}
+            "num_slots": len(slot_p)}
+        if device_ops:
+            _device_stage(args, dev)
         out.append(("stage", args))
     return out
 
 
+def _device_stage(args, dev):
+    """What gbsv_adjoint_stage reads from the device."""
+    from .fusion import _to_device
+    slot_p, slot_s = args["params"]
+    args["ops"] = _to_device(args["records"].view(np.uint8), dev)
+    args["slot_param"] = torch.tensor(list(slot_p) or [0], dtype=torch.int32,
+                                      device=dev)
+    args["slot_scale"] = torch.tensor(list(slot_s) or [0.0],
+                                      dtype=torch.float64, device=dev)
+
+
 def _plan_backward_native(pc: ParamCircuit, a: int, b: int, dtype, dev,
-                          m: int):
+                          m: int, device_ops: bool = True):
     """_plan_backward with the stages planned by gbsv_plan (C++) and the
     adjoint records assembled by column: the same stages, records and
     values (one pool for all stages instead of one per stage)."""
-    from .fusion import (DESC_DTYPE, _KIND_CODE, _to_device, native_plan)
+    from .fusion import DESC_DTYPE, _KIND_CODE, native_plan
     n = pc.num_qubits
     ops = list(reversed(pc.ops[a:b]))
     G = len(ops)
@@ -609,20 +619,100 @@ def _plan_backward_native(pc: ParamCircuit, a: int, b: int, dtype, dev,
         ad["pidx"] = np.where(rot, pidxs[idx], 0)
         ad["scale"] = np.where(rot, scales[idx], 0.0)
         ad["g"][~rot] = r[~rot]
-        out.append(("stage", {
+        args = {
             "c": int(op["contiguous"]),
             "positions": (ctypes_int32 * m)(
                 *[int(x) for x in op["positions"][:m]]),
-            "ops": _to_device(ad.view(np.uint8), dev),
+            "records": ad, "host_pool": nat["pool"],
+            "params": (pidxs[idx][rot], scales[idx][rot]),
             "num_ops": count,
             "pool": pool,
-            "num_slots": int(rot.sum()),
-            "slot_param": torch.tensor(pidxs[idx][rot].tolist() or [0],
-                                       dtype=torch.int32, device=dev),
-            "slot_scale": torch.tensor(scales[idx][rot].tolist() or [0.0],
-                                       dtype=torch.float64, device=dev)}))
+            "num_slots": int(rot.sum())}
+        if device_ops:
+            _device_stage(args, dev)
+        out.append(("stage", args))
     assert nxt == G
     return out
+
+
+REGOP_DTYPE = np.dtype([("type", "<i4"), ("slot", "<i4"), ("nq", "<i4"),
+                        ("signs", "<i4"), ("k", "<i4", 2), ("t", "<u4", 2),
+                        ("o", "<i4", 2), ("mat", "<i8"), ("cmask", "<u8"),
+                        ("cval", "<u8")])
+LAYOUT_DTYPE = np.dtype([("rb", "i1", 4), ("tb", "i1", 12), ("first", "<i4"),
+                         ("count", "<i4"), ("pad", "<i4", 2)])
+ANGLE_DTYPE = np.dtype([("pidx", "<i4"), ("pad", "<i4"), ("half", "<f8")])
+
+
+def _register_plan(entries, m: int, dtype, dev):
+    """The register form of a segment's stages: per stage its ops and layouts
+    (byte offsets into one device buffer), the segment's rotations in slot
+    order and the chains that join the slots of one parameter.  None where
+    the stages do not fit it (small tiles, per-state gates)."""
+    from .fusion import _to_device
+    L = _lib.load()
+    code = _core.complex_code(dtype)
+    rb = int(L.gbsv_adjoint_register_bits(code))
+    if not rb + 5 <= m <= rb + 8:
+        return None
+    pieces, size = [], 0
+
+    def add(arr):
+        nonlocal size
+        raw = np.ascontiguousarray(arr).view(np.uint8).reshape(-1)
+        pad = -len(raw) % 64
+        at = size
+        pieces.append(raw)
+        if pad:
+            pieces.append(np.zeros(pad, np.uint8))
+        size += len(raw) + pad
+        return at
+
+    stages, params, scales = [], [], []
+    for kind, st in entries:
+        if kind != "stage":
+            continue
+        G = st["num_ops"]
+        rec = np.ascontiguousarray(st["records"])
+        ops = np.empty(max(4 * G, 1), REGOP_DTYPE)
+        lays = np.zeros(max(G, 1), LAYOUT_DTYPE)
+        hp = st["host_pool"]
+        nops, count = ctypes.c_int(0), ctypes.c_int(0)
+        rc = L.gbsv_adjoint_layouts(
+            rec.ctypes.data, G, m, rb,
+            hp.ctypes.data if hp is not None and len(hp) else None, code,
+            ops.ctypes.data, ctypes.byref(nops), lays.ctypes.data, len(lays),
+            ctypes.byref(count))
+        if rc == _lib.GBSV_ERR_UNSUPPORTED:
+            return None
+        _lib.check(rc, "adjoint_layouts")
+        stages.append((add(ops[:max(nops.value, 1)]), nops.value,
+                       add(lays[:max(count.value, 1)]), count.value,
+                       len(params)))
+        params.extend(int(x) for x in st["params"][0])
+        scales.extend(float(x) for x in st["params"][1])
+    total = len(params)
+    rots = np.zeros(max(total, 1), ANGLE_DTYPE)
+    prev = np.full(max(total, 1), -1, np.int32)
+    nxt = np.full(max(total, 1), -1, np.int32)
+    last = {}
+    for k, p in enumerate(params):
+        rots[k] = (p, 0, 0.5 * scales[k])
+        if p in last:
+            prev[k] = last[p]
+            nxt[last[p]] = k
+        last[p] = k
+    at = {"rots": add(rots), "prev": add(prev), "next": add(nxt),
+          "param": add(np.array(params or [0], np.int32)),
+          "scale": add(np.array(scales or [0.0], np.float64))}
+    most = max([st["num_slots"] for kind, st in entries if kind == "stage"],
+               default=0)
+    return {"buf": _to_device(np.concatenate(pieces), dev),
+            "stages": stages, "at": at, "total": total, "most": most}
+
+
+# gradient partials kept before they are summed (bytes)
+_PARTIAL_BYTES = 64 << 20
 
 
 def _backward_fused(pc, params, H, psi_L, saved, dtype):
@@ -645,7 +735,7 @@ def _backward_fused(pc, params, H, psi_L, saved, dtype):
     segs = pc.segments() if saved else [(0, len(pc.ops))]
     cache = pc.__dict__.setdefault("_adj_cache", {})
     tiles = B << (n - m)
-    scratch = None
+    scratch = partial = None
     both = buf.view(2 * B, N)
     for si in range(len(segs) - 1, -1, -1):
         a, b = segs[si]
@@ -653,10 +743,58 @@ def _backward_fused(pc, params, H, psi_L, saved, dtype):
         if key not in cache:
             host = all(op[0] == "rot" or not op[1].is_cuda
                        for op in pc.ops[a:b])
-            cache[key] = (_plan_backward_native if host else _plan_backward)(
-                pc, a, b, dtype, dev, m)
-        for entry in cache[key]:
-            if entry[0] == "stage":
+            plan = (_plan_backward_native if host else _plan_backward)(
+                pc, a, b, dtype, dev, m, device_ops=False)
+            regs = _register_plan(plan, m, dtype, dev)
+            if regs is None:
+                for kind, st in plan:
+                    if kind == "stage":
+                        _device_stage(st, dev)
+            cache[key] = (plan, regs)
+        entries, regs = cache[key]
+        if regs is not None and regs["total"]:
+            buf0, at = regs["buf"].data_ptr(), regs["at"]
+            total = regs["total"]
+            angles = torch.empty(B, total, 2, dtype=torch.float64, device=dev)
+            rc = L.gbsv_adjoint_angles(
+                p.data_ptr(), pcode, pc.num_params, B, buf0 + at["rots"],
+                total, angles.data_ptr(), stream)
+            _lib.check(rc, "adjoint_angles")
+            room = min(total, max(regs["most"],
+                                  _PARTIAL_BYTES // (8 * tiles)))
+            if partial is None or partial.numel() < room * tiles:
+                partial = torch.empty(room * tiles, dtype=torch.float64,
+                                      device=dev)
+        first = slot = 0  # slots [first, slot) are in partial, unsummed
+
+        def sum_slots():
+            rc = L.gbsv_adjoint_grad_sum(
+                partial.data_ptr(), first, slot, B, 1 << (n - m),
+                buf0 + at["param"], buf0 + at["scale"], buf0 + at["prev"],
+                buf0 + at["next"], grads.data_ptr(), pc.num_params, stream)
+            _lib.check(rc, "adjoint_grad_sum")
+
+        index = 0
+        for entry in entries:
+            if entry[0] == "stage" and regs is not None:
+                st = entry[1]
+                op_at, G, lay_at, nlay, slot = regs["stages"][index]
+                index += 1
+                ns = st["num_slots"]
+                if ns and slot + ns - first > room:
+                    sum_slots()
+                    first = slot
+                base = regs["buf"].data_ptr()
+                rc = L.gbsv_adjoint_stage_regs(
+                    psi.data_ptr(), lam.data_ptr(), code, n, B, m, st["c"],
+                    st["positions"], base + op_at, G, base + lay_at, nlay,
+                    st["pool"].data_ptr(),
+                    angles.data_ptr() if ns else None, regs["total"], slot,
+                    ns, partial.data_ptr() + (slot - first) * tiles * 8
+                    if ns else None, stream)
+                _lib.check(rc, "adjoint_stage")
+                slot += ns
+            elif entry[0] == "stage":
                 st = entry[1]
                 need = st["num_slots"] * (tiles + 2 * B) * 8
                 if need and (scratch is None or scratch.numel() < need):
@@ -692,6 +830,8 @@ def _backward_fused(pc, params, H, psi_L, saved, dtype):
                 _lib.check(rc, "apply_operator")
                 if wide:
                     both.copy_(dst)
+        if slot > first:
+            sum_slots()
         if saved:
             psi.copy_(saved[si])
     return grads

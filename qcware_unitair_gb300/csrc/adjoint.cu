@@ -1016,7 +1016,9 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
   }
 }
 
-// grad[s * P + pidx[slot]] += scale[slot] * sum over the state's tiles
+// grad[s * P + pidx[slot]] += scale[slot] * sum over the state's tiles.  A
+// parameter that drives several slots of the stage has one writer, the block
+// of its first slot, which adds the slots in order.
 __global__ void adjoint_stage_finalize(const double* partial, int num_slots,
                                        uint64_t tiles_per_state,
                                        uint64_t num_tiles,
@@ -1028,19 +1030,30 @@ __global__ void adjoint_stage_finalize(const double* partial, int num_slots,
   const int slot = (int)(item / num_states);
   const uint64_t s = item % num_states;
   if (slot >= num_slots) return;
-  double acc = 0.0;
-  for (uint64_t t = threadIdx.x; t < tiles_per_state; t += blockDim.x)
-    acc += partial[(uint64_t)slot * num_tiles + s * tiles_per_state + t];
+  const int32_t p = pidx[slot];
+  int earlier = 0;
+  for (int k = threadIdx.x; k < slot; k += blockDim.x) earlier |= pidx[k] == p;
+  if (__syncthreads_or(earlier)) return;
   __shared__ double red[8];
+  double total = 0.0;
+  for (int k = slot; k < num_slots; ++k) {
+    if (pidx[k] != p) continue;
+    double acc = 0.0;
+    for (uint64_t t = threadIdx.x; t < tiles_per_state; t += blockDim.x)
+      acc += partial[(uint64_t)k * num_tiles + s * tiles_per_state + t];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    grad[s * num_params + pidx[slot]] += scale[slot] * t;
+    for (int o = 16; o > 0; o >>= 1)
+      acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
+      total += scale[k] * t;
+    }
+    __syncthreads();
   }
+  if (threadIdx.x == 0) grad[s * num_params + p] += total;
 }
 
 }  // namespace gbsv

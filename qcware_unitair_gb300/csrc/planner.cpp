@@ -425,3 +425,236 @@ extern "C" int gbsv_plan(const gbsv_gate_desc_t* gates, int num_gates,
   plan->used_layouts = layouts ? 1 : 0;
   return GBSV_OK;
 }
+
+// ---- register layouts of backward stages ----------------------------------
+namespace {
+
+// gbsv_adjoint_op_t as the stage entry points lay it out
+struct HostAdjOp {
+  int32_t kind, gen, bit, slot, pidx, pad_;
+  double scale;
+  gbsv_fused_gate_t g;
+};
+static_assert(sizeof(HostAdjOp) == 80, "gbsv_adjoint_op_t is 80 bytes");
+
+struct PoolView {
+  const void* p;
+  int dtype;
+  cd at(int64_t i) const {
+    if (dtype == GBSV_C64) {
+      const float* f = static_cast<const float*>(p) + 2 * i;
+      return cd(f[0], f[1]);
+    }
+    const double* f = static_cast<const double*>(p) + 2 * i;
+    return cd(f[0], f[1]);
+  }
+};
+
+// diag(I, U) on two qubits, the first controlling
+bool controlled(const PoolView& v, int64_t mat) {
+  if (!v.p) return false;
+  for (int r = 0; r < 4; ++r)
+    for (int c = 0; c < 4; ++c) {
+      if (r >= 2 && c >= 2) continue;
+      if (v.at(mat + 4 * r + c) != cd(r == c ? 1.0 : 0.0)) return false;
+    }
+  return true;
+}
+
+}  // namespace
+
+extern "C" int gbsv_adjoint_layouts(const void* ops, int num_ops,
+                                    int tile_qubits, int register_bits,
+                                    const void* pool, int dtype,
+                                    gbsv_adjoint_regop_t* regops,
+                                    int* num_regops,
+                                    gbsv_adjoint_layout_t* layouts,
+                                    int max_layouts, int* num_layouts) {
+  const int m = tile_qubits, rb = register_bits;
+  if (num_ops < 0 || !num_layouts || !num_regops || rb < 2 || rb > 4 || m < rb ||
+      m - rb > 12 || (dtype != GBSV_C64 && dtype != GBSV_C128) ||
+      (num_ops > 0 && (!ops || !regops || !layouts)))
+    return GBSV_ERR_INVALID_ARG;
+  const HostAdjOp* in = static_cast<const HostAdjOp*>(ops);
+  const PoolView view{pool, dtype};
+  *num_layouts = *num_regops = 0;
+  struct Info {
+    uint32_t need;     // tile bits that must be register bits
+    uint32_t touch;    // tile bits it acts on
+    bool diag, ctrl;
+  };
+  std::vector<Info> info(num_ops);
+  for (int i = 0; i < num_ops; ++i) {
+    const HostAdjOp& o = in[i];
+    Info& f = info[i];
+    f = Info{0, 0, false, false};
+    auto bit = [](int b) { return b >= 0 ? 1u << b : 0u; };
+    if (o.kind == 0) {
+      f.touch = bit(o.bit);
+      f.diag = o.gen == 2;
+      f.need = f.diag ? 0u : f.touch;
+    } else if (o.g.mat_bstride != 0) {
+      return GBSV_ERR_UNSUPPORTED;
+    } else if (o.g.kind == 2) {
+      f.touch = bit(o.g.b0) | (o.g.nq > 1 ? bit(o.g.b1) : 0u);
+      f.diag = true;
+    } else if (o.g.kind == 1) {
+      f.touch = bit(o.g.b0) | bit(o.g.b1);
+      f.ctrl = controlled(view, o.g.mat);
+      f.need = f.ctrl ? bit(o.g.b1) : f.touch;
+    } else if (o.g.kind == 0) {
+      f.touch = f.need = bit(o.g.b0);
+    } else {
+      return GBSV_ERR_UNSUPPORTED;
+    }
+  }
+  std::vector<char> done(num_ops, 0);
+  int left = num_ops, out = 0;
+  const int classes = dtype == GBSV_C64 ? 4 : 3;  // bank bits of a slot
+  while (left > 0) {
+    if (*num_layouts >= max_layouts) return GBSV_ERR_SCRATCH;
+    gbsv_adjoint_layout_t& L = layouts[(*num_layouts)++];
+    memset(&L, 0, sizeof(L));
+    L.first = out;
+    // take ops in order; one may pass the ops left behind if it shares no
+    // tile bit with them, or only bits on which both are diagonal
+    uint32_t regs = 0, behind = 0, behind_diag = 0;
+    std::vector<int> taken;
+    for (int i = 0; i < num_ops; ++i) {
+      if (done[i]) continue;
+      const Info& f = info[i];
+      const bool free = f.diag ? !(f.touch & behind)
+                               : !(f.touch & (behind | behind_diag));
+      if (free && __builtin_popcount(regs | f.need) <= rb) {
+        regs |= f.need;
+        taken.push_back(i);
+        done[i] = 1;
+        --left;
+      } else if (f.diag) {
+        behind_diag |= f.touch;
+      } else {
+        behind |= f.touch;
+      }
+    }
+    // fill up with tile bits of the most numerous bank classes
+    while (__builtin_popcount(regs) < rb) {
+      int best = -1, most = -1;
+      for (int b = m - 1; b >= 0; --b) {
+        if ((regs >> b) & 1) continue;
+        int cnt = 0;
+        for (int q = b % classes; q < m; q += classes)
+          cnt += !((regs >> q) & 1);
+        if (cnt > most) {
+          most = cnt;
+          best = b;
+        }
+      }
+      regs |= 1u << best;
+    }
+    int reg_of[32], k = 0, t = 0;
+    for (int b = 0; b < 32; ++b) reg_of[b] = -1;
+    for (int b = 0; b < m; ++b)
+      if ((regs >> b) & 1) {
+        reg_of[b] = k;
+        L.rb[k++] = (int8_t)b;
+      }
+    // thread bits: one of each bank class first, then the rest ascending
+    uint32_t used = regs;
+    for (int c = 0; c < classes; ++c)
+      for (int b = c; b < m; b += classes)
+        if (!((used >> b) & 1)) {
+          used |= 1u << b;
+          L.tb[t++] = (int8_t)b;
+          break;
+        }
+    for (int b = 0; b < m; ++b)
+      if (!((used >> b) & 1)) L.tb[t++] = (int8_t)b;
+    for (int i : taken) {
+      const HostAdjOp& o = in[i];
+      gbsv_adjoint_regop_t r;
+      memset(&r, 0, sizeof(r));
+      r.nq = 1;
+      auto place = [&](int j, int b) {
+        r.k[j] = b >= 0 ? reg_of[b] : -1;
+        r.t[j] = b >= 0 && reg_of[b] < 0 ? 1u << b : 0u;
+        r.o[j] = b < 0 ? -1 - b : -1;
+      };
+      if (o.kind == 0) {
+        place(0, o.bit);
+        r.slot = o.slot;
+        r.type = r.k[0] >= 0 ? 4 * o.gen + r.k[0] : o.bit >= 0 ? 12 : 13;
+        regops[out++] = r;
+        continue;
+      }
+      r.mat = o.g.mat;
+      r.cmask = o.g.cmask;
+      r.cval = o.g.cval;
+      if (o.g.kind == 2) {
+        r.nq = o.g.nq;
+        place(0, o.g.b0);
+        if (o.g.nq > 1) place(1, o.g.b1);
+        int minus = 0;  // entries -1
+        bool sign = pool != nullptr;
+        for (int e = 0; sign && e < (1 << r.nq); ++e) {
+          const cd v = view.at(r.mat + e);
+          if (v == cd(-1.0)) minus |= 1 << e;
+          else if (v != cd(1.0)) sign = false;
+        }
+        if (!sign) {
+          r.type = 15;
+          regops[out++] = r;
+          continue;
+        }
+        // the sign as a XOR of products of bits: for each set of qubits
+        // (bit 1 of `set`: qubit 0 where there are two), the parity of the
+        // -1 entries whose index lies within the set
+        for (int set = 0; set < (1 << r.nq); ++set) {
+          int par = 0;
+          for (int e = 0; e < (1 << r.nq); ++e)
+            if ((e & ~set) == 0) par ^= (minus >> e) & 1;
+          if (!par) continue;
+          gbsv_adjoint_regop_t q;
+          memset(&q, 0, sizeof(q));
+          q.type = 14;
+          q.cmask = r.cmask;
+          q.cval = r.cval;
+          uint32_t regsel = 0xFFFFu;
+          static const uint32_t kRegs[4] = {0xAAAAu, 0xCCCCu, 0xF0F0u,
+                                            0xFF00u};
+          for (int j = 0; j < r.nq; ++j) {
+            if (!((set >> (r.nq - 1 - j)) & 1)) continue;
+            if (r.k[j] >= 0) {
+              regsel &= kRegs[r.k[j]];
+            } else if (r.t[j]) {
+              q.t[0] |= r.t[j];
+            } else {
+              q.cmask |= uint64_t(1) << r.o[j];
+              q.cval |= uint64_t(1) << r.o[j];
+            }
+          }
+          q.signs = (int32_t)regsel;
+          regops[out++] = q;
+        }
+        continue;
+      }
+      if (o.g.kind == 0) {
+        r.type = 16;
+        place(0, o.g.b0);
+      } else if (info[i].ctrl) {
+        r.type = 16;
+        r.nq = 2;
+        place(0, o.g.b1);
+        place(1, o.g.b0);
+      } else {
+        r.type = 17;
+        r.nq = 2;
+        place(0, o.g.b0);
+        place(1, o.g.b1);
+      }
+      regops[out++] = r;
+    }
+    L.count = out - L.first;
+  }
+  *num_regops = out;
+  return GBSV_OK;
+}
