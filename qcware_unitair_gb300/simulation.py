@@ -459,6 +459,15 @@ class _ApplyPhase(torch.autograd.Function):
     def backward(ctx, g):
         angles, state, out = ctx.saved_tensors
         need_angles, need_state = ctx.needs_input_grad[:2]
+        if torch.is_grad_enabled():  # create_graph: keep ga differentiable
+            ga = gs = None
+            if need_state:
+                gs = _phase_kernel(-angles, g.contiguous())
+                gs = gs.to(state.dtype).sum_to_size(state.shape)
+            if need_angles:
+                ga = (1j * g * out.conj()).real.to(angles.dtype)
+                ga = ga.sum_to_size(angles.shape)
+            return ga, gs
         # out = exp(-i a) psi  =>  dL/dpsi = exp(i a) g and
         # dL/da = Re(i * g * conj(out)), both from one read of g
         a = _phase_angles(angles).contiguous()

@@ -49,3 +49,27 @@ def test_phase_and_gradients(shape_a, shape_s, da, ds):
         # both factors of dL/da are up to |w| |out|
         size = want.detach().abs().max() + w.abs().max() * s.abs().max()
         assert off <= 8 * eps * rows * size
+
+
+def test_second_derivative_of_the_angles():
+    """d2/da2 of sum_k d_k |(U exp(-i a) psi)_k|^2 through create_graph: the
+    angles' gradient stays differentiable."""
+    rng = np.random.default_rng(5)
+    n = 16
+    a = torch.from_numpy(rng.uniform(-2, 2, n)).to(DEV).requires_grad_()
+    psi = torch.from_numpy(rng.normal(size=n) + 1j * rng.normal(size=n)).to(
+        DEV)
+    u = torch.from_numpy(np.linalg.qr(rng.normal(size=(n, n)) + 1j *
+                                      rng.normal(size=(n, n)))[0]).to(DEV)
+    d = torch.from_numpy(rng.normal(size=n)).to(DEV)
+
+    def energy(x, phase):
+        out = u @ phase(x, psi)
+        return (d * (out.conj() * out).real).sum()
+
+    got, ref = [], []
+    for phase, into in ((ug.apply_phase, got),
+                        (lambda x, s: torch.exp(-1j * x) * s, ref)):
+        g, = torch.autograd.grad(energy(a, phase), a, create_graph=True)
+        into.append(torch.autograd.grad(g[3], a)[0])
+    assert (got[0] - ref[0]).abs().max() <= 1e-12 * n * n
