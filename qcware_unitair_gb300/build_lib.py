@@ -1,10 +1,11 @@
 """Build recipe for libgbsv.so (the CUDA kernels behind the C ABI).
 
 Each ``csrc/*.cu`` translation unit is compiled for sm_103a only, in
-parallel, then linked into ``_build/libgbsv.so`` beside this file.  Nothing
-is installed into site-packages, so the library that Python loads is the
-in-tree one.  A stamp of source hashes skips the rebuild when nothing
-changed.
+parallel, then linked into ``_build/libgbsv.so`` beside this file; the native
+host path (``csrc/host/host.cpp``, against the installed torch) becomes an
+extension module beside it.  Nothing is installed into site-packages, so the
+libraries that Python loads are the in-tree ones.  A stamp of source hashes
+skips the rebuild when nothing changed.
 """
 from __future__ import annotations
 
@@ -14,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -22,6 +24,8 @@ CSRC = PKG_DIR / "csrc"
 INCLUDE = REPO_DIR / "include"
 BUILD_DIR = PKG_DIR / "_build"
 LIB_NAME = "libgbsv.so"
+HOST_MODULE = "_gbsv_host"
+HOST_SOURCE = CSRC / "host" / "host.cpp"
 ARCH_FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr",
@@ -48,17 +52,46 @@ def _cxx() -> str:
 
 def _stamp() -> str:
     h = hashlib.sha256()
-    for p in sorted(list(CSRC.glob("*")) + list(INCLUDE.glob("*.h"))):
+    for p in sorted(list(CSRC.rglob("*")) + list(INCLUDE.glob("*.h"))):
         if p.is_file():
             h.update(p.name.encode())
             h.update(p.read_bytes())
     h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS).encode())
     h.update(os.uname().machine.encode())
+    h.update(f"{_torch_version()} {sys.version}".encode())
     return h.hexdigest()
+
+
+def _torch_version() -> str:
+    import torch
+    return torch.__version__
+
+
+def _host_flags(nvcc: str) -> tuple[list[str], list[str]]:
+    """(compile flags, link flags) of the host module: torch's headers and
+    libraries, the C ABI's library found beside the module."""
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc).resolve().parent.parent
+    inc = [root / "include",
+           root / "include" / "torch" / "csrc" / "api" / "include",
+           Path(sysconfig.get_paths()["include"]), cuda / "include", INCLUDE]
+    abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
+    compile_flags = ["-O2", "-std=c++17", "-fPIC",
+                     f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
+                     *[f"-isystem{i}" for i in inc]]
+    link_flags = [f"-L{BUILD_DIR}", "-lgbsv", "-Wl,-rpath,$ORIGIN",
+                  f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+                  "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    return compile_flags, link_flags
 
 
 def lib_path() -> Path:
     return BUILD_DIR / LIB_NAME
+
+
+def host_path() -> Path:
+    return BUILD_DIR / f"{HOST_MODULE}.so"
 
 
 def build(verbose: bool = False, force: bool = False,
@@ -68,17 +101,20 @@ def build(verbose: bool = False, force: bool = False,
     stamp_file = BUILD_DIR / "stamp.txt"
     stamp = _stamp() + (" ".join(extra_flags) if extra_flags else "")
     out = lib_path()
-    if (not force and out.exists() and stamp_file.exists()
-            and stamp_file.read_text() == stamp):
+    if (not force and out.exists() and host_path().exists()
+            and stamp_file.exists() and stamp_file.read_text() == stamp):
         return out
     nvcc = _nvcc()
     flags = ARCH_FLAGS + NVCC_FLAGS + (extra_flags or []) + [
         f"-I{INCLUDE}", f"-I{CSRC}"]
     objs = []
+    host_compile, host_link = _host_flags(nvcc)
 
     def compile_one(src: Path) -> Path:
         obj = BUILD_DIR / (src.stem + ".o")
-        if src.suffix == ".cpp":  # host-only code
+        if src == HOST_SOURCE:
+            cmd = [_cxx(), *host_compile, "-c", str(src), "-o", str(obj)]
+        elif src.suffix == ".cpp":  # host-only code
             cmd = [_cxx(), "-O3", "-std=c++17", "-fPIC", f"-I{INCLUDE}",
                    f"-I{CSRC}", "-c", str(src), "-o", str(obj)]
         else:
@@ -92,16 +128,23 @@ def build(verbose: bool = False, force: bool = False,
             print(res.stderr, file=sys.stderr)
         return obj
 
-    srcs = sources()
+    srcs = sources() + [HOST_SOURCE]
     with cf.ThreadPoolExecutor(max_workers=min(len(srcs), os.cpu_count() or 4)) as ex:
         objs = list(ex.map(compile_one, srcs))
     tmp = out.with_suffix(".so.tmp")
-    cmd = [nvcc, *ARCH_FLAGS, "-shared", "-o", str(tmp), *map(str, objs),
-           "-lcudart"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"link failed:\n{res.stderr}")
+
+    def link(cmd):
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"link failed:\n{res.stderr}")
+
+    *lib_objs, host_obj = objs
+    link([nvcc, *ARCH_FLAGS, "-shared", "-o", str(tmp),
+          f"-Xlinker=-soname={LIB_NAME}", *map(str, lib_objs), "-lcudart"])
     os.replace(tmp, out)
+    tmp = host_path().with_suffix(".so.tmp")
+    link([_cxx(), "-shared", "-o", str(tmp), str(host_obj), *host_link])
+    os.replace(tmp, host_path())
     stamp_file.write_text(stamp)
     return out
 

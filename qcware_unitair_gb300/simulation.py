@@ -24,7 +24,7 @@ from typing import Iterable, Optional, Sequence, Tuple
 
 import torch
 
-from . import _core, _lib
+from . import _core, _lib, _native
 from .measurement import measure  # noqa: F401  (unitair.simulation.measure)
 from .states import (count_qubits, count_qubits_gate_matrix,
                      StateShapeError)  # noqa: F401  (re-exported errors)
@@ -156,7 +156,7 @@ def _op_grad(gop, plan, tail, target):
 
 
 def _dagger(ops: torch.Tensor) -> torch.Tensor:
-    return ops.conj().transpose(-1, -2).contiguous()
+    return ops.conj().transpose(-1, -2).resolve_conj().contiguous()
 
 
 def _apply_forward(operator, state, qubits, n, k):
@@ -237,12 +237,14 @@ def apply_operator(operator: torch.Tensor, qubits: Iterable[int],
     the most significant bit of the amplitude index.  Returns a new
     contiguous tensor; differentiable with respect to both inputs.
     """
+    out = _native.apply_operator(operator, qubits, state)
+    if out is not None:
+        return out
     n, qubits, k = _validate_apply(operator, qubits, state)
     if torch.is_grad_enabled() and (operator.requires_grad or
                                     state.requires_grad):
         return _ApplyOperator.apply(operator, state, tuple(qubits), n, k)
     # no gradient can flow: the same launch without the autograd Function
-    # (its bookkeeping is most of a small state's per-gate host time)
     return _apply_forward(operator, state, qubits, n, k)[0]
 
 
@@ -382,10 +384,13 @@ class _ApplyAllQubits(torch.autograd.Function):
         return grad_op, gs.reshape(ctx.state_shape), None, None, None
 
 
-def _all_qubits_passes(operator, state, n) -> int:
+def _all_qubits_passes(operator, state, n, each) -> int:
     """Passes of the one-node form, or 0 where the loop over the qubits
-    runs: complex128, fewer than 9 qubits, no states."""
+    runs: complex128, fewer than 9 qubits, no states, per-qubit operators
+    with more batch dims than the state."""
     if not state.numel() or not operator.numel():
+        return 0
+    if each and state.dim() > 1 and operator.dim() - 3 > state.dim() - 1:
         return 0
     return _lib.load().gbsv_all_qubits_passes(
         _core.complex_code(state.dtype), n)
@@ -395,6 +400,9 @@ def apply_all_qubits(operator: torch.Tensor,
                      state: torch.Tensor) -> torch.Tensor:
     """The same single-qubit operator on every qubit
     (operations.py:332-413); batch rules as apply_operator."""
+    out = _native.apply_layer(operator, state, False)
+    if out is not None:
+        return out
     if count_qubits_gate_matrix(operator) != 1:
         raise ValueError(
             "Expected operator on 1 qubit, found a "
@@ -407,7 +415,7 @@ def apply_all_qubits(operator: torch.Tensor,
                            "qubit")
     if torch.is_grad_enabled() and (operator.requires_grad
                                     or state.requires_grad):
-        passes = _all_qubits_passes(operator, state, num_qubits)
+        passes = _all_qubits_passes(operator, state, num_qubits, False)
         if passes:
             return _ApplyAllQubits.apply(operator, state, num_qubits, False,
                                          passes)
@@ -427,6 +435,9 @@ def apply_each_qubit(operators: torch.Tensor,
     the batched per-qubit rotation layer (e.g. RX(angles) with angles of
     shape (*batch, n)).  Batch rules as apply_operator.
     """
+    out = _native.apply_layer(operators, state, True)
+    if out is not None:
+        return out
     num_qubits = count_qubits(state)
     if operators.dim() < 3 or operators.shape[-3] != num_qubits or \
             operators.shape[-1] != 2 or operators.shape[-2] != 2:
@@ -437,7 +448,7 @@ def apply_each_qubit(operators: torch.Tensor,
     _check_dtypes(operators, state)
     if torch.is_grad_enabled() and (operators.requires_grad
                                     or state.requires_grad):
-        passes = _all_qubits_passes(operators, state, num_qubits)
+        passes = _all_qubits_passes(operators, state, num_qubits, True)
         if passes:
             return _ApplyAllQubits.apply(operators, state, num_qubits, True,
                                          passes)
@@ -528,6 +539,9 @@ def apply_phase(angles: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
     """Multiply the k-th amplitude by exp(-i angles_k) with torch
     broadcasting (operations.py:15-42).  float64 angles on a complex64
     state give a complex128 result, as in unitair."""
+    out = _native.apply_phase(angles, state)
+    if out is not None:
+        return out
     return _ApplyPhase.apply(angles, state)
 
 

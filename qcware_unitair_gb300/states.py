@@ -14,7 +14,7 @@ from typing import List, Tuple, Union
 
 import torch
 
-from . import _core, _lib
+from . import _core, _lib, _native
 
 
 class StateLayout(str, enum.Enum):
@@ -302,24 +302,28 @@ class _DiagExpectation(torch.autograd.Function):
 
 def abs_squared(state: torch.Tensor) -> torch.Tensor:
     """|x_k|^2 for every amplitude (innerprod.py:4-26)."""
-    return _AbsSquared.apply(state)
+    out = _native.abs_squared(state)
+    return out if out is not None else _AbsSquared.apply(state)
 
 
 def norm_squared(state: torch.Tensor) -> torch.Tensor:
     """<state|state> per batch entry (innerprod.py:29-46)."""
-    return _NormSquared.apply(state)
+    out = _native.norm_squared(state)
+    return out if out is not None else _NormSquared.apply(state)
 
 
 def diag_expectation_value(diag_values: torch.Tensor,
                            state: torch.Tensor) -> torch.Tensor:
     """sum_k d_k |x_k|^2 with broadcasting (innerprod.py:49-59)."""
-    return _DiagExpectation.apply(diag_values, state)
+    out = _native.diag_expectation_value(diag_values, state)
+    return out if out is not None else _DiagExpectation.apply(diag_values, state)
 
 
 def inner_product(state_1: torch.Tensor, state_2: torch.Tensor):
     """<state_1|state_2>, conjugate-linear in the left entry
     (innerprod.py:62-65)."""
-    return _InnerProduct.apply(state_1, state_2)
+    out = _native.inner_product(state_1, state_2)
+    return out if out is not None else _InnerProduct.apply(state_1, state_2)
 
 
 def norm_squared_fp64(state: torch.Tensor) -> torch.Tensor:
