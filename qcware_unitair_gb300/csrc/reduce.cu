@@ -11,6 +11,7 @@
 // Otherwise every block writes an FP64 partial into caller-provided scratch
 // and a second kernel sums the partials of each row in a fixed order, so the
 // result is deterministic (no atomics).
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -36,13 +37,12 @@ struct Plan {
   int64_t part_len;
 };
 
-// blocks_per_sm: the launching kernel's resident blocks per SM, so that a
-// single row splits into one wave; 16 (the most any reduction kernel keeps
-// resident) gives the largest split, which sizes the scratch
-static Plan make_plan(int64_t rows, int64_t dim, int blocks_per_sm = 16) {
+// The largest split (16 blocks per SM, the most any reduction kernel keeps
+// resident), which sizes the scratch.
+static Plan make_plan(int64_t rows, int64_t dim) {
   Plan p{1, dim};
   if (rows <= 0 || dim <= 0) return p;
-  const int64_t want_blocks = (int64_t)sm_count() * blocks_per_sm;
+  const int64_t want_blocks = (int64_t)sm_count() * 16;
   const int64_t min_len = 8192;
   if (rows >= want_blocks || dim <= min_len) return p;
   int64_t parts = (want_blocks + rows - 1) / rows;
@@ -68,6 +68,34 @@ static int resident_blocks(Kernel kernel) {
     nb = 16;
   }
   return nb < 1 ? 1 : (nb > 16 ? 16 : nb);
+}
+
+// Parts of a row for a kernel with `per_sm` resident blocks: the time goes
+// with waves / parts, so of the splits that fill 1, 2, ... waves without
+// going over, the smallest within 3% of the best.  Rounding up to fill the
+// chip instead leaves a last wave that is nearly empty: 33 rows of 2^20
+// amplitudes in 19 parts are 627 blocks for 608 places, two waves (inner
+// product 127 us; 18 parts 93 us, HBM 83 us).  At most the parts that
+// make_plan sizes the scratch for.
+static Plan make_wave_plan(int64_t rows, int64_t dim, int per_sm) {
+  Plan p{1, dim};
+  const int64_t most = make_plan(rows, dim).parts;
+  if (most <= 1) return p;
+  const int64_t places = (int64_t)sm_count() * per_sm;
+  auto cost = [&](int64_t parts) {
+    return (double)((rows * parts + places - 1) / places) / (double)parts;
+  };
+  int64_t parts = 1;
+  for (int64_t wave = (rows + places - 1) / places; wave <= 16; ++wave) {
+    const int64_t q = std::min(most, places * wave / rows);
+    if (q >= 1 && cost(q) < 0.97 * cost(parts)) parts = q;
+    if (q == most) break;
+  }
+  int64_t len = (dim + parts - 1) / parts;
+  len = (len + 7) & ~int64_t(7);  // keep slices 16-byte aligned for c64
+  p.parts = (int)((dim + len - 1) / len);
+  p.part_len = len;
+  return p;
 }
 
 __device__ __forceinline__ void row_offsets(const RowArgs& a, int64_t row,
@@ -469,9 +497,10 @@ extern "C" int gbsv_norm_squared(const void* state, int dtype,
   if (num_rows == 0) return GBSV_OK;
   if (!out || (dim > 0 && !state))
     return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
-  // two waves of the read-only kernel (measured 2% faster on a 30-qubit
-  // row than one wave)
-  const Plan p = make_plan(num_rows, dim);
+  static const int nb_f = resident_blocks(norm2_kernel<float>);
+  static const int nb_d = resident_blocks(norm2_kernel<double>);
+  const Plan p =
+      make_wave_plan(num_rows, dim, dtype == GBSV_C64 ? nb_f : nb_d);
   int rc = check_scratch(p, num_rows, 0, scratch, scratch_bytes);
   if (!rc) rc = check_grid(p, num_rows);
   if (rc) return rc;
@@ -575,7 +604,8 @@ extern "C" int gbsv_inner_product(const void* a, const void* b, int dtype,
     return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
   static const int nb_f = resident_blocks(inner_kernel<float>);
   static const int nb_d = resident_blocks(inner_kernel<double>);
-  const Plan p = make_plan(ra.rows, dim, dtype == GBSV_C64 ? nb_f : nb_d);
+  const Plan p =
+      make_wave_plan(ra.rows, dim, dtype == GBSV_C64 ? nb_f : nb_d);
   ra.parts = p.parts;
   ra.part_len = p.part_len;
   rc = check_scratch(p, ra.rows, 1, scratch, scratch_bytes);
@@ -616,7 +646,13 @@ extern "C" int gbsv_diag_expectation(const void* diag, int diag_dtype,
   if (ra.rows == 0) return GBSV_OK;
   if (!out || (dim > 0 && (!diag || !state)))
     return set_error(GBSV_ERR_INVALID_ARG, "null pointer");
-  const Plan p = make_plan(ra.rows, dim);
+  static const int nb[4] = {resident_blocks(diag_kernel<float, float>),
+                            resident_blocks(diag_kernel<double, float>),
+                            resident_blocks(diag_kernel<float, double>),
+                            resident_blocks(diag_kernel<double, double>)};
+  const Plan p = make_wave_plan(
+      ra.rows, dim,
+      nb[(diag_dtype == GBSV_F64) + 2 * (state_dtype == GBSV_C128)]);
   ra.parts = p.parts;
   ra.part_len = p.part_len;
   rc = check_scratch(p, ra.rows, 0, scratch, scratch_bytes);
