@@ -181,6 +181,19 @@ int gbsv_apply_phase_grad(const void* angles, int angle_dtype,
                           int out_dtype, const gbsv_bcast_t* bc,
                           void* grad_state, void* grad_angles, void* stream);
 
+/* Gates exp(-i a P) (axis 0 X, 1 Y, 2 Z) for `count` real angles a, element
+ * i at angles + i * stride, in the real type of dtype (GBSV_C64 /
+ * GBSV_C128); out is count dense 2x2 matrices.  Replaces unitair's exp_x,
+ * exp_y, exp_z (src/unitair/gates/gates.py:6-91). */
+int gbsv_rotation_gates(const void* angles, int dtype, int64_t stride,
+                        int64_t count, int axis, void* out, void* stream);
+
+/* Their backward: grad_angles[i] = Re sum grad[i] conj(d out[i] / d a_i),
+ * dense. */
+int gbsv_rotation_gates_grad(const void* angles, int dtype, int64_t stride,
+                             int64_t count, int axis, const void* grad,
+                             void* grad_angles, void* stream);
+
 /* ---- fused gate stages ------------------------------------------------ */
 
 /* One fused-stage gate record (48 bytes, device memory).  kind:

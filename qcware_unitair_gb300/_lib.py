@@ -97,6 +97,8 @@ SIGNATURES = {
                                         _P, _SZ, _P]),
     "gbsv_apply_phase": (_I, [_P, _I, _P, _I, _P, _I, _BC, _P]),
     "gbsv_apply_phase_grad": (_I, [_P, _I, _P, _P, _I, _BC, _P, _P, _P]),
+    "gbsv_rotation_gates": (_I, [_P, _I, _I64, _I64, _I, _P, _P]),
+    "gbsv_rotation_gates_grad": (_I, [_P, _I, _I64, _I64, _I, _P, _P, _P]),
     "gbsv_fused_max_tile_qubits": (_I, [_I]),
     "gbsv_run_stage": (_I, [_P, _P, _I, _I, _I64, _I64, _I, _I,
                             ctypes.POINTER(_I32), _P, _I, _P, _P]),

@@ -14,7 +14,8 @@ import threading
 from . import build_lib
 
 NAMES = ("apply_operator", "apply_layer", "apply_phase", "norm_squared",
-         "abs_squared", "inner_product", "diag_expectation_value")
+         "abs_squared", "inner_product", "diag_expectation_value",
+         "rotation")
 
 _lock = threading.Lock()
 

@@ -769,7 +769,82 @@ PyObject* py_diag(PyObject*, PyObject* const* args, Py_ssize_t na) {
 }
 
 
+// ------------------------------------------------------- rotation gates --
+// The angles as the kernel reads them: a dim of any stride, or dense.
+int64_t angle_stride(const Tensor& a) {
+  return a.dim() == 1 && a.size(0) > 1 ? a.stride(0) : 1;
+}
+
+Tensor run_rotation(const Tensor& a, int axis) {
+  const auto dt = a.scalar_type() == at::kDouble ? at::kComplexDouble
+                                                 : at::kComplexFloat;
+  Sizes shape = a.sizes().vec();
+  shape.insert(shape.end(), {2, 2});
+  Tensor out = at::empty(shape, a.options().dtype(dt));
+  check(gbsv_rotation_gates(a.data_ptr(), complex_code(dt), angle_stride(a),
+                            a.numel(), axis, out.data_ptr(), stream_of(a)),
+        "rotation_gates");
+  return out;
+}
+
+Tensor angles_of(const Tensor& a) {
+  return a.dim() <= 1 && angle_stride(a) >= 0 ? a : a.contiguous();
+}
+
+struct Rotation : public Function<Rotation> {
+  static Variable forward(AutogradContext* ctx, const Variable& angles,
+                          int64_t axis) {
+    ctx->save_for_backward({angles});
+    ctx->saved_data["axis"] = axis;
+    return run_rotation(angles_of(angles), (int)axis);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list gout) {
+    const Tensor angles = ctx->get_saved_variables()[0];
+    const int axis = (int)ctx->saved_data["axis"].toInt();
+    if (at::GradMode::is_enabled()) {  // create_graph: differentiable again
+      const Tensor g = gout[0];
+      const Tensor g00 = g.select(-1, 0).select(-1, 0);
+      const Tensor g01 = g.select(-1, 1).select(-1, 0);
+      const Tensor g10 = g.select(-1, 0).select(-1, 1);
+      const Tensor g11 = g.select(-1, 1).select(-1, 1);
+      const Tensor off = axis == 0   ? -(at::imag(g01) + at::imag(g10))
+                         : axis == 1 ? at::real(g10) - at::real(g01)
+                                     : at::imag(g11) - at::imag(g00);
+      return {angles.cos() * off -
+                  angles.sin() * (at::real(g00) + at::real(g11)),
+              Variable()};
+    }
+    const Tensor a = angles_of(angles.detach()), g = dense_grad(gout[0]);
+    Tensor ga = at::empty(a.sizes(), a.options());
+    check(gbsv_rotation_gates_grad(a.data_ptr(),
+                                   complex_code(g.scalar_type()),
+                                   angle_stride(a), a.numel(), axis,
+                                   g.data_ptr(), ga.data_ptr(), stream_of(a)),
+          "rotation_gates_grad");
+    return {ga, Variable()};
+  }
+};
+
+// (axis, angles): exp(-i a P), complex in the angles' precision.
+PyObject* py_rotation(PyObject*, PyObject* const* args, Py_ssize_t na) {
+  GBSV_CALL
+  if (na != 2 || !PyLong_CheckExact(args[0]) || !plain_context())
+    return none();
+  const long axis = PyLong_AsLong(args[0]);
+  const Tensor* a = unpack(args[1]);
+  if (!a || axis < 0 || axis > 2 || real_code(a->scalar_type()) < 0 ||
+      a->numel() == 0)
+    return none();
+  return THPVariable_Wrap(needs_grad(*a)
+                              ? Rotation::apply(*a, (int64_t)axis)
+                              : run_rotation(angles_of(*a), (int)axis));
+  GBSV_END_CALL
+}
+
 PyMethodDef kMethods[] = {
+    {"rotation",
+     reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_rotation)),
+     METH_FASTCALL, "(axis, angles) -> Tensor or None"},
     {"apply_operator",
      reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_apply_operator)),
      METH_FASTCALL, "(operator, qubits, state) -> Tensor or None"},

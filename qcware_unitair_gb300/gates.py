@@ -9,8 +9,8 @@ Angles may be Python floats (-> (2, 2)) or tensors of any shape
 Divergence: unitair never forwards ``dtype`` to the builder, so its
 rotation gates are complex64 whatever is asked (gate_construction.py:24);
 here an explicit ``dtype`` is honoured.  The default is complex64 as in
-unitair.  Builders are small torch ops: they produce inputs, they are not
-the hot path.
+unitair.  Builders are small torch ops; the rotations of CUDA angles are one
+kernel each way, since a variational step builds them anew.
 """
 from __future__ import annotations
 
@@ -19,6 +19,8 @@ import math
 from typing import Dict, Iterable, Optional, Union
 
 import torch
+
+from . import _native
 
 Angle = Union[torch.Tensor, float]
 
@@ -39,10 +41,22 @@ def _check_complex(dtype):
         raise TypeError(f"gate dtype must be complex, got {dtype}")
 
 
+def _kernel(axis: int, a: torch.Tensor, dtype: torch.dtype):
+    """The gates of CUDA angles in one launch, one more for their gradient;
+    None for other angles (and while torch.compile traces)."""
+    if not a.is_cuda or dtype not in (torch.complex64, torch.complex128) or \
+            torch.compiler.is_compiling():
+        return None
+    return _native.rotation(axis, a)
+
+
 def exp_x(angle: Angle, dtype: torch.dtype = torch.complex64):
     """e^{-i angle X} (gates.py:6-32)."""
     _check_complex(dtype)
     a = _angles(angle, dtype)
+    out = _kernel(0, a, dtype)
+    if out is not None:
+        return out
     c = torch.cos(a).to(dtype)
     s = (torch.sin(a) * 1j).to(dtype)
     return _stack2(c, -s, -s, c)
@@ -52,6 +66,9 @@ def exp_y(angle: Angle, dtype: torch.dtype = torch.complex64):
     """e^{-i angle Y} (gates.py:35-61)."""
     _check_complex(dtype)
     a = _angles(angle, dtype)
+    out = _kernel(1, a, dtype)
+    if out is not None:
+        return out
     c = torch.cos(a).to(dtype)
     s = torch.sin(a).to(dtype)
     return _stack2(c, -s, s, c)
@@ -61,6 +78,9 @@ def exp_z(angle: Angle, dtype: torch.dtype = torch.complex64):
     """e^{-i angle Z} = diag(e^{-i angle}, e^{i angle}) (gates.py:64-91)."""
     _check_complex(dtype)
     a = _angles(angle, dtype)
+    out = _kernel(2, a, dtype)
+    if out is not None:
+        return out
     c = torch.cos(a)
     s = torch.sin(a)
     zero = torch.zeros_like(c).to(dtype)
