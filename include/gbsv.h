@@ -451,6 +451,18 @@ int gbsv_plan(const gbsv_gate_desc_t* gates, int num_gates,
               int min_contiguous, int register_bits, int fuse,
               gbsv_plan_t* plan);
 
+/* Plan gates (all on at most 5 positions) into tensor-core stages: gate i
+ * acts on the amplitude-index positions masks[i] (diagonal[i] != 0: it is
+ * diagonal there) and is assigned stage[i], block[i] (within the stage) and
+ * post[i] (a diagonal applied after its block, on positions the block does
+ * not use).  A stage uses at most 12 positions, the lowest min_contiguous
+ * among them; a block at most 5.  Within a block gates keep the caller's
+ * order.  Gates move past others only where they commute: on disjoint
+ * positions, or both diagonal.  All arrays HOST. */
+int gbsv_plan_tc(const uint64_t* masks, const uint8_t* diagonal,
+                 int num_gates, int min_contiguous, int32_t* stage,
+                 int32_t* block, uint8_t* post);
+
 /* ---- gradients --------------------------------------------------------- */
 
 /* Scratch bytes gbsv_operator_grad needs (0 = none). */

@@ -114,6 +114,7 @@ SIGNATURES = {
     "gbsv_tc_status": (_I, [ctypes.POINTER(_I), _I]),
     "gbsv_plan": (_I, [_P, _I, _P, _I, _I, _I, _I, _I,
                        ctypes.POINTER(Plan)]),
+    "gbsv_plan_tc": (_I, [_P, _P, _I, _I, _P, _P, _P]),
     "gbsv_operator_grad_scratch_bytes": (_SZ, [_I64, _I, _I, _I]),
     "gbsv_operator_grad": (_I, [_P, _P, _I, _I, _I64, _I64,
                                 ctypes.POINTER(_I32), _I, _P, _I, _P, _SZ,

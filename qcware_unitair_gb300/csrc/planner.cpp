@@ -658,3 +658,174 @@ extern "C" int gbsv_adjoint_layouts(const void* ops, int num_ops,
   *num_regops = out;
   return GBSV_OK;
 }
+
+// ---- tensor-core stages -----------------------------------------------------
+namespace {
+
+struct TcGate {
+  uint64_t m;   // positions it acts on
+  bool diag;
+  int id;       // index in the caller's list
+};
+
+constexpr int TCP_BITS = 5, TCP_TILE = 12, TCP_BLOCKS = 64;
+
+// Walks the gates in order and reports what a block on positions B takes:
+// gates inside B, and diagonals disjoint from B (which commute with the
+// block and cost nothing).  A gate may pass those left behind when it shares
+// no position with them, or when both are diagonal there.  f(index, post).
+template <typename F>
+void tc_scan(const std::vector<TcGate>& g, uint64_t B, uint64_t all, F f) {
+  uint64_t dense = 0, diag = 0;  // positions of the gates left behind
+  for (size_t i = 0; i < g.size() && dense != all; ++i) {
+    const TcGate& x = g[i];
+    if (!(x.m & (x.diag ? dense : dense | diag))) {
+      if (!(x.m & ~B)) {
+        f(i, false);
+        continue;
+      }
+      if (x.diag && !(x.m & B)) {
+        f(i, true);
+        continue;
+      }
+    }
+    (x.diag ? diag : dense) |= x.m;
+  }
+}
+
+// Gates a block on B takes in, diagonals a little less (another block may
+// take them along), tile positions it would add to the stage last.
+double tc_value(const std::vector<TcGate>& g, uint64_t B, uint64_t all,
+                uint64_t tile) {
+  double v = 0;
+  tc_scan(g, B, all, [&](size_t i, bool post) {
+    if (!post) v += g[i].diag ? 0.9 : 1.0;
+  });
+  return v - 0.01 * __builtin_popcountll(B & ~tile);
+}
+
+// The best positions found for the next block within `tile` (grown to at
+// most 12): from each gate that can run now, grown by whole gates while that
+// takes more in, then improved by exchanging single positions.
+uint64_t tc_best(const std::vector<TcGate>& g, uint64_t all, uint64_t tile,
+                 double* value) {
+  auto fits = [&](uint64_t B) {
+    return __builtin_popcountll(B) <= TCP_BITS &&
+           __builtin_popcountll(tile | B) <= TCP_TILE;
+  };
+  std::vector<uint64_t> seeds, grow;
+  auto add = [](std::vector<uint64_t>& v, uint64_t m, size_t most) {
+    if (v.size() < most && std::find(v.begin(), v.end(), m) == v.end())
+      v.push_back(m);
+  };
+  uint64_t dense = 0, diag = 0;
+  for (size_t i = 0; i < g.size() && dense != all; ++i) {
+    if (!(g[i].m & (g[i].diag ? dense : dense | diag))) add(seeds, g[i].m, 24);
+    add(grow, g[i].m, 48);
+    (g[i].diag ? diag : dense) |= g[i].m;
+  }
+  uint64_t best = 0;
+  *value = 0;
+  for (uint64_t B : seeds) {
+    if (!fits(B)) continue;
+    double v = tc_value(g, B, all, tile);
+    while (true) {
+      uint64_t next = 0;
+      double nv = 0, gain = 0;
+      for (uint64_t m : grow) {
+        const uint64_t nb = B | m;
+        if (nb == B || !fits(nb)) continue;
+        const double x = tc_value(g, nb, all, tile);
+        const double per = (x - v) / __builtin_popcountll(nb & ~B);
+        if (!next || per > gain || (per == gain && x > nv)) {
+          next = nb;
+          nv = x;
+          gain = per;
+        }
+      }
+      if (!next || nv <= v) break;
+      B = next;
+      v = nv;
+    }
+    if (v > *value) {
+      *value = v;
+      best = B;
+    }
+  }
+  if (!best) return 0;
+  uint64_t reach = 0;
+  for (uint64_t m : grow) reach |= m;
+  for (int round = 0; round < 3; ++round) {
+    uint64_t next = best;
+    double nv = *value;
+    for (uint64_t out = best; out; out &= out - 1)
+      for (uint64_t in = reach & ~best; in; in &= in - 1) {
+        const uint64_t nb = (best & ~(out & -out)) | (in & -in);
+        if (!fits(nb)) continue;
+        const double x = tc_value(g, nb, all, tile);
+        if (x > nv) {
+          next = nb;
+          nv = x;
+        }
+      }
+    if (next == best) break;
+    best = next;
+    *value = nv;
+  }
+  return best;
+}
+
+}  // namespace
+
+// A block costs about twice what a stage costs beside its blocks (0.15 and
+// 0.08 ms on 26 qubits), so the next block stays in the stage's tile unless
+// a new tile would take in half as much again.
+extern "C" int gbsv_plan_tc(const uint64_t* masks, const uint8_t* diagonal,
+                            int num_gates, int min_contiguous, int32_t* stage,
+                            int32_t* block, uint8_t* post) {
+  if (num_gates < 0 || min_contiguous < 0 || min_contiguous > TCP_TILE ||
+      (num_gates > 0 && (!masks || !diagonal || !stage || !block || !post)))
+    return GBSV_ERR_INVALID_ARG;
+  const uint64_t low = (uint64_t(1) << min_contiguous) - 1;
+  std::vector<TcGate> left;
+  uint64_t all = 0;
+  for (int i = 0; i < num_gates; ++i) {
+    const int k = __builtin_popcountll(masks[i]);
+    if (k > TCP_BITS || __builtin_popcountll(low | masks[i]) > TCP_TILE)
+      return GBSV_ERR_UNSUPPORTED;
+    left.push_back(TcGate{masks[i], diagonal[i] != 0, i});
+    all |= masks[i];
+  }
+  uint64_t tile = low;
+  int s = 0, b = 0;  // current stage and its number of blocks
+  while (!left.empty()) {
+    double v = 0, fresh = 0;
+    uint64_t B = b < TCP_BLOCKS ? tc_best(left, all, tile, &v) : 0;
+    if (b > 0) {
+      const uint64_t F = tc_best(left, all, low, &fresh);
+      if (!B || v < 0.65 * fresh) {
+        ++s;
+        b = 0;
+        tile = low;
+        B = F;
+      }
+    }
+    if (!B) B = left[0].m;  // gates on no position, or none found
+    std::vector<char> take(left.size(), 0);
+    tc_scan(left, B, all, [&](size_t i, bool p) {
+      take[i] = 1;
+      const int id = left[i].id;
+      stage[id] = s;
+      block[id] = b;
+      post[id] = p;
+    });
+    std::vector<TcGate> rest;
+    for (size_t i = 0; i < left.size(); ++i)
+      if (!take[i]) rest.push_back(left[i]);
+    if (rest.size() == left.size()) return GBSV_ERR_UNSUPPORTED;
+    left.swap(rest);
+    tile |= B;
+    ++b;
+  }
+  return GBSV_OK;
+}

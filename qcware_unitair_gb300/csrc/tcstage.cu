@@ -29,13 +29,17 @@
 //     1024 * (1024 * 8 + 32) < 2^24 (a unitary's real-form columns have
 //     L1 norm <= 8), so every partial sum is an exact FP32 integer and the
 //     truncating accumulator makes no error;
-//   * Dc = hi * Bl + lo * Bh (the three-product split of Ootomo & Yokota
-//     2022, as one K = 128 product [hi | lo] * [Bl; Bh]) carries the
+//   * Dc = hi * Bl + lo * Bh + lo * Bl (the split of Ootomo & Yokota 2022,
+//     the first two as one K = 128 product [hi | lo] * [Bl; Bh]) carries the
 //     correction, about 2^-11 of D1's magnitude, where the truncation
 //     costs about 2^-34 relative;
 //   * y = (D1 + Dc) / (1024 s), an exact power-of-two scaling.
-// The representation error is about 2^-22 of each column's largest
-// amplitude per block.
+// The last product is a quarter more tensor work on a pipe that is 13%
+// busy, and most of the accuracy: a block's matrix has few exact entries, so
+// each lo * Bl is up to 1/4 and 64 of them about 2^-21 of the column's
+// largest amplitude; with it the fp16 rounding of lo and Bl is left, about
+// 2^-23 (120 gates on 26 qubits in 10 blocks: 3.7e-6 of the state without,
+// 8.5e-7 with it).
 //
 // Diagonal gates whose bits are all outside a block's bits (thread bits,
 // or positions outside the tile) commute with the block.  The host folds
@@ -437,6 +441,11 @@ __global__ void __launch_bounds__(TC_ROLE_THREADS, 2)
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             tc_mma<64>(tmem + 128, tmem + 8 * j, tc_desc(im + 256 * j), j > 0);
+          // lo * Bl
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            tc_mma<64>(tmem + 128, tmem + 32 + 8 * j, tc_desc(im + 256 * j),
+                       1);
         } else {
           fail(1);
         }
