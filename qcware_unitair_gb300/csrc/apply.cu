@@ -915,9 +915,9 @@ __global__ void __launch_bounds__(256)
 
 // k = 3..5 target qubits: one thread per group of 2^k amplitudes (two
 // groups when one matrix serves all states and both fit in 256 bytes of
-// registers).  complex64 5-qubit operators, and 4-qubit ones with a target
-// among the three lowest bits, go to dense_wide_kernel instead
-// (wide_applies); this kernel remains their in-place fallback.  The thread reads its group once (consecutive threads take consecutive groups,
+// registers).  Most complex64 operators with a target among the lowest bits,
+// and 5-qubit ones, go to dense_stream_kernel or dense_wide_kernel instead
+// (stream_applies, wide_applies).  The thread reads its group once (consecutive threads take consecutive groups,
 // so every load instruction of a warp is contiguous when bit 0 is not a
 // target), multiplies by the matrix (in shared memory when one matrix
 // serves all states) and writes the group; in place is safe.
@@ -1236,6 +1236,240 @@ static int apply_small(const void* in, void* out, int dtype, int n,
   if (dtype == GBSV_C64)
     return dispatch_chunk<float>(V, k, nh, rb[0], rb[1], in, out, ops, a, st);
   return dispatch_chunk<double>(V, k, nh, rb[0], rb[1], in, out, ops, a, st);
+}
+
+// ---------------------------------------- 3 to 5 qubits, streamed (c64) ----
+// One complex64 operator on K = 3..5 qubits for every state: warp steps as
+// in dense_c128_stream_kernel.  A step covers 2^(K + 5) amplitudes, its
+// inner index bits the targets and the five lowest others, so it is made of
+// contiguous runs of at least 32 amplitudes (256 bytes).  Lanes copy it
+// lane-contiguously into the warp's slot by 16-byte cp.async, STAGES - 1
+// steps ahead, each takes its group of 2^K amplitudes into registers,
+// multiplies by the matrix (shared memory, broadcast reads) and puts the
+// results back, and the warp stores the step lane-contiguously.  Whatever
+// the targets, global memory sees whole lines; reading groups straight from
+// global memory moves 8 bytes of each 32-byte sector per access when the
+// lowest bits are targets.
+template <int K> struct Step64 {
+  static constexpr int D = 1 << K;
+  static constexpr int INNER = K + 5;
+  static constexpr int BLOCK = 1 << INNER;           // amplitudes per step
+  static constexpr int PIECES = BLOCK / 64;          // 16-byte pieces a lane
+  static constexpr int STAGES = K == 5 ? 2 : 3;
+  static constexpr int THREADS = 256;
+  static constexpr size_t SMEM =
+      (size_t)(THREADS / 32) * STAGES * BLOCK * 8 + (size_t)D * D * 8;
+};
+
+struct Step64Args {
+  uint64_t total_steps;  // num_states << log_steps
+  int log_steps;         // n - INNER
+  int n;
+  int64_t in_stride;
+  int low;               // inner bits 0 .. low - 1 are index bits 0 ..,
+  int nhigh;             // the rest these index bits, ascending
+  int hpos[5];
+  int tb[5];             // inner bit of matrix bit j (j = 0 the lowest)
+  uint64_t lane_off[5];  // offset of inner bits 1 .. 5
+  uint64_t piece_off[16];
+};
+
+// Slot of an inner index: 16-byte units (two amplitudes) XOR-swizzled.
+__device__ __forceinline__ int step64_swz(int l) {
+  const int u = l >> 1;
+  return ((u ^ ((u >> 3) & 7) ^ ((u >> 6) & 7)) << 1) | (l & 1);
+}
+
+template <int K>
+__global__ void __launch_bounds__(256, K == 5 ? 1 : 2)
+    dense_stream_kernel(const float2* in, float2* out, const float2* ops,
+                        const __grid_constant__ Step64Args a) {
+  using W = Step64<K>;
+  constexpr int D = W::D, P = W::STAGES - 1;
+  extern __shared__ __align__(16) float2 step_sm[];
+  float2* const msm = step_sm;  // [D][D]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2* const slot = step_sm + D * D + warp * (W::STAGES * W::BLOCK);
+  for (int i = threadIdx.x; i < D * D; i += W::THREADS) msm[i] = ops[i];
+
+  uint64_t loff = 0;
+#pragma unroll
+  for (int j = 0; j < 5; ++j)
+    if ((lane >> j) & 1) loff += a.lane_off[j];
+  const uint64_t nw = (uint64_t)gridDim.x * (W::THREADS / 32);
+  const uint64_t smask = (uint64_t(1) << a.log_steps) - 1;
+  auto place = [&](uint64_t ws, uint64_t& st) {
+    st = ws >> a.log_steps;
+    uint64_t x = (ws & smask) << a.low;
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+      if (j < a.nhigh) x = insert_zero(x, a.hpos[j]);
+    return x + loff;
+  };
+  auto issue = [&](uint64_t ws, int stage) {
+    if (ws < a.total_steps) {
+      uint64_t st;
+      const uint64_t x = place(ws, st);
+      const float2* src = in + (int64_t)st * a.in_stride + x;
+      float2* const S = slot + stage * W::BLOCK;
+#pragma unroll
+      for (int i = 0; i < W::PIECES; ++i)
+        cp_async16(&S[step64_swz(2 * (lane + 32 * i))], src + a.piece_off[i]);
+    }
+    cp_async_commit();
+  };
+
+  // the lane's group: inner index with the target bits zero, and the slot
+  // part of each matrix bit (the swizzle is linear over XOR)
+  int group = lane;
+  {
+    int t[K];
+#pragma unroll
+    for (int j = 0; j < K; ++j) t[j] = a.tb[j];
+#pragma unroll
+    for (int i = 1; i < K; ++i)
+#pragma unroll
+      for (int j = K - 1; j >= 1; --j)
+        if (t[j - 1] > t[j]) {
+          const int x = t[j];
+          t[j] = t[j - 1];
+          t[j - 1] = x;
+        }
+#pragma unroll
+    for (int j = 0; j < K; ++j) group = (int)insert_zero((uint64_t)group, t[j]);
+  }
+  const int at = step64_swz(group);
+  int tx[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) tx[j] = step64_swz(1 << a.tb[j]);
+  auto member = [&](int b) {
+    int o = at;
+#pragma unroll
+    for (int j = 0; j < K; ++j)
+      if ((b >> j) & 1) o ^= tx[j];
+    return o;
+  };
+
+  uint64_t ws = (uint64_t)blockIdx.x * (W::THREADS / 32) + warp;
+#pragma unroll
+  for (int p = 0; p < P; ++p) issue(ws + p * nw, p);
+  __syncthreads();  // the matrix
+  for (int k = 0; ws < a.total_steps; ++k, ws += nw) {
+    float2* const S = slot + (k % W::STAGES) * W::BLOCK;
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(P - 1) : "memory");
+    __syncwarp();  // every lane's copies of this step have landed, and every
+                   // lane is done with the slot reused below
+    issue(ws + P * nw, (k + P) % W::STAGES);
+    float2 x[D];
+#pragma unroll
+    for (int b = 0; b < D; ++b) x[b] = S[member(b)];
+    // rows in fours: four independent sums hide the FMA latency
+#pragma unroll 1
+    for (int r = 0; r < D; r += 4) {
+      float2 acc[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int b = 0; b < D; b += 2)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 m =
+              *reinterpret_cast<const float4*>(&msm[(r + q) * D + b]);
+          acc[q] = cmad(make_float2(m.x, m.y), x[b], acc[q]);
+          acc[q] = cmad(make_float2(m.z, m.w), x[b + 1], acc[q]);
+        }
+      const int row = at ^ (r & 4 ? tx[2] : 0) ^
+                      (K > 3 && (r & 8) ? tx[K > 3 ? 3 : 0] : 0) ^
+                      (K > 4 && (r & 16) ? tx[K > 4 ? 4 : 0] : 0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        S[row ^ (q & 1 ? tx[0] : 0) ^ (q & 2 ? tx[1] : 0)] = acc[q];
+    }
+    __syncwarp();
+    uint64_t st;
+    const uint64_t xb = place(ws, st);
+    float2* dst = out + (st << a.n) + xb;
+#pragma unroll
+    for (int i = 0; i < W::PIECES; ++i)
+      __stcs(reinterpret_cast<float4*>(dst + a.piece_off[i]),
+             *reinterpret_cast<const float4*>(
+                 &S[step64_swz(2 * (lane + 32 * i))]));
+  }
+}
+
+template <int K>
+static int launch_stream(const float2* in, float2* out, const float2* ops,
+                         int n, int64_t num_states, int64_t in_stride,
+                         const int* pos, cudaStream_t st) {
+  using W = Step64<K>;
+  Step64Args a{};
+  a.n = n;
+  a.log_steps = n - W::INNER;
+  a.total_steps = (uint64_t)num_states << a.log_steps;
+  a.in_stride = in_stride;
+  uint64_t inner_mask = 0;
+  for (int j = 0; j < K; ++j) inner_mask |= uint64_t(1) << pos[j];
+  for (int b = 0; __builtin_popcountll(inner_mask) < W::INNER; ++b)
+    inner_mask |= uint64_t(1) << b;
+  int inner[W::INNER], q = 0;
+  for (int b = 0; b < n; ++b)
+    if ((inner_mask >> b) & 1) {
+      for (int j = 0; j < K; ++j)
+        if (pos[j] == b) a.tb[K - 1 - j] = q;
+      inner[q++] = b;
+    }
+  while (a.low < W::INNER && inner[a.low] == a.low) ++a.low;
+  a.nhigh = W::INNER - a.low;
+  for (int j = 0; j < a.nhigh; ++j) a.hpos[j] = inner[a.low + j];
+  for (int j = 0; j < 5; ++j) a.lane_off[j] = uint64_t(1) << inner[1 + j];
+  for (int i = 0; i < W::PIECES; ++i)
+    for (int j = 0; j + 6 < W::INNER; ++j)
+      if ((i >> j) & 1) a.piece_off[i] += uint64_t(1) << inner[6 + j];
+  // the shared-memory opt-in and the occupancy, once per device
+  static std::atomic<int> per_sm_of[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::atomic<int>& per_sm = per_sm_of[dev & 63];
+  int bps = per_sm.load(std::memory_order_relaxed);
+  if (bps == 0) {
+    cudaError_t e = cudaFuncSetAttribute(
+        dense_stream_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (int)W::SMEM);
+    if (e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+          &bps, dense_stream_kernel<K>, W::THREADS, W::SMEM);
+    if (e != cudaSuccess || bps < 1)
+      return set_error(GBSV_ERR_CUDA, "dense_stream_kernel<%d> setup: %s", K,
+                       cudaGetErrorString(e));
+    per_sm.store(bps, std::memory_order_relaxed);
+  }
+  const uint64_t warps = W::THREADS / 32;
+  uint64_t blocks = (a.total_steps + warps - 1) / warps;
+  const uint64_t cap = (uint64_t)sm_count() * bps;
+  if (blocks > cap) blocks = cap;
+  dense_stream_kernel<K>
+      <<<(unsigned)blocks, W::THREADS, W::SMEM, st>>>(in, out, ops, a);
+  return after_launch("dense_stream_kernel");
+}
+
+// Whether dense_stream_kernel takes this operator: aligned states of at
+// least one step under one operator.  With 3 or 4 targets all above bit 4 a
+// warp of dense_group_kernel reads whole lines as it is and needs no shared
+// memory.  26 qubits, us, group (5 qubits: wide) against streamed:
+//   3 qubits  high 164 / 172   low 367 / 165   mixed 193 / 163
+//   4 qubits  high 217 / 226   low 329 / 228   mixed 329 / 231
+//   5 qubits  high 442 / 390   low 486 / 402   mixed 488 / 404
+// (HBM 160; the FMAs at the rate of three distinct registers each 90, 175
+// and 350).
+static bool stream_applies(const void* in, const void* out, int dtype, int n,
+                           int k, const int* pos, int64_t num_states,
+                           int64_t in_stride, int64_t op_stride,
+                           bool in_place) {
+  if (dtype != GBSV_C64 || k < 3 || k > 5 || n < k + 5 || op_stride != 0 ||
+      (uintptr_t)in % 16 || (uintptr_t)out % 16 || in_stride % 2 ||
+      (in_place && num_states > 1 && in_stride != (int64_t(1) << n)))
+    return false;
+  return k == 5 || *std::min_element(pos, pos + k) < 5;
 }
 
 // ------------------------------------------------ wide operators (c64) ----
@@ -1636,6 +1870,15 @@ static int apply_generic(const void* in, void* out, int dtype, int n,
                          int64_t num_states, int64_t in_stride,
                          const void* ops, int64_t op_stride, const int* pos,
                          int k, cudaStream_t st) {
+  if (stream_applies(in, out, dtype, n, k, pos, num_states, in_stride,
+                     op_stride, in == out)) {
+    const float2* i = static_cast<const float2*>(in);
+    float2* o = static_cast<float2*>(out);
+    const float2* m = static_cast<const float2*>(ops);
+    if (k == 3) return launch_stream<3>(i, o, m, n, num_states, in_stride, pos, st);
+    if (k == 4) return launch_stream<4>(i, o, m, n, num_states, in_stride, pos, st);
+    return launch_stream<5>(i, o, m, n, num_states, in_stride, pos, st);
+  }
   if (wide_applies(dtype, n, k, num_states, in_stride, op_stride, in == out,
                    pos))
     return apply_wide(in, out, n, num_states, in_stride, ops, op_stride, pos,
