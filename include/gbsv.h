@@ -377,6 +377,12 @@ int gbsv_phase_flip(const void* in, void* out, int dtype, int num_qubits,
                     int64_t num_states, const void* masks, int num_masks,
                     void* stream);
 
+/* gbsv_phase_flip with the masks in HOST memory: they travel as a kernel
+ * parameter. */
+int gbsv_phase_flip_host(const void* in, void* out, int dtype,
+                         int num_qubits, int64_t num_states,
+                         const uint64_t* masks, int num_masks, void* stream);
+
 /* X on `target` where every control qubit (HOST array) is 1; in place
  * allowed.  unitair's multi_controlled_x (operations.py:786-805) builds it
  * as H, multi_controlled_z, H. */

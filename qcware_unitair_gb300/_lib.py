@@ -133,6 +133,8 @@ SIGNATURES = {
     "gbsv_permute_qubits": (_I, [_P, _P, _I, _I, _I64,
                                  ctypes.POINTER(_I32), _P]),
     "gbsv_phase_flip": (_I, [_P, _P, _I, _I, _I64, _P, _I, _P]),
+    "gbsv_phase_flip_host": (_I, [_P, _P, _I, _I, _I64,
+                                  ctypes.POINTER(ctypes.c_uint64), _I, _P]),
     "gbsv_multi_controlled_x": (_I, [_P, _P, _I, _I, _I64,
                                      ctypes.POINTER(_I32), _I, _I, _P]),
     "gbsv_sample_scratch_bytes": (_SZ, [_I64]),

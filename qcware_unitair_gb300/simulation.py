@@ -19,6 +19,7 @@ extra dim raises RuntimeError.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import Iterable, Optional, Sequence, Tuple
 
@@ -669,11 +670,10 @@ def _phase_flip(state: torch.Tensor, masks) -> torch.Tensor:
     out = torch.empty_like(s)
     if s.numel() == 0:
         return out
-    host = torch.tensor([int(m) for m in masks] or [0], dtype=torch.int64)
-    dev_masks = host.pin_memory().to(s.device, non_blocking=True)
-    rc = _lib.load().gbsv_phase_flip(
-        s.data_ptr(), out.data_ptr(), code, n, s.numel() >> n,
-        dev_masks.data_ptr(), len(masks), _core.stream_of(s.device))
+    host = (ctypes.c_uint64 * max(len(masks), 1))(*masks)
+    rc = _lib.load().gbsv_phase_flip_host(
+        s.data_ptr(), out.data_ptr(), code, n, s.numel() >> n, host,
+        len(masks), _core.stream_of(s.device))
     _lib.check(rc, "phase_flip")
     return out
 
