@@ -195,6 +195,7 @@ struct AqPlan {
   int64_t lstride; // amplitudes between a thread's registers: first layout,
   int64_t sstride; // last layout where it stores directly, 0 where the tile
                    // goes back to the first layout for the store
+  uint32_t slot[3][16];  // byte offset of register i's slot part, layout k
 };
 
 // One pass.  256 threads hold the CTA's 4096 amplitudes, 16 each, with four
@@ -209,16 +210,19 @@ struct AqPlan {
 // copies missed the instruction cache: 2.6 of 9 stall cycles per issue) and
 // every global address is a base plus i strides.  One layer on 256 states
 // of 16 qubits (134 MB): 16 passes of the gate kernel 655 us, two passes
-// with a kernel per tile size and unrolled layouts 165 us, here 143 us (HBM
-// alone 80 us); on 7 states of 20 qubits 315, 66 and 61 us.
+// with a kernel per tile size and unrolled layouts 165 us, here 108 us (HBM
+// alone 80 us); on 7 states of 20 qubits 315, 66 and 54 us, 145 and 78 us
+// where the operator has no zero part.  Two-lane FMAs, which halve the FMA
+// instructions, were no faster: the lanes of a complex product cross, and
+// the moves cost what the FMAs gave.
 __global__ void __launch_bounds__(AQ_THREADS, 4)
     allq_kernel(const float2* in, float2* out, const float2* ops,
                 const __grid_constant__ AllqArgs a,
                 const __grid_constant__ AqPlan w) {
   __shared__ float2 sm[1 << AQ_TILE];
+  __shared__ AqOp sop[AQ_TILE];  // of tile bit b, where the CTA has one state
   const int sub = threadIdx.x >> (w.m - 4);
   const int u = threadIdx.x & ((1 << (w.m - 4)) - 1);
-  float2* const S = sm + (sub << w.m);
   uint64_t base, s;
   bool live = true;
   if (w.m == AQ_TILE) {
@@ -232,28 +236,46 @@ __global__ void __launch_bounds__(AQ_THREADS, 4)
   if (live) ops += (int64_t)s * a.op_stride;
 
   float2 r[16];
-  {
+  if (live) {
     const float2* src = in + (int64_t)s * a.in_stride + first;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      r[i] = live ? __ldcs(src) : make_float2(0.f, 0.f);
+      r[i] = __ldcs(src);
       src += w.lstride;
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) r[i] = make_float2(0.f, 0.f);
   }
-  // slot of tile index (thread part) | (register part): the swizzle is
-  // linear over XOR
+  // One load and one look at an operator's kind per CTA instead of one per
+  // thread and layout, behind the amplitudes' loads: 16 qubits x 256 with an
+  // operator per qubit 126 -> 108 us.  Smaller states have too many
+  // operators in a CTA for that.
+  const bool staged = w.m == AQ_TILE;
+  if (staged) {
+    if (threadIdx.x < AQ_TILE && ((a.mask >> threadIdx.x) & 1))
+      sop[threadIdx.x] = aq_load_op(ops, a, aq_pos(a, threadIdx.x));
+    __syncthreads();
+  }
+  // byte offset of the slot of tile index (thread part) | (register part):
+  // the swizzle is linear over XOR
   auto slot = [&](int rb) {
     const int lo = (1 << rb) - 1;
-    return aq_swz((u & lo) | ((u & ~lo) << 4));
+    return (uint32_t)((sub << w.m) + aq_swz((u & lo) | ((u & ~lo) << 4))) * 8;
+  };
+  auto at_slot = [&](uint32_t off) -> float2& {
+    return *reinterpret_cast<float2*>(reinterpret_cast<char*>(sm) + off);
   };
 #pragma unroll 1
   for (int k = 0;; ++k) {
     const int bits = w.bits[k];
-    AqOp o = aq_load_op(ops, a, w.pos[k] + 3 < a.n ? w.pos[k] + 3 : a.n - 1);
+    AqOp o;
+    if (!staged) o = aq_load_op(ops, a, w.pos[k]);
     const bool finite = aq_finite(r);
 #define AQ_BIT(J)                                                      \
   if ((bits >> J) & 1) {                                               \
-    if (a.op_qstride) o = aq_load_op(ops, a, w.pos[k] + J);            \
+    if (staged) o = sop[w.rb[k] + J];                                  \
+    else if (a.op_qstride) o = aq_load_op(ops, a, w.pos[k] + J);       \
     aq_apply<J>(r, o, finite ? o.kind : AQ_FULL);                      \
   }
     AQ_BIT(3)
@@ -265,14 +287,14 @@ __global__ void __launch_bounds__(AQ_THREADS, 4)
     if (last && (k == 0 || w.sstride)) break;
     // to the next layout, or back to the first for the store.  Each thread
     // writes the slots it read last, so one barrier is enough.
-    int at = slot(w.rb[k]);
+    uint32_t at = slot(w.rb[k]);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) S[at ^ aq_swz(i << w.rb[k])] = r[i];
+    for (int i = 0; i < 16; ++i) at_slot(at ^ w.slot[k][i]) = r[i];
     __syncthreads();
-    const int to = last ? w.rb[0] : w.rb[k + 1];
-    at = slot(to);
+    const int to = last ? 0 : k + 1;
+    at = slot(w.rb[to]);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) r[i] = S[at ^ aq_swz(i << to)];
+    for (int i = 0; i < 16; ++i) r[i] = at_slot(at ^ w.slot[to][i]);
     if (last) break;
   }
   if (!live) return;
@@ -301,6 +323,14 @@ static int aq_passes(int n) {
   return n <= AQ_TILE ? 1 : 1 + (n - AQ_TILE + AQ_HIGH - 1) / AQ_HIGH;
 }
 
+static void aq_slots(AqPlan* w) {
+  for (int k = 0; k < w->rounds; ++k)
+    for (int i = 0; i < 16; ++i) {
+      const int l = i << w->rb[k];
+      w->slot[k][i] = (uint32_t)(l ^ ((l >> 4) & 15)) * 8;
+    }
+}
+
 static AqPlan aq_pass(AllqArgs* a, int pass) {
   const int m = std::min(a->n, AQ_TILE);
   AqPlan w{};
@@ -318,6 +348,7 @@ static AqPlan aq_pass(AllqArgs* a, int pass) {
       w.bits[w.rounds] = (1 << (done - rb)) - 1;
       done = rb;
     }
+    aq_slots(&w);
     return w;
   }
   const int low = AQ_TILE + (up - 1) * AQ_HIGH;
@@ -337,6 +368,7 @@ static AqPlan aq_pass(AllqArgs* a, int pass) {
     w.bits[1] = (a->mask >> 4) & 15;
     w.sstride = int64_t(1) << a->p;
   }
+  aq_slots(&w);
   return w;
 }
 
