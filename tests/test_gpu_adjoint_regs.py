@@ -77,3 +77,39 @@ def test_register_stage_sums_more_slots_than_fit_at_once(monkeypatch):
     monkeypatch.setattr(ad, "_PARTIAL_BYTES", 0)  # one stage at a time
     got = ad._backward_fused(pc, params, H, psi_L, saved, torch.complex64)
     assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n,layers,checkpoints", [(3, 1, True), (9, 5, True),
+                                                  (13, 4, True),
+                                                  (13, 4, False)])
+def test_sweep_in_its_own_states_equals_the_copying_one(n, layers, checkpoints,
+                                                        dtype):
+    """The public call lets the sweep run in the forward pass's own states;
+    the same kernels on copies give the same bits, also with a psi0, which
+    keeps the copies."""
+    B = 3
+    pc = ad.hardware_efficient_ansatz(n, layers)
+    if layers == 5:  # a gate outside the stages
+        a = np.random.default_rng(n).normal(size=(8, 8))
+        pc.gate(torch.from_numpy(np.linalg.qr(a)[0] + 0j), [0, n // 2, n - 1])
+    H = ad.PauliSum(n).z(0).xx(0, n - 1, 0.5)
+    g = torch.Generator().manual_seed(n)
+    params = torch.randn(B, pc.num_params, generator=g,
+                         dtype=torch.float64).to(DEV)
+    psi_L, saved = ad._forward(pc, params, dtype, None, checkpoints)
+    ref = ad._backward_fused(pc, params, H, psi_L, saved, dtype)
+    vals, got = ad.expectation_and_grad(pc, params, H, dtype=dtype,
+                                        checkpoints=checkpoints)
+    assert torch.equal(got, ref)
+    assert torch.equal(vals, ad.pauli_expectation(H, psi_L))
+    p = params.clone().requires_grad_()
+    out = ad.expectation(pc, p, H, dtype=dtype, checkpoints=checkpoints)
+    assert torch.equal(out.detach(), vals)
+    out.sum().backward()
+    assert torch.equal(p.grad, ref)
+    psi0 = torch.zeros(B, 2 ** n, dtype=dtype, device=DEV)
+    psi0[:, 0] = 1
+    _, again = ad.expectation_and_grad(pc, params, H, psi0=psi0, dtype=dtype,
+                                       checkpoints=checkpoints)
+    assert torch.equal(again, ref)
