@@ -2185,10 +2185,12 @@ struct PhaseRowArgs {
 // batch of angles.  A block takes 1024 columns of up to eight rows and finds
 // the row offsets once (one element at a time, their 64-bit divisions cost
 // more than the element); a phase factor is formed once where the rows
-// share the angles.  7 states of 20 qubits, one set of angles: 43 us by
-// element, 25 us here (HBM: 18 us without the L2).
-template <typename RA, typename RS, typename RO>
-__global__ void __launch_bounds__(256)
+// share the angles.  VEC: complex64 two amplitudes at a time, at a register
+// count that lets five blocks share an SM (four 22 us, six 23 us, spilling).
+// 7 states of 20 qubits, one set of angles: 43 us by element, 25 us by rows,
+// 20.5 us in pairs (HBM: 18 us without the L2).
+template <typename RA, typename RS, typename RO, bool VEC>
+__global__ void __launch_bounds__(256, sizeof(RA) == 4 && VEC ? 5 : 1)
     phase_rows_kernel(const RA* ang, const Cx<RS>* psi, Cx<RO>* out,
                       PhaseRowArgs a) {
   __shared__ int64_t off_a[PHASE_ROWS], off_b[PHASE_ROWS];
@@ -2201,14 +2203,28 @@ __global__ void __launch_bounds__(256)
               &off_b[threadIdx.x]);
   __syncthreads();
   const int64_t s0 = a.p.sa[a.p.ndim - 1], s1 = a.p.sb[a.p.ndim - 1];
-  const uint64_t c0 = cb * PHASE_COLS + threadIdx.x;
+  // the thread's columns: every 256th, or two neighbouring ones in each half
+  auto column = [&](int k) -> uint64_t {
+    return cb * PHASE_COLS +
+           (VEC ? 2 * threadIdx.x + 512 * (k >> 1) + (k & 1)
+                : threadIdx.x + 256 * k);
+  };
   PhaseFactor<RA> f[4];
   Cx<RS> v[4], next[4];
   auto load = [&](int r, Cx<RS>* x) {
+    if constexpr (VEC) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint64_t c = c0 + 256 * k;
-      if (c < a.cols) x[k] = psi[off_b[r] + (int64_t)c * s1];
+      for (int k = 0; k < 4; k += 2) {
+        if (column(k) >= a.cols) continue;
+        const float4 w =
+            *reinterpret_cast<const float4*>(psi + off_b[r] + column(k));
+        x[k] = make_float2(w.x, w.y);
+        x[k + 1] = make_float2(w.z, w.w);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (column(k) < a.cols) x[k] = psi[off_b[r] + (int64_t)column(k) * s1];
     }
   };
   load(0, v);
@@ -2216,17 +2232,25 @@ __global__ void __launch_bounds__(256)
     if (r + 1 < nrows) load(r + 1, next);  // in flight during this row
     if (r == 0 || !a.shared) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint64_t c = c0 + 256 * k;
-        if (c < a.cols)
-          f[k] = phase_factor(ang[off_a[r] + (int64_t)c * s0], a.p.df);
-      }
+      for (int k = 0; k < 4; ++k)
+        if (column(k) < a.cols)
+          f[k] = phase_factor(ang[off_a[r] + (int64_t)column(k) * s0], a.p.df);
     }
     Cx<RO>* dst = out + (row0 + r) * a.cols;
+    if constexpr (VEC) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint64_t c = c0 + 256 * k;
-      if (c < a.cols) dst[c] = phase_times<RA, RS, RO>(f[k], v[k]);
+      for (int k = 0; k < 4; k += 2) {
+        if (column(k) >= a.cols) continue;
+        const float2 x = phase_times<RA, RS, RO>(f[k], v[k]);
+        const float2 y = phase_times<RA, RS, RO>(f[k + 1], v[k + 1]);
+        *reinterpret_cast<float4*>(dst + column(k)) =
+            make_float4(x.x, x.y, y.x, y.y);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (column(k) < a.cols)
+          dst[column(k)] = phase_times<RA, RS, RO>(f[k], v[k]);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = next[k];
@@ -2301,6 +2325,18 @@ static PhaseRowArgs phase_row_args(const PhaseArgs& a, int most_rows) {
   return r;
 }
 
+// Whether the rows can move two complex64 amplitudes at a time: an even
+// number of neighbouring columns, and every row at a 16-byte address.
+static bool phase_pairs(const PhaseArgs& a, const void* psi, const void* out) {
+  if (a.sb[a.ndim - 1] != 1 || a.shape[a.ndim - 1] % 2 ||
+      ((reinterpret_cast<uintptr_t>(psi) | reinterpret_cast<uintptr_t>(out)) &
+       15))
+    return false;
+  for (int d = 0; d + 1 < a.ndim; ++d)
+    if (a.sb[d] % 2) return false;
+  return true;
+}
+
 template <typename RA, typename RS, typename RO>
 static int launch_phase(const void* ang, const void* psi, void* out,
                         const PhaseArgs& a, cudaStream_t st) {
@@ -2308,7 +2344,15 @@ static int launch_phase(const void* ang, const void* psi, void* out,
     const PhaseRowArgs r = phase_row_args(a, PHASE_ROWS);
     const uint64_t grid = r.col_blocks * ((r.rows + r.per - 1) / r.per);
     if (grid <= 0x7fffffffull) {
-      phase_rows_kernel<RA, RS, RO><<<(unsigned)grid, 256, 0, st>>>(
+      if constexpr (sizeof(RS) == 4 && sizeof(RO) == 4) {
+        if (phase_pairs(a, psi, out)) {
+          phase_rows_kernel<RA, RS, RO, true><<<(unsigned)grid, 256, 0, st>>>(
+              static_cast<const RA*>(ang), static_cast<const Cx<RS>*>(psi),
+              static_cast<Cx<RO>*>(out), r);
+          return after_launch("phase_rows_kernel");
+        }
+      }
+      phase_rows_kernel<RA, RS, RO, false><<<(unsigned)grid, 256, 0, st>>>(
           static_cast<const RA*>(ang), static_cast<const Cx<RS>*>(psi),
           static_cast<Cx<RO>*>(out), r);
       return after_launch("phase_rows_kernel");

@@ -73,3 +73,25 @@ def test_second_derivative_of_the_angles():
         g, = torch.autograd.grad(energy(a, phase), a, create_graph=True)
         into.append(torch.autograd.grad(g[3], a)[0])
     assert (got[0] - ref[0]).abs().max() <= 1e-12 * n * n
+
+
+@pytest.mark.parametrize("cols", [2, 254, 1022, 1024, 1026, 4096])
+@pytest.mark.parametrize("per_row", [False, True])
+def test_pairs_equal_single_amplitudes(cols, per_row):
+    """Two amplitudes at a time where every row is 16-byte aligned; the same
+    data one amplitude off takes the other form and gives the same bits."""
+    rng = np.random.default_rng(cols)
+    rows = 9
+    a = torch.from_numpy(rng.uniform(-9, 9, (rows, cols) if per_row else cols)
+                         ).float().to(DEV)
+    store = torch.zeros(rows * cols + 2, dtype=torch.complex64, device=DEV)
+    off = store[1:1 + rows * cols].view(rows, cols)
+    off.copy_(torch.from_numpy(rng.normal(size=(rows, cols)) +
+                               1j * rng.normal(size=(rows, cols))))
+    even = off.clone()
+    assert torch.equal(ug.apply_phase(a, even), ug.apply_phase(a, off))
+    # rows an odd number of amplitudes apart
+    wide = torch.zeros(rows, cols + 1, dtype=torch.complex64, device=DEV)
+    wide[:, :cols] = even
+    assert torch.equal(ug.apply_phase(a, wide[:, :cols]),
+                       ug.apply_phase(a, even))
