@@ -180,34 +180,34 @@ __device__ __forceinline__ void scale_sel(C* r, const C& m, int cls) {
 }
 
 // the same in double-float pairs (e: the entry's exact triple)
-template <typename C, int NR, int MASK, int PAT>
+template <typename C, int NR, int MASK, int PAT, bool FAST = false>
 __device__ __forceinline__ void scale_sel_df(C* r, const DEC& e, int cls) {
   switch (cls) {
     case EC_REAL:
 #pragma unroll
       for (int i = 0; i < NR; ++i)
         if ((i & MASK) == PAT) {
-          const DC y = df_rmul(e.re, df_split2(r[i].x, r[i].y));
-          r[i].x = df_join(y.re);
-          r[i].y = df_join(y.im);
+          const DC y = df_rmul(e.re, df_split2<FAST>(r[i].x, r[i].y));
+          r[i].x = df_join_add(y.re);
+          r[i].y = df_join_add(y.im);
         }
       return;
     case EC_IMAG:
 #pragma unroll
       for (int i = 0; i < NR; ++i)
         if ((i & MASK) == PAT) {
-          const DC y = df_imul(e.im, df_split2(r[i].x, r[i].y));
-          r[i].x = df_join(y.re);
-          r[i].y = df_join(y.im);
+          const DC y = df_imul(e.im, df_split2<FAST>(r[i].x, r[i].y));
+          r[i].x = df_join_add(y.re);
+          r[i].y = df_join_add(y.im);
         }
       return;
     case EC_FULL:
 #pragma unroll
       for (int i = 0; i < NR; ++i)
         if ((i & MASK) == PAT) {
-          const DC y = df_cmul(e, df_split2(r[i].x, r[i].y));
-          r[i].x = df_join(y.re);
-          r[i].y = df_join(y.im);
+          const DC y = df_cmul(e, df_split2<FAST>(r[i].x, r[i].y));
+          r[i].x = df_join_add(y.re);
+          r[i].y = df_join_add(y.im);
         }
       return;
     default:
@@ -314,7 +314,7 @@ __device__ __forceinline__ void apply_2x2(C* r, const C& m0, const C& m1,
 }
 
 // The same in double-float pairs, entries from their exact triples.
-template <typename C, int NR, int T, int CM, int CV>
+template <typename C, int NR, int T, int CM, int CV, bool FAST = false>
 __device__ __forceinline__ void apply_2x2_df(C* r, const DEC& e0,
                                              const DEC& e1, const DEC& e2,
                                              const DEC& e3, int kind,
@@ -331,8 +331,8 @@ __device__ __forceinline__ void apply_2x2_df(C* r, const DEC& e0,
       }
       return;
     case K1_DIAG:
-      scale_sel_df<C, NR, B | CM, CV>(r, e0, c[0]);
-      scale_sel_df<C, NR, B | CM, B | CV>(r, e3, c[3]);
+      scale_sel_df<C, NR, B | CM, CV, FAST>(r, e0, c[0]);
+      scale_sel_df<C, NR, B | CM, B | CV, FAST>(r, e3, c[3]);
       return;
     case K1_ANTI:
 #pragma unroll
@@ -342,15 +342,15 @@ __device__ __forceinline__ void apply_2x2_df(C* r, const DEC& e0,
         r[i] = r[i | B];
         r[i | B] = t;
       }
-      scale_sel_df<C, NR, B | CM, CV>(r, e1, c[1]);
-      scale_sel_df<C, NR, B | CM, B | CV>(r, e2, c[2]);
+      scale_sel_df<C, NR, B | CM, CV, FAST>(r, e1, c[1]);
+      scale_sel_df<C, NR, B | CM, B | CV, FAST>(r, e2, c[2]);
       return;
     default:
 #pragma unroll
       for (int i = 0; i < NR; ++i) {
         if ((i & B) || (i & CM) != CV) continue;
-        const DC a0 = df_split2(r[i].x, r[i].y);
-        const DC a1 = df_split2(r[i | B].x, r[i | B].y);
+        const DC a0 = df_split2<FAST>(r[i].x, r[i].y);
+        const DC a1 = df_split2<FAST>(r[i | B].x, r[i | B].y);
         DC y0, y1;
         if (kind == K1_REAL) {
           y0 = df_row2_real(e0.re, a0, e1.re, a1);
@@ -362,10 +362,10 @@ __device__ __forceinline__ void apply_2x2_df(C* r, const DEC& e0,
           y0 = df_row2(e0, a0, e1, a1);
           y1 = df_row2(e2, a0, e3, a1);
         }
-        r[i].x = df_join(y0.re);
-        r[i].y = df_join(y0.im);
-        r[i | B].x = df_join(y1.re);
-        r[i | B].y = df_join(y1.im);
+        r[i].x = df_join_add(y0.re);
+        r[i].y = df_join_add(y0.im);
+        r[i | B].x = df_join_add(y1.re);
+        r[i | B].y = df_join_add(y1.im);
       }
       return;
   }
@@ -514,11 +514,11 @@ __device__ __forceinline__ void apply_c128(C* r, const C* m,
 }
 
 // The same in double-float pairs (e: the entries' exact triples).
-template <typename C, int NR, int K, int RB0, int RB1>
+template <typename C, int NR, int K, int RB0, int RB1, bool FAST = false>
 __device__ __forceinline__ void apply_c128_df(C* r, const DEC* e,
                                               const OpKind& k) {
   if constexpr (K == 1) {
-    apply_2x2_df<C, NR, RB0, 0, 0>(r, e[0], e[1], e[2], e[3], k.kind, k.c);
+    apply_2x2_df<C, NR, RB0, 0, 0, FAST>(r, e[0], e[1], e[2], e[3], k.kind, k.c);
   } else {
     constexpr int M0 = 1 << RB0, M1 = 1 << RB1;
     switch (k.kind) {
@@ -526,23 +526,23 @@ __device__ __forceinline__ void apply_c128_df(C* r, const DEC* e,
         permute4<C, NR, RB0, RB1>(r, k.perm);
         if (k.c[0] != EC_ONE || k.c[1] != EC_ONE || k.c[2] != EC_ONE ||
             k.c[3] != EC_ONE) {
-          scale_sel_df<C, NR, M0 | M1, 0>(r, e[k.perm & 3], k.c[0]);
-          scale_sel_df<C, NR, M0 | M1, M1>(r, e[4 + ((k.perm >> 2) & 3)],
+          scale_sel_df<C, NR, M0 | M1, 0, FAST>(r, e[k.perm & 3], k.c[0]);
+          scale_sel_df<C, NR, M0 | M1, M1, FAST>(r, e[4 + ((k.perm >> 2) & 3)],
                                            k.c[1]);
-          scale_sel_df<C, NR, M0 | M1, M0>(r, e[8 + ((k.perm >> 4) & 3)],
+          scale_sel_df<C, NR, M0 | M1, M0, FAST>(r, e[8 + ((k.perm >> 4) & 3)],
                                            k.c[2]);
-          scale_sel_df<C, NR, M0 | M1, M0 | M1>(
+          scale_sel_df<C, NR, M0 | M1, M0 | M1, FAST>(
               r, e[12 + ((k.perm >> 6) & 3)], k.c[3]);
         }
         return;
       case 2:
-        scale_sel_df<C, NR, M0 | M1, 0>(r, e[0], k.c[0]);
-        scale_sel_df<C, NR, M0 | M1, M1>(r, e[5], k.c[1]);
-        scale_sel_df<C, NR, M0 | M1, M0>(r, e[10], k.c[2]);
-        scale_sel_df<C, NR, M0 | M1, M0 | M1>(r, e[15], k.c[3]);
+        scale_sel_df<C, NR, M0 | M1, 0, FAST>(r, e[0], k.c[0]);
+        scale_sel_df<C, NR, M0 | M1, M1, FAST>(r, e[5], k.c[1]);
+        scale_sel_df<C, NR, M0 | M1, M0, FAST>(r, e[10], k.c[2]);
+        scale_sel_df<C, NR, M0 | M1, M0 | M1, FAST>(r, e[15], k.c[3]);
         return;
       case 3:
-        apply_2x2_df<C, NR, RB1, M0, M0>(r, e[10], e[11], e[14], e[15],
+        apply_2x2_df<C, NR, RB1, M0, M0, FAST>(r, e[10], e[11], e[14], e[15],
                                          k.sub, k.c);
         return;
       default:
@@ -553,12 +553,12 @@ __device__ __forceinline__ void apply_c128_df(C* r, const DEC* e,
           DC a[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            a[j] = df_split2(r[idx[j]].x, r[idx[j]].y);
+            a[j] = df_split2<FAST>(r[idx[j]].x, r[idx[j]].y);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const DC y = df_row4(e + 4 * j, a);
-            r[idx[j]].x = df_join(y.re);
-            r[idx[j]].y = df_join(y.im);
+            r[idx[j]].x = df_join_add(y.re);
+            r[idx[j]].y = df_join_add(y.im);
           }
         }
         return;
@@ -618,6 +618,18 @@ __device__ __forceinline__ bool pairs_in_range(const C* r) {
     mx = max(mx, max(df_hiword(r[i].x) & 0x7ff00000u,
                      df_hiword(r[i].y) & 0x7ff00000u));
   return mx < ((DF_EMAX + 1) << 20) && (mx == 0 || mx >= (DF_EMIN << 20));
+}
+
+// Whether every component's exponent is in [DF_EMIN, DF_EMAX]: none is zero
+// or small, so the split needs no special cases.
+template <typename C, int NR>
+__device__ __forceinline__ bool pairs_all_in_range(const C* r) {
+  constexpr uint32_t LOW = DF_EMIN << 21;  // in units of 2 * hiword
+  uint32_t mx = 0;
+#pragma unroll
+  for (int i = 0; i < NR; ++i)
+    mx = max(mx, max(df_hiword(r[i].x) * 2 - LOW, df_hiword(r[i].y) * 2 - LOW));
+  return mx < ((DF_EMAX + 1 - DF_EMIN) << 21);
 }
 
 // NH high targets (chunks per unit = 2^NH); RB0 / RB1 are the register-index
@@ -733,6 +745,13 @@ __global__ void __launch_bounds__(256, 3)
 // compute.  Lanes never share a pair, so each lane writes back only what
 // it read.  Warp steps cover disjoint amplitudes, so in-place updates are
 // safe.
+//
+// A gate with arithmetic is bound by the ALU pipe, whose integer operations
+// are the conversions between doubles and pairs (69% busy, DRAM 62%).  Where
+// a whole warp's amplitudes are in the middle of the pairs' range the split
+// has no special cases, and the join is an FP64 addition: 3 states of 24
+// qubits (HBM alone 241 us) H 320 -> 279, RX 315 -> 274, RZ 333 -> 273, a
+// full matrix 397 -> 354 us; gates that only move 262 us as before.
 constexpr int C128_STAGES = 3;    // slots per warp: two in flight, one in use
 constexpr int C128_THREADS = 256;
 constexpr int C128_BLOCK = 128;   // amplitudes per warp step
@@ -847,8 +866,13 @@ __global__ void __launch_bounds__(C128_THREADS, 2)
     for (int j = 0; j < 4; ++j) r[j] = S[idx[j]];
 
     bool pairs = pairs_mode;
-    if (pairs && kind.arith) pairs = pairs_in_range<C, 4>(r);
-    if (pairs || !kind.arith)
+    const bool all =
+        pairs && kind.arith &&
+        __all_sync(0xffffffffu, pairs_all_in_range<C, 4>(r));
+    if (pairs && kind.arith && !all) pairs = pairs_in_range<C, 4>(r);
+    if (all)
+      apply_c128_df<C, 4, K, RB0, RB1, true>(r, op.e, kind);
+    else if (pairs || !kind.arith)
       apply_c128_df<C, 4, K, RB0, RB1>(r, op.e, kind);
     else
       apply_c128<C, 4, K, RB0, RB1>(r, op.raw, kind);
@@ -993,8 +1017,8 @@ __global__ void __launch_bounds__(128)
           for (int r = 0; r < D; ++r) {
             const DC y = df_rowD<D>(msd + r * D, xs);
             C o;
-            o.x = df_join(y.re);
-            o.y = df_join(y.im);
+            o.x = df_join_add(y.re);
+            o.y = df_join_add(y.im);
             dst[offs[r]] = o;
           }
         } else {

@@ -4,7 +4,7 @@
 // that does its arithmetic in FP64 is bound by the FP64 pipe, not by HBM.
 // The gate kernels instead carry each amplitude component as an unevaluated
 // pair of floats (hi + lo) and each matrix entry as an exact triple
-// (hi + mid + lo), and compute with FP32 / INT32 instructions only:
+// (hi + mid + lo), and compute with FP32 / INT32 instructions:
 //
 //   * df_split: a double -> pair by integer bit operations: hi is the double
 //     rounded to 24 significant bits, lo the signed remainder rounded to
@@ -21,7 +21,8 @@
 //   * sums of products use Knuth's TwoSum on the leading parts and add the
 //     error terms, then one fast renormalisation (Dekker's Fast2Sum);
 //   * df_join: pair -> double by integer operations on the bit pattern of
-//     hi, adding lo as a rounded integer number of double ulps of hi.
+//     hi, adding lo as a rounded integer number of double ulps of hi
+//     (df_join_add: by one FP64 addition, for kernels bound by the ALU).
 //
 // The relative error of one gate is a few units of 2^-47, unbiased; the
 // complex128 engine keeps native FP64 arithmetic as an option
@@ -166,6 +167,11 @@ GBSV_HD uint32_t df_expo(uint32_t hw) { return (hw >> 20) & 0x7ffu; }
 // [DF_EMIN, DF_EMAX], or every component is zero.
 constexpr uint32_t DF_EMIN = 1023 - 40, DF_EMAX = 1023 + 60;
 
+// FAST: |x| in [2^-40, 2^61) (pairs_all_in_range of the gate kernels), so
+// neither word is a special case; the signed count is taken times 8, which
+// leaves its sign where it is, and the factor of 8 comes off by a float
+// product (the ALU pipe bounds the gate kernels).  Same bits.
+template <bool FAST = false>
 GBSV_HD DF df_split(double x) {
   const uint32_t hw = df_hiword(x), lw = df_loword(x);
   const uint32_t sign = hw & 0x80000000u;
@@ -181,10 +187,16 @@ GBSV_HD DF df_split(double x) {
   // hi was rounded up), times 2^(e - 1075) with the original exponent e,
   // whose float exponent field e - 948 comes from the 9 low exponent bits
   // (mod 512) for e in [949, 1083]
-  const int32_t rest = (int32_t)(lw << 3) >> 3;
   const uint32_t sb = (((hw << 3) - (436u << 23)) & 0x7f800000u) | sign;
-  const float lo = df_mul_rn(df_i2f(rest), df_float(sb));
   DF d;
+  if constexpr (FAST) {
+    d.hi = df_float(hb);
+    d.lo = df_mul_rn(df_mul_rn(df_i2f((int32_t)(lw << 3)), 0.125f),
+                     df_float(sb));
+    return d;
+  }
+  const int32_t rest = (int32_t)(lw << 3) >> 3;
+  const float lo = df_mul_rn(df_i2f(rest), df_float(sb));
   d.hi = eb >= (897u << 20) ? df_float(hb) : 0.f;  // |x| >= 2^-126
   d.lo = eb >= (949u << 20) ? lo : 0.f;            // scale a normal float
   return d;
@@ -327,6 +339,31 @@ GBSV_HD double df_join(DF x) {
                   : df_make((uint32_t)(b >> 32), (uint32_t)b);
 }
 
+// The same by one FP64 addition of the two words as doubles.  A gate kernel
+// that moves its state between every split and join is bound by the ALU
+// pipe (82 of its integer operations per amplitude were conversions, with
+// the FP64 pipe idle), and this takes half of df_join's; the fused stages,
+// which join once per stage, are faster with df_join.  A zero or subnormal
+// word counts as up to 2^-126 (hi: exactly zero).
+GBSV_HD double df_widen(uint32_t b) {
+#ifdef __CUDA_ARCH__
+  uint64_t w;  // one multiply-add for the shift and the exponent's rebias
+  asm("mad.wide.u32 %0, %1, 268435456, %2;"
+      : "=l"(w)
+      : "r"(b + b), "l"(0x3800000000000000ull));
+#else
+  const uint64_t w = (uint64_t)(b + b) * 268435456u + 0x3800000000000000ull;
+#endif
+  return df_make((uint32_t)(w >> 32) | (b & 0x80000000u), (uint32_t)w);
+}
+GBSV_HD double df_join_add(DF x) {
+  const uint32_t hb = df_fbits(x.hi);
+  const double y = df_widen(hb) + df_widen(df_fbits(x.lo));
+  const bool zero = (hb & 0x7f800000u) == 0;
+  return df_make(zero ? hb & 0x80000000u : df_hiword(y),
+                 zero ? 0u : df_loword(y));
+}
+
 // ----------------------------------------------------- complex forms ----
 // The gate kernels' arithmetic on one amplitude pair, shared with the host
 // test.  Amplitudes are pairs per component, entries exact triples.
@@ -337,10 +374,11 @@ struct DEC {
   DE re, im;
 };
 
+template <bool FAST = false>
 GBSV_HD DC df_split2(double re, double im) {
   DC a;
-  a.re = df_split(re);
-  a.im = df_split(im);
+  a.re = df_split<FAST>(re);
+  a.im = df_split<FAST>(im);
   return a;
 }
 GBSV_HD DEC df_entry2(double re, double im) {
