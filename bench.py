@@ -1327,7 +1327,7 @@ def run_gpu(args, ws, rank, local):
             "speedup_vs_register_stages": round(reg_ms / fused_ms, 3),
             "register_stages_final_norm": reg_norm},
         "roofline_fused": {
-            "bound": "hbm", "kernel": "tc_stage_kernel" if prog.tensor_cores
+            "bound": "hbm", "kernel": "tc_wide_kernel" if prog.tensor_cores
             else "fused_reg_kernel",
             "achieved": round(bytes_per_gate / (statistics.mean(tc_stage_ms)
                                                 / 1e3) / 1e9, 1)

@@ -1849,8 +1849,9 @@ static int launch_wide(const float2* in, float2* out, const float2* ops,
 
 // Whether dense_wide_kernel takes this operator: complex64, 4 <= k <= 12,
 // one operator or a tile inside one state, and in place only over
-// contiguous states.  Below 6 qubits the group kernel is the alternative:
-// the tile kernel takes every 5-qubit operator (the group kernel's 32
+// contiguous states.  Below 6 qubits dense_stream_kernel is asked first
+// (stream_applies); of what it leaves (small or unaligned states, per-state
+// operators) the group kernel is the alternative: the tile kernel takes every 5-qubit operator (the group kernel's 32
 // amplitudes per thread leave it at half the tile kernel's rate) and
 // 4-qubit operators with a target among the three lowest bits (groups of
 // contiguous amplitudes, where consecutive threads of the group kernel
