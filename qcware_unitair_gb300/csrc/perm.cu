@@ -650,13 +650,15 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t x, int src) {
   return ((uint64_t)hi << 32) | lo;
 }
 
-// SPT samples per thread in flight at once (independent search chains).
-// The searches run per thread; the chunk's group sums (64 B) and the
-// group's amplitudes (128 B) are then read cooperatively, 4 and 8 lanes
-// per sample, so that one warp load touches 8 or 4 cache lines instead of
-// 32 (the L1's per-line work bounded the per-thread version).  The sample
+// One sample per thread: a chain of dependent reads, so what counts is how
+// many warps run it (four chains per thread, at the registers they took and
+// a quarter of the blocks, was slower at every count: 100,000 samples of 24
+// qubits 30.5 against 15.9 us, a million 108 against 77, of 16 qubits 62
+// against 49).  The searches run per thread; the chunk's group sums (64 B)
+// and the group's amplitudes (128 B) are then read cooperatively, 4 and 8
+// lanes per sample, so that one warp load touches 8 or 4 cache lines instead
+// of 32 (the L1's per-line work bounded the per-thread version).  The sample
 // loop is warp-uniform: all lanes take part in the shuffles.
-template <int SPT>
 __global__ void __launch_bounds__(256)
     sample_c64_kernel(const float4* psi, const double* lcdf,
                       const float* subs, const double* off, int nb,
@@ -670,96 +672,76 @@ __global__ void __launch_bounds__(256)
   const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
   const float4* subs4 = reinterpret_cast<const float4*>(subs);
   for (uint64_t wb = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
-       wb < num_samples; wb += nthreads * SPT) {
-    const uint64_t s0 = wb + lane;
-    uint64_t c[SPT], lo[SPT], hi[SPT];
-    double ub[SPT];
-    bool live[SPT];
-#pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-      const uint64_t sidx = s0 + k * nthreads;
-      live[k] = sidx < num_samples;
-      const uint64_t h = mix64(seed ^ mix64(sidx));
-      const double u = (double)(h >> 11) * (1.0 / 9007199254740992.0) * total;
-      // the last segment whose offset is <= u (zero-mass segments are
-      // skipped)
-      int blo = 0, bhi = nb - 1;
-      while (blo < bhi) {
-        const int mid = (blo + bhi + 1) >> 1;
-        if (soff[mid] <= u) blo = mid; else bhi = mid - 1;
-      }
-      ub[k] = u - soff[blo];
-      lo[k] = (uint64_t)blo * per;
-      hi[k] = lo[k] + per < nchunks ? lo[k] + per - 1 : nchunks - 1;
+       wb < num_samples; wb += nthreads) {
+    const uint64_t sidx = wb + lane;
+    const uint64_t h = mix64(seed ^ mix64(sidx));
+    const double u = (double)(h >> 11) * (1.0 / 9007199254740992.0) * total;
+    // the last segment whose offset is <= u (zero-mass segments are
+    // skipped)
+    int blo = 0, bhi = nb - 1;
+    while (blo < bhi) {
+      const int mid = (blo + bhi + 1) >> 1;
+      if (soff[mid] <= u) blo = mid; else bhi = mid - 1;
     }
+    const double ub = u - soff[blo];
+    const uint64_t bfirst = (uint64_t)blo * per;
     // first chunk of the segment whose local prefix exceeds the rest
     // (rounding can leave the rest above the segment's total: last chunk)
-    bool busy = true;
-    while (busy) {
-      busy = false;
+    uint64_t ck = bfirst;
+    uint64_t hi = bfirst + per < nchunks ? bfirst + per - 1 : nchunks - 1;
+    while (ck < hi) {
+      const uint64_t mid = (ck + hi) >> 1;
+      if (lcdf[mid] > ub) hi = mid; else ck = mid + 1;
+    }
+    __syncwarp();
+    const double run = ck > bfirst ? lcdf[ck - 1] : 0.0;
+    float rem = (float)(ub - run);
+    // group sums: in round r, lanes 4 q .. 4 q + 3 read the 16 group sums of
+    // owner lane 8 r + q
+    float4 gq[4];
 #pragma unroll
-      for (int k = 0; k < SPT; ++k) {
-        if (lo[k] < hi[k]) {
-          const uint64_t mid = (lo[k] + hi[k]) >> 1;
-          if (lcdf[mid] > ub[k]) hi[k] = mid; else lo[k] = mid + 1;
-          busy = true;
-        }
+    for (int r = 0; r < 4; ++r) {
+      const uint64_t co = shfl64(ck, 8 * r + (lane >> 2));
+      gq[r] = subs4[co * (SGROUPS / 4) + (lane & 3)];
+    }
+    int grp = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float rem_o = __shfl_sync(0xffffffffu, rem, 8 * r + (lane >> 2));
+      const float v[4] = {gq[r].x, gq[r].y, gq[r].z, gq[r].w};
+      float ge;
+      const int gi = seg_pick<4, 4>(v, rem_o, &ge);
+      // owners 8 r .. 8 r + 7 take their segment's result
+      const int src = ((lane - 8 * r) & 7) * 4;
+      const int gi_o = __shfl_sync(0xffffffffu, gi, src);
+      const float ge_o = __shfl_sync(0xffffffffu, ge, src);
+      if ((lane >> 3) == r) {
+        grp = gi_o < 0 ? 0 : gi_o;
+        rem -= ge_o;
       }
     }
+    // amplitudes: in round r, lanes 8 q .. 8 q + 7 read the 16 amplitudes
+    // (two each) of owner lane 4 r + q
+    const uint64_t gbase = ck * SCHUNK + (uint64_t)grp * SGROUP;
+    float4 aq[8];
 #pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-      const uint64_t ck = lo[k];
-      c[k] = ck;
-      const uint64_t bfirst = (ck / per) * per;
-      const double run = ck > bfirst ? lcdf[ck - 1] : 0.0;
-      float rem = (float)(ub[k] - run);
-      // group sums: in round r, lanes 4 q .. 4 q + 3 read the 16 group
-      // sums of owner lane 8 r + q
-      float4 gq[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const uint64_t co = shfl64(ck, 8 * r + (lane >> 2));
-        gq[r] = subs4[co * (SGROUPS / 4) + (lane & 3)];
-      }
-      int grp = 0;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float rem_o = __shfl_sync(0xffffffffu, rem, 8 * r + (lane >> 2));
-        const float v[4] = {gq[r].x, gq[r].y, gq[r].z, gq[r].w};
-        float ge;
-        const int gi = seg_pick<4, 4>(v, rem_o, &ge);
-        // owners 8 r .. 8 r + 7 take their segment's result
-        const int src = ((lane - 8 * r) & 7) * 4;
-        const int gi_o = __shfl_sync(0xffffffffu, gi, src);
-        const float ge_o = __shfl_sync(0xffffffffu, ge, src);
-        if ((lane >> 3) == r) {
-          grp = gi_o < 0 ? 0 : gi_o;
-          rem -= ge_o;
-        }
-      }
-      // amplitudes: in round r, lanes 8 q .. 8 q + 7 read the 16 amplitudes
-      // (two each) of owner lane 4 r + q
-      const uint64_t gbase = ck * SCHUNK + (uint64_t)grp * SGROUP;
-      float4 aq[8];
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const uint64_t gb = shfl64(gbase, 4 * r + (lane >> 3));
-        aq[r] = psi[gb / 2 + (lane & 7)];
-      }
-      int res = 0;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) {
-        const float rem_o = __shfl_sync(0xffffffffu, rem, 4 * r + (lane >> 3));
-        const float v[2] = {fmaf(aq[r].x, aq[r].x, aq[r].y * aq[r].y),
-                            fmaf(aq[r].z, aq[r].z, aq[r].w * aq[r].w)};
-        float ae;
-        const int ai = seg_pick<8, 2>(v, rem_o, &ae);
-        const int src = ((lane - 4 * r) & 3) * 8;
-        const int ai_o = __shfl_sync(0xffffffffu, ai, src);
-        if ((lane >> 2) == r) res = ai_o < 0 ? 0 : ai_o;
-      }
-      if (live[k]) out[s0 + k * nthreads] = (int64_t)gbase + res;
+    for (int r = 0; r < 8; ++r) {
+      const uint64_t gb = shfl64(gbase, 4 * r + (lane >> 3));
+      aq[r] = psi[gb / 2 + (lane & 7)];
     }
+    int res = 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float rem_o = __shfl_sync(0xffffffffu, rem, 4 * r + (lane >> 3));
+      const float v[2] = {fmaf(aq[r].x, aq[r].x, aq[r].y * aq[r].y),
+                          fmaf(aq[r].z, aq[r].z, aq[r].w * aq[r].w)};
+      float ae;
+      const int ai = seg_pick<8, 2>(v, rem_o, &ae);
+      const int src = ((lane - 4 * r) & 3) * 8;
+      const int ai_o = __shfl_sync(0xffffffffu, ai, src);
+      if ((lane >> 2) == r) res = ai_o < 0 ? 0 : ai_o;
+    }
+    if (sidx < num_samples) out[sidx] = (int64_t)gbase + res;
   }
 }
 
@@ -1032,12 +1014,11 @@ static int sample_c64_fine(const void* state, int64_t dim,
   sample_offsets_kernel<<<1, 1024, 0, st>>>(tot, (int)nb);
   rc = after_launch("sample_offsets_kernel");
   if (rc) return rc;
-  constexpr int SPT = 4;
-  uint64_t blocks = ((uint64_t)num_samples + 256 * SPT - 1) / (256 * SPT);
+  uint64_t blocks = ((uint64_t)num_samples + 255) / 256;
   const uint64_t cap = (uint64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   const size_t smem = (nb + 1) * sizeof(double);
-  sample_c64_kernel<SPT><<<(unsigned)blocks, 256, smem, st>>>(
+  sample_c64_kernel<<<(unsigned)blocks, 256, smem, st>>>(
       static_cast<const float4*>(state), lcdf, subs, tot, (int)nb, per,
       nchunks, (uint64_t)num_samples, seed, out_indices);
   return after_launch("sample_c64_kernel");
