@@ -632,6 +632,65 @@ __device__ __forceinline__ bool pairs_all_in_range(const C* r) {
   return mx < ((DF_EMAX + 1 - DF_EMIN) << 21);
 }
 
+// A 2x2 of its own for each state, FP64.  Rotations have entries that are
+// real, imaginary or zero in a fixed pattern; leaving out the products with
+// the zeros halves the FP64 operations, which bound this path.  The choice
+// is per warp (a choice per thread is turned into selects that run every
+// form), and where an amplitude is not finite, so that a product with zero
+// is not zero, the full form runs.
+template <typename C, int NR, int T>
+__device__ __forceinline__ void apply_own_2x2(C* r, const C* m) {
+  constexpr int B = 1 << T;
+  const unsigned lanes = __activemask();
+  // by integers: a comparison of doubles is FP64 work
+  auto zero = [](double x) {
+    return ((df_hiword(x) << 1) | df_loword(x)) == 0;
+  };
+  const bool re1 = zero(m[1].y) && zero(m[2].y);
+  const bool im1 = zero(m[1].x) && zero(m[2].x);
+  const bool real03 = zero(m[0].y) && zero(m[3].y);
+  int form = re1 && im1 ? 3 : !real03 ? 0 : re1 ? 1 : im1 ? 2 : 0;
+  if (__any_sync(lanes, form != 0)) {
+#pragma unroll
+    for (int i = 0; i < NR; ++i)
+      if ((df_hiword(r[i].x) & 0x7ff00000u) == 0x7ff00000u ||
+          (df_hiword(r[i].y) & 0x7ff00000u) == 0x7ff00000u)
+        form = 0;
+  }
+  if (__all_sync(lanes, form == 1)) {  // real
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      if (i & B) continue;
+      const C a0 = r[i], a1 = r[i | B];
+      r[i].x = fma(m[1].x, a1.x, m[0].x * a0.x);
+      r[i].y = fma(m[1].x, a1.y, m[0].x * a0.y);
+      r[i | B].x = fma(m[3].x, a1.x, m[2].x * a0.x);
+      r[i | B].y = fma(m[3].x, a1.y, m[2].x * a0.y);
+    }
+  } else if (__all_sync(lanes, form == 2)) {  // real, imaginary off-diagonal
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      if (i & B) continue;
+      const C a0 = r[i], a1 = r[i | B];
+      r[i].x = fma(-m[1].y, a1.y, m[0].x * a0.x);
+      r[i].y = fma(m[1].y, a1.x, m[0].x * a0.y);
+      r[i | B].x = fma(m[3].x, a1.x, -(m[2].y * a0.y));
+      r[i | B].y = fma(m[3].x, a1.y, m[2].y * a0.x);
+    }
+  } else if (__all_sync(lanes, form == 3)) {  // diagonal
+#pragma unroll
+    for (int i = 0; i < NR; ++i) r[i] = cmul(i & B ? m[3] : m[0], r[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      if (i & B) continue;
+      const C a0 = r[i], a1 = r[i | B];
+      r[i] = cmad(m[1], a1, cmul(m[0], a0));
+      r[i | B] = cmad(m[3], a1, cmul(m[2], a0));
+    }
+  }
+}
+
 // NH high targets (chunks per unit = 2^NH); RB0 / RB1 are the register-index
 // bits of the first / second target in matrix order.
 template <typename R, int V, int K, int NH, int RB0, int RB1>
@@ -715,7 +774,10 @@ __global__ void __launch_bounds__(256, 3)
       const C* mp = ops + state[u] * a.op_stride;
 #pragma unroll
       for (int j = 0; j < D * D; ++j) m[j] = __ldg(mp + j);
-      apply_regs<C, NR, K, RB0, RB1>(reg[u], m);
+      if constexpr (kC128 && K == 1)
+        apply_own_2x2<C, NR, RB0>(reg[u], m);
+      else
+        apply_regs<C, NR, K, RB0, RB1>(reg[u], m);
     } else if constexpr (!kC128) {
       apply_regs<C, NR, K, RB0, RB1>(reg[u], m);
     }
