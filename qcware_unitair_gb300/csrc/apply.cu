@@ -2427,22 +2427,28 @@ static bool phase_pairs(const PhaseArgs& a, const void* psi, const void* out) {
 template <typename RA, typename RS, typename RO>
 static int launch_phase(const void* ang, const void* psi, void* out,
                         const PhaseArgs& a, cudaStream_t st) {
-  if (a.ndim > 1 && phase_by_rows(a)) {
-    const PhaseRowArgs r = phase_row_args(a, PHASE_ROWS);
-    const uint64_t grid = r.col_blocks * ((r.rows + r.per - 1) / r.per);
-    if (grid <= 0x7fffffffull) {
-      if constexpr (sizeof(RS) == 4 && sizeof(RO) == 4) {
-        if (phase_pairs(a, psi, out)) {
+  // By rows in single precision, and beyond one wave of the kernel by
+  // element, whose threads then take one element each (26 states of 13
+  // qubits 3.1 us by rows, 2.8 by element; of 14 qubits 3.4 and 4.1; 100 of
+  // 14 6.0 and 10.8).  In double precision a phase factor is a long chain
+  // and wants a thread to itself: 26 states of 13 qubits 12.5 and 6.4 us,
+  // 7 of 20 139 and 124.
+  if constexpr (sizeof(RA) == 4 && sizeof(RS) == 4) {
+    if (a.ndim > 1 && phase_by_rows(a) &&
+        a.total > (uint64_t)sm_count() * 2048) {
+      const PhaseRowArgs r = phase_row_args(a, PHASE_ROWS);
+      const uint64_t grid = r.col_blocks * ((r.rows + r.per - 1) / r.per);
+      if (grid <= 0x7fffffffull) {
+        if (phase_pairs(a, psi, out))
           phase_rows_kernel<RA, RS, RO, true><<<(unsigned)grid, 256, 0, st>>>(
               static_cast<const RA*>(ang), static_cast<const Cx<RS>*>(psi),
               static_cast<Cx<RO>*>(out), r);
-          return after_launch("phase_rows_kernel");
-        }
+        else
+          phase_rows_kernel<RA, RS, RO, false><<<(unsigned)grid, 256, 0, st>>>(
+              static_cast<const RA*>(ang), static_cast<const Cx<RS>*>(psi),
+              static_cast<Cx<RO>*>(out), r);
+        return after_launch("phase_rows_kernel");
       }
-      phase_rows_kernel<RA, RS, RO, false><<<(unsigned)grid, 256, 0, st>>>(
-          static_cast<const RA*>(ang), static_cast<const Cx<RS>*>(psi),
-          static_cast<Cx<RO>*>(out), r);
-      return after_launch("phase_rows_kernel");
     }
   }
   uint64_t blocks = (a.total + 255) / 256;
@@ -2533,7 +2539,11 @@ extern "C" int gbsv_apply_phase_grad(const void* angles, int angle_dtype,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const PhaseRowArgs r = phase_row_args(a, 1);
   const uint64_t row_grid = r.col_blocks * r.rows;
-  const bool rows = phase_by_rows(a) && row_grid <= 0x7fffffffull;
+  // as forward: in single precision beyond a wave by element (26 states of
+  // 13 qubits 3.7 us by rows, 3.2 by element; 100 of 14 8.0 and 12.5)
+  const bool rows = out_dtype == GBSV_C64 && phase_by_rows(a) &&
+                    a.total > (uint64_t)sm_count() * 2048 &&
+                    row_grid <= 0x7fffffffull;
   const uint64_t grid =
       rows ? row_grid
            : std::min<uint64_t>((a.total + 255) / 256,
@@ -2548,11 +2558,9 @@ extern "C" int gbsv_apply_phase_grad(const void* angles, int angle_dtype,
     if (rows) GBSV_PHASE_GRAD(float, float, true);
     else GBSV_PHASE_GRAD(float, float, false);
   } else if (angle_dtype == GBSV_F32) {
-    if (rows) GBSV_PHASE_GRAD(float, double, true);
-    else GBSV_PHASE_GRAD(float, double, false);
+    GBSV_PHASE_GRAD(float, double, false);
   } else {
-    if (rows) GBSV_PHASE_GRAD(double, double, true);
-    else GBSV_PHASE_GRAD(double, double, false);
+    GBSV_PHASE_GRAD(double, double, false);
   }
 #undef GBSV_PHASE_GRAD
   return after_launch("phase_grad_kernel");

@@ -95,3 +95,31 @@ def test_pairs_equal_single_amplitudes(cols, per_row):
     wide[:, :cols] = even
     assert torch.equal(ug.apply_phase(a, wide[:, :cols]),
                        ug.apply_phase(a, even))
+
+
+@pytest.mark.parametrize("rows,cols", [(304, 1024), (305, 1024), (613, 512),
+                                       (97, 4098), (330, 1026), (80, 4097)])
+def test_rows_and_elements_agree(rows, cols):
+    """Around 2048 elements per SM, where rows take over from elements: the
+    forms give the same bits forward, and gradients within a rounding."""
+    rng = np.random.default_rng(rows)
+    a = torch.from_numpy(rng.uniform(-9, 9, cols)).float().to(DEV)
+    s = torch.from_numpy(rng.normal(size=(rows, cols)) +
+                         1j * rng.normal(size=(rows, cols))
+                         ).to(torch.complex64).to(DEV)
+    whole = ug.apply_phase(a, s)
+    parts = torch.cat([ug.apply_phase(a, s[i:i + 8])
+                       for i in range(0, rows, 8)])
+    assert torch.equal(whole, parts)
+    w = torch.from_numpy(rng.normal(size=(rows, cols)) + 0j
+                         ).to(torch.complex64).to(DEV)
+    grads = []
+    for step in (rows, 8):
+        x = s.clone().requires_grad_()
+        t = a.expand(rows, cols).clone().requires_grad_()
+        for i in range(0, rows, step):
+            ug.apply_phase(t[i:i + step], x[i:i + step]).backward(
+                w[i:i + step])
+        grads.append((x.grad, t.grad))
+    for g, h in zip(*grads):
+        assert torch.equal(g, h)
