@@ -314,7 +314,11 @@ int gbsv_run_programs(int dtype, int num_qubits, int num_ctas,
  * state's bits at positions opos[0 .. nout-1], bit k of p from opos[k]) --
  * the diagonal gates that commute with the block, folded on the host -- and
  * by the post-diagonals diags[first_diag .. first_diag + num_diag).  flags
- * bit 0: register bit 0 is tile bit 0. */
+ * bit 0: register bit 0 is tile bit 0; bit 1: the amplitude of register
+ * index i is multiplied by float i of factors[cols .. cols + 16) first.  An
+ * image holds entries up to 2 with the L1 norms of B's columns up to 8, as
+ * every unitary has; the matrix of other blocks is divided by powers of two,
+ * one per column of U, which those floats put back. */
 typedef struct gbsv_tc_block {
   int16_t rspo[5];
   int16_t tspo[7];
@@ -325,7 +329,8 @@ typedef struct gbsv_tc_block {
   int32_t fac;
   int8_t nout;
   int8_t opos[7];
-  int32_t pad_[3];
+  int32_t cols;
+  int32_t pad_[2];
 } gbsv_tc_block_t;
 
 /* A 1- or 2-qubit diagonal applied after a block (48 bytes): each qubit is

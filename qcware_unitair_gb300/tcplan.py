@@ -33,12 +33,12 @@ from . import _lib
 
 TC_M, TC_RB, TC_TB = 12, 5, 7
 TC_MAX_BLOCKS = 64
-TC_PAIRS = 1
+TC_PAIRS, TC_COLS = 1, 2
 BLOCK_DTYPE = np.dtype([("rspo", "<i2", (5,)), ("tspo", "<i2", (7,)),
                         ("mat", "<i4"), ("first_diag", "<i4"),
                         ("num_diag", "<i4"), ("flags", "<i4"), ("fac", "<i4"),
                         ("nout", "i1"), ("opos", "i1", (7,)),
-                        ("pad", "<i4", (3,))])
+                        ("cols", "<i4"), ("pad", "<i4", (2,))])
 TC_MAX_OUT = 5  # outside bits a block's factor table may depend on
 DIAG_DTYPE = np.dtype([("nq", "<i4"), ("enc", "<i4", (2,)), ("reg", "<i4"),
                        ("d", "<f4", (8,))])
@@ -194,6 +194,39 @@ def _embed(mat: np.ndarray, kbits: List[int]) -> np.ndarray:
     return np.where(same, mat[sub[:, None], sub[None, :]], 0)
 
 
+# What the exact-integer product of the kernel needs of a block's matrix: its
+# rows' L1 norm (real form) at most 8, every entry at most 2.  An image keeps
+# 22 bits below 1, so a column whose entries are all far below that (a
+# unitary's largest is at least 1/8) would lose bits as well.
+_ROW_L1, _COL_MOST, _COL_LEAST = 8.0, 2.0, 0.12
+
+
+def _row_l1(U: np.ndarray) -> float:
+    return float((np.abs(U.real) + np.abs(U.imag)).sum(axis=1).max())
+
+
+def column_scales(U: np.ndarray):
+    """(scales, matrix) with U = matrix * scales (by column), the scales
+    powers of two (0 for a column of zeros) that bring the matrix into the
+    range of an image; (None, U) where U is in it, as every unitary is.  The
+    kernel multiplies the amplitudes by the scales, which is exact."""
+    big = np.maximum(np.abs(U.real), np.abs(U.imag)).max(axis=0)
+    if not np.isfinite(big).all() or (
+            big.min() >= _COL_LEAST and big.max() <= _COL_MOST
+            and _row_l1(U) <= 1.001 * _ROW_L1):
+        return None, U
+    e = np.where(big > 0, np.frexp(big)[1], -126)
+    # room for the halvings below; beyond FP32's range the product is 0 or
+    # infinite in any order
+    e = np.clip(e, -126, 120)
+    while True:
+        scales = np.where(big > 0, np.ldexp(1.0, e), 0.0)
+        W = U / np.where(big > 0, scales, 1.0)
+        if _row_l1(W) <= _ROW_L1 or e.max() >= 127:
+            return scales, W
+        e = e + 1
+
+
 def block_image(U: np.ndarray) -> np.ndarray:
     """fp16 image (8192 values, [Bl; Bh]) of the real form B of U^T:
     Bh = rint(1024 B) (integers), Bl = 1024 B - Bh."""
@@ -223,8 +256,8 @@ def image_matrix(img: np.ndarray) -> np.ndarray:
 def encode_stage(plan: TcStagePlan, n: int, blocks_out: list,
                  diags_out: list, images_out: list, factors_out: list):
     """Records of one stage appended to the program's arrays (factor tables
-    to factors_out as complex64 arrays of 128 * 2^nout entries); returns
-    (c, positions)."""
+    to factors_out as complex64 arrays of 128 * 2^nout entries, column scales
+    as 16, two floats each); returns (c, positions)."""
     tile = set(plan.tile)
     p = 0
     while len(tile) < TC_M:
@@ -311,6 +344,11 @@ def encode_stage(plan: TcStagePlan, n: int, blocks_out: list,
                 tab = tab * vals[idx]
             fac = sum(f.size for f in factors_out)
             factors_out.append(tab.astype(np.complex64).reshape(-1))
+        scales, U = column_scales(U)
+        cols = 0
+        if scales is not None:
+            cols = sum(f.size for f in factors_out)
+            factors_out.append(scales.astype(np.float32).view(np.complex64))
         first_diag = len(diags_out)
         for it, enc in listed:
             vals = np.diagonal(_host_matrix(it.gate)).astype(np.complex64)
@@ -337,7 +375,9 @@ def encode_stage(plan: TcStagePlan, n: int, blocks_out: list,
         brec["mat"] = len(images_out)
         brec["first_diag"] = first_diag
         brec["num_diag"] = len(diags_out) - first_diag
-        brec["flags"] = TC_PAIRS if pairs else 0
+        brec["flags"] = (TC_PAIRS if pairs else 0) | (
+            TC_COLS if scales is not None else 0)
+        brec["cols"] = cols
         brec["fac"] = fac
         brec["nout"] = len(opos)
         brec["opos"][:len(opos)] = opos
