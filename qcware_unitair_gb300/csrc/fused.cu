@@ -1157,6 +1157,9 @@ __device__ __forceinline__ void fused_reg_body(const Cx<R>* in, Cx<R>* out,
       const C* src = pool + g.mat + (int64_t)s * g.mat_bstride;
       const int mo = nv[gi];
       const int vm = vp[gi];  // value permutation from relabelling
+      // a one-qubit diagonal leaves half its slot, which to_pairs looks at
+      if constexpr (kPairs)
+        for (int j = k; j < 4; ++j) mats[mo + j] = czero<C>();
       if (vm == 0) {
         for (int j = 0; j < k; ++j) mats[mo + j] = src[j];
       } else if (vm == VP_REV4) {
