@@ -179,35 +179,48 @@ __device__ __forceinline__ void scale_sel(C* r, const C& m, int cls) {
   }
 }
 
+// How a thread's amplitudes go to pairs and back.
+enum {
+  PAIRS_ANY,    // any magnitude
+  PAIRS_ZEROS,  // each component is zero or in [2^-40, 2^61),
+  PAIRS_FAST    // or in it, and the operator's entries are C128Op::even
+};
+template <int P, typename C>
+__device__ __forceinline__ void join_pair(const DC& y, C* r) {
+  if constexpr (P == PAIRS_ANY) {
+    df_join2(y, r);
+  } else {
+    r->x = df_join_add(y.re);
+    r->y = df_join_add(y.im);
+  }
+}
+
 // the same in double-float pairs (e: the entry's exact triple)
-template <typename C, int NR, int MASK, int PAT, bool FAST = false>
+template <typename C, int NR, int MASK, int PAT, int P = PAIRS_ANY>
 __device__ __forceinline__ void scale_sel_df(C* r, const DEC& e, int cls) {
   switch (cls) {
     case EC_REAL:
 #pragma unroll
       for (int i = 0; i < NR; ++i)
         if ((i & MASK) == PAT) {
-          const DC y = df_rmul(e.re, df_split2<FAST>(r[i].x, r[i].y));
-          r[i].x = df_join_add(y.re);
-          r[i].y = df_join_add(y.im);
+          const DC y = df_rmul(e.re, df_split2<P == PAIRS_FAST>(r[i].x, r[i].y));
+          join_pair<P>(y, &r[i]);
         }
       return;
     case EC_IMAG:
 #pragma unroll
       for (int i = 0; i < NR; ++i)
         if ((i & MASK) == PAT) {
-          const DC y = df_imul(e.im, df_split2<FAST>(r[i].x, r[i].y));
-          r[i].x = df_join_add(y.re);
-          r[i].y = df_join_add(y.im);
+          const DC y = df_imul(e.im, df_split2<P == PAIRS_FAST>(r[i].x, r[i].y));
+          join_pair<P>(y, &r[i]);
         }
       return;
     case EC_FULL:
 #pragma unroll
       for (int i = 0; i < NR; ++i)
         if ((i & MASK) == PAT) {
-          const DC y = df_cmul(e, df_split2<FAST>(r[i].x, r[i].y));
-          r[i].x = df_join_add(y.re);
-          r[i].y = df_join_add(y.im);
+          const DC y = df_cmul(e, df_split2<P == PAIRS_FAST>(r[i].x, r[i].y));
+          join_pair<P>(y, &r[i]);
         }
       return;
     default:
@@ -314,7 +327,7 @@ __device__ __forceinline__ void apply_2x2(C* r, const C& m0, const C& m1,
 }
 
 // The same in double-float pairs, entries from their exact triples.
-template <typename C, int NR, int T, int CM, int CV, bool FAST = false>
+template <typename C, int NR, int T, int CM, int CV, int P = PAIRS_ANY>
 __device__ __forceinline__ void apply_2x2_df(C* r, const DEC& e0,
                                              const DEC& e1, const DEC& e2,
                                              const DEC& e3, int kind,
@@ -331,8 +344,8 @@ __device__ __forceinline__ void apply_2x2_df(C* r, const DEC& e0,
       }
       return;
     case K1_DIAG:
-      scale_sel_df<C, NR, B | CM, CV, FAST>(r, e0, c[0]);
-      scale_sel_df<C, NR, B | CM, B | CV, FAST>(r, e3, c[3]);
+      scale_sel_df<C, NR, B | CM, CV, P>(r, e0, c[0]);
+      scale_sel_df<C, NR, B | CM, B | CV, P>(r, e3, c[3]);
       return;
     case K1_ANTI:
 #pragma unroll
@@ -342,15 +355,15 @@ __device__ __forceinline__ void apply_2x2_df(C* r, const DEC& e0,
         r[i] = r[i | B];
         r[i | B] = t;
       }
-      scale_sel_df<C, NR, B | CM, CV, FAST>(r, e1, c[1]);
-      scale_sel_df<C, NR, B | CM, B | CV, FAST>(r, e2, c[2]);
+      scale_sel_df<C, NR, B | CM, CV, P>(r, e1, c[1]);
+      scale_sel_df<C, NR, B | CM, B | CV, P>(r, e2, c[2]);
       return;
     default:
 #pragma unroll
       for (int i = 0; i < NR; ++i) {
         if ((i & B) || (i & CM) != CV) continue;
-        const DC a0 = df_split2<FAST>(r[i].x, r[i].y);
-        const DC a1 = df_split2<FAST>(r[i | B].x, r[i | B].y);
+        const DC a0 = df_split2<P == PAIRS_FAST>(r[i].x, r[i].y);
+        const DC a1 = df_split2<P == PAIRS_FAST>(r[i | B].x, r[i | B].y);
         DC y0, y1;
         if (kind == K1_REAL) {
           y0 = df_row2_real(e0.re, a0, e1.re, a1);
@@ -362,10 +375,8 @@ __device__ __forceinline__ void apply_2x2_df(C* r, const DEC& e0,
           y0 = df_row2(e0, a0, e1, a1);
           y1 = df_row2(e2, a0, e3, a1);
         }
-        r[i].x = df_join_add(y0.re);
-        r[i].y = df_join_add(y0.im);
-        r[i | B].x = df_join_add(y1.re);
-        r[i | B].y = df_join_add(y1.im);
+        join_pair<P>(y0, &r[i]);
+        join_pair<P>(y1, &r[i | B]);
       }
       return;
   }
@@ -514,11 +525,11 @@ __device__ __forceinline__ void apply_c128(C* r, const C* m,
 }
 
 // The same in double-float pairs (e: the entries' exact triples).
-template <typename C, int NR, int K, int RB0, int RB1, bool FAST = false>
+template <typename C, int NR, int K, int RB0, int RB1, int P = PAIRS_ANY>
 __device__ __forceinline__ void apply_c128_df(C* r, const DEC* e,
                                               const OpKind& k) {
   if constexpr (K == 1) {
-    apply_2x2_df<C, NR, RB0, 0, 0, FAST>(r, e[0], e[1], e[2], e[3], k.kind, k.c);
+    apply_2x2_df<C, NR, RB0, 0, 0, P>(r, e[0], e[1], e[2], e[3], k.kind, k.c);
   } else {
     constexpr int M0 = 1 << RB0, M1 = 1 << RB1;
     switch (k.kind) {
@@ -526,23 +537,23 @@ __device__ __forceinline__ void apply_c128_df(C* r, const DEC* e,
         permute4<C, NR, RB0, RB1>(r, k.perm);
         if (k.c[0] != EC_ONE || k.c[1] != EC_ONE || k.c[2] != EC_ONE ||
             k.c[3] != EC_ONE) {
-          scale_sel_df<C, NR, M0 | M1, 0, FAST>(r, e[k.perm & 3], k.c[0]);
-          scale_sel_df<C, NR, M0 | M1, M1, FAST>(r, e[4 + ((k.perm >> 2) & 3)],
+          scale_sel_df<C, NR, M0 | M1, 0, P>(r, e[k.perm & 3], k.c[0]);
+          scale_sel_df<C, NR, M0 | M1, M1, P>(r, e[4 + ((k.perm >> 2) & 3)],
                                            k.c[1]);
-          scale_sel_df<C, NR, M0 | M1, M0, FAST>(r, e[8 + ((k.perm >> 4) & 3)],
+          scale_sel_df<C, NR, M0 | M1, M0, P>(r, e[8 + ((k.perm >> 4) & 3)],
                                            k.c[2]);
-          scale_sel_df<C, NR, M0 | M1, M0 | M1, FAST>(
+          scale_sel_df<C, NR, M0 | M1, M0 | M1, P>(
               r, e[12 + ((k.perm >> 6) & 3)], k.c[3]);
         }
         return;
       case 2:
-        scale_sel_df<C, NR, M0 | M1, 0, FAST>(r, e[0], k.c[0]);
-        scale_sel_df<C, NR, M0 | M1, M1, FAST>(r, e[5], k.c[1]);
-        scale_sel_df<C, NR, M0 | M1, M0, FAST>(r, e[10], k.c[2]);
-        scale_sel_df<C, NR, M0 | M1, M0 | M1, FAST>(r, e[15], k.c[3]);
+        scale_sel_df<C, NR, M0 | M1, 0, P>(r, e[0], k.c[0]);
+        scale_sel_df<C, NR, M0 | M1, M1, P>(r, e[5], k.c[1]);
+        scale_sel_df<C, NR, M0 | M1, M0, P>(r, e[10], k.c[2]);
+        scale_sel_df<C, NR, M0 | M1, M0 | M1, P>(r, e[15], k.c[3]);
         return;
       case 3:
-        apply_2x2_df<C, NR, RB1, M0, M0, FAST>(r, e[10], e[11], e[14], e[15],
+        apply_2x2_df<C, NR, RB1, M0, M0, P>(r, e[10], e[11], e[14], e[15],
                                          k.sub, k.c);
         return;
       default:
@@ -553,12 +564,11 @@ __device__ __forceinline__ void apply_c128_df(C* r, const DEC* e,
           DC a[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            a[j] = df_split2<FAST>(r[idx[j]].x, r[idx[j]].y);
+            a[j] = df_split2<P == PAIRS_FAST>(r[idx[j]].x, r[idx[j]].y);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const DC y = df_row4(e + 4 * j, a);
-            r[idx[j]].x = df_join_add(y.re);
-            r[idx[j]].y = df_join_add(y.im);
+            join_pair<P>(y, &r[idx[j]]);
           }
         }
         return;
@@ -572,6 +582,11 @@ template <int D>
 struct C128Op {
   OpKind k;
   int pairs_ok;     // entries within the pair range
+  int even;         // no component but zeros below 2^-60, and each row's
+                    // largest at least 2^-38 (or the row zero): a product
+                    // with an amplitude from 2^-40 up is then at least
+                    // 2^-100, and of terms that cancel to less their own
+                    // rounding, 2^-48 of 2^-78, is all that is left
   DEC e[D * D];     // exact triples, for the pairs
   double2 raw[D * D];  // the entries, for the FP64 form
 };
@@ -586,17 +601,31 @@ __device__ __forceinline__ void c128_prologue(const C* ops,
   const int lane = threadIdx.x & 31;
   int cls = EC_ZERO;
   uint32_t mag = 0;
+  bool small = false;  // a component not zero, but below 2^-60
   if (lane < D * D) {
     const C mj = __ldg(ops + lane);
     cls = entry_class(mj);
     op.e[lane] = df_entry2(mj.x, mj.y);
     op.raw[lane] = mj;
-    mag = max(df_hiword(mj.x) & 0x7fffffffu, df_hiword(mj.y) & 0x7fffffffu);
+    const uint32_t mr = df_hiword(mj.x) & 0x7fffffffu;
+    const uint32_t mi = df_hiword(mj.y) & 0x7fffffffu;
+    mag = max(mr, mi);
+    constexpr uint32_t LEAST = (1023u - 60) << 20;
+    small = (mr && mr < LEAST) || (mi && mi < LEAST);
   }
   const uint32_t mx = __reduce_max_sync(0xffffffffu, mag);
   const uint32_t p0 = __ballot_sync(0xffffffffu, cls & 1);
   const uint32_t p1 = __ballot_sync(0xffffffffu, cls & 2);
   const uint32_t p2 = __ballot_sync(0xffffffffu, cls & 4);
+  const uint32_t large = __ballot_sync(0xffffffffu, mag >= ((1023u - 38) << 20));
+  const uint32_t some = __ballot_sync(0xffffffffu, mag != 0);
+  const uint32_t tiny = __ballot_sync(0xffffffffu, small);
+  bool even = tiny == 0;
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    const uint32_t row = ((1u << D) - 1) << (D * j);
+    even = even && ((large & row) || !(some & row));
+  }
   int cl[D * D];
 #pragma unroll
   for (int j = 0; j < D * D; ++j)
@@ -604,6 +633,7 @@ __device__ __forceinline__ void c128_prologue(const C* ops,
   if (lane == 0) {
     op.k = classify_classes<K>(cl);
     op.pairs_ok = mx >= (DF_EMIN << 20) && mx < ((DF_EMAX + 1) << 20);
+    op.even = even;
   }
   __syncwarp();
 }
@@ -621,14 +651,17 @@ __device__ __forceinline__ bool pairs_in_range(const C* r) {
 }
 
 // Whether every component's exponent is in [DF_EMIN, DF_EMAX]: none is zero
-// or small, so the split needs no special cases.
-template <typename C, int NR>
+// or small, so the split needs no special cases.  ZEROS: or it is zero.
+template <typename C, int NR, bool ZEROS = false>
 __device__ __forceinline__ bool pairs_all_in_range(const C* r) {
   constexpr uint32_t LOW = DF_EMIN << 21;  // in units of 2 * hiword
+  auto above = [](double x) {
+    const uint32_t e = df_hiword(x) * 2;
+    return ZEROS && e == 0 ? 0 : e - LOW;
+  };
   uint32_t mx = 0;
 #pragma unroll
-  for (int i = 0; i < NR; ++i)
-    mx = max(mx, max(df_hiword(r[i].x) * 2 - LOW, df_hiword(r[i].y) * 2 - LOW));
+  for (int i = 0; i < NR; ++i) mx = max(mx, max(above(r[i].x), above(r[i].y)));
   return mx < ((DF_EMAX + 1 - DF_EMIN) << 21);
 }
 
@@ -812,8 +845,10 @@ __global__ void __launch_bounds__(256, 3)
 // are the conversions between doubles and pairs (69% busy, DRAM 62%).  Where
 // a whole warp's amplitudes are in the middle of the pairs' range the split
 // has no special cases, and the join is an FP64 addition: 3 states of 24
-// qubits (HBM alone 241 us) H 320 -> 279, RX 315 -> 274, RZ 333 -> 273, a
-// full matrix 397 -> 354 us; gates that only move 262 us as before.
+// qubits (HBM alone 241 us) H 320 -> 277, RX 315 -> 281, RZ 333 -> 276, a
+// full matrix 397 -> 356 us; gates that only move 262 us as before.  Where
+// amplitudes are zero the split stays general (H 320, RZ 312 us), and only
+// what is small or uneven goes back through df_join2.
 constexpr int C128_STAGES = 3;    // slots per warp: two in flight, one in use
 constexpr int C128_THREADS = 256;
 constexpr int C128_BLOCK = 128;   // amplitudes per warp step
@@ -916,6 +951,7 @@ __global__ void __launch_bounds__(C128_THREADS, 2)
   c128_prologue<C, K>(ops, op);
   const OpKind kind = op.k;
   const bool pairs_mode = a.df != 0 && op.pairs_ok;
+  const bool even = pairs_mode && kind.arith && op.even;
 
   for (int k = 0; ws < a.total_steps; ++k, ws += nw) {
     C* const S = slot + (k % C128_STAGES) * C128_BLOCK;
@@ -929,11 +965,16 @@ __global__ void __launch_bounds__(C128_THREADS, 2)
 
     bool pairs = pairs_mode;
     const bool all =
-        pairs && kind.arith &&
-        __all_sync(0xffffffffu, pairs_all_in_range<C, 4>(r));
-    if (pairs && kind.arith && !all) pairs = pairs_in_range<C, 4>(r);
+        even && __all_sync(0xffffffffu, pairs_all_in_range<C, 4>(r));
+    const bool zeros =
+        even && !all &&
+        __all_sync(0xffffffffu, pairs_all_in_range<C, 4, true>(r));
+    if (pairs && kind.arith && !all && !zeros)
+      pairs = pairs_in_range<C, 4>(r);
     if (all)
-      apply_c128_df<C, 4, K, RB0, RB1, true>(r, op.e, kind);
+      apply_c128_df<C, 4, K, RB0, RB1, PAIRS_FAST>(r, op.e, kind);
+    else if (zeros)
+      apply_c128_df<C, 4, K, RB0, RB1, PAIRS_ZEROS>(r, op.e, kind);
     else if (pairs || !kind.arith)
       apply_c128_df<C, 4, K, RB0, RB1>(r, op.e, kind);
     else
@@ -1079,8 +1120,7 @@ __global__ void __launch_bounds__(128)
           for (int r = 0; r < D; ++r) {
             const DC y = df_rowD<D>(msd + r * D, xs);
             C o;
-            o.x = df_join_add(y.re);
-            o.y = df_join_add(y.im);
+            df_join2(y, &o);
             dst[offs[r]] = o;
           }
         } else {

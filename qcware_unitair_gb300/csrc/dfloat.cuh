@@ -22,7 +22,8 @@
 //     error terms, then one fast renormalisation (Dekker's Fast2Sum);
 //   * df_join: pair -> double by integer operations on the bit pattern of
 //     hi, adding lo as a rounded integer number of double ulps of hi
-//     (df_join_add: by one FP64 addition, for kernels bound by the ALU).
+//     (df_join_add, df_join2: by one FP64 addition, for kernels bound by the
+//     ALU).
 //
 // The relative error of one gate is a few units of 2^-47, unbiased; the
 // complex128 engine keeps native FP64 arithmetic as an option
@@ -343,8 +344,10 @@ GBSV_HD double df_join(DF x) {
 // that moves its state between every split and join is bound by the ALU
 // pipe (82 of its integer operations per amplitude were conversions, with
 // the FP64 pipe idle), and this takes half of df_join's; the fused stages,
-// which join once per stage, are faster with df_join.  A zero or subnormal
-// word counts as up to 2^-126 (hi: exactly zero).
+// which join once per stage, are faster with df_join.  df_widen takes a zero
+// or subnormal low word for up to 2^-126, at most 2^-127 too much (hi:
+// exactly zero), so this is for values that are zero, at least 2^-101, or
+// no more than the rounding of larger terms; df_join2 is for any.
 GBSV_HD double df_widen(uint32_t b) {
 #ifdef __CUDA_ARCH__
   uint64_t w;  // one multiply-add for the shift and the exponent's rebias
@@ -373,6 +376,20 @@ struct DC {
 struct DEC {
   DE re, im;
 };
+
+// Both components to doubles: by addition where both are at least 2^-101,
+// else by df_join, so that no magnitude has a larger error than there.
+template <typename C>
+GBSV_HD void df_join2(const DC& a, C* y) {
+  const uint32_t r = df_fbits(a.re.hi) << 1, i = df_fbits(a.im.hi) << 1;
+  if ((r < i ? r : i) >= (26u << 24)) {
+    y->x = df_widen(df_fbits(a.re.hi)) + df_widen(df_fbits(a.re.lo));
+    y->y = df_widen(df_fbits(a.im.hi)) + df_widen(df_fbits(a.im.lo));
+  } else {
+    y->x = df_join(a.re);
+    y->y = df_join(a.im);
+  }
+}
 
 template <bool FAST = false>
 GBSV_HD DC df_split2(double re, double im) {
