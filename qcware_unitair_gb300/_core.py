@@ -48,6 +48,18 @@ def require_cuda(*tensors: torch.Tensor) -> torch.device:
     return dev
 
 
+def dense(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as the kernels read it: contiguous memory that holds its values.
+    conj(), and what autograd hands to a backward, may be lazy: a bit on the
+    tensor over unchanged memory, which contiguous() keeps."""
+    return t.resolve_conj().resolve_neg().contiguous()
+
+
+def lazy(t: torch.Tensor) -> bool:
+    """Whether t's memory holds something else than its values."""
+    return t.is_conj() or t.is_neg()
+
+
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 

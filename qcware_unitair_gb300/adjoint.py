@@ -292,7 +292,7 @@ ROT_DTYPE = np.dtype([("gen", "<i4"), ("nv", "<i4"), ("pidx", "<i4"),
 
 def _real_params(params: torch.Tensor) -> torch.Tensor:
     """Parameters as the kernels read them: contiguous float32/float64."""
-    p = params.detach().contiguous()
+    p = _core.dense(params.detach())
     if p.dtype not in (torch.float32, torch.float64):
         p = p.to(torch.float64)
     return p
@@ -324,7 +324,7 @@ def _initial_state(n, B, dtype, device, psi0):
     s = psi0.to(device=device, dtype=dtype)
     if s.dim() == 1:
         s = s.expand(B, -1)
-    return s.reshape(B, 2 ** n).contiguous()
+    return _core.dense(s.reshape(B, 2 ** n))
 
 
 def _forward(pc: ParamCircuit, params, dtype, psi0, checkpoints: bool,
@@ -371,8 +371,9 @@ def _pauli_apply(H: PauliSum, psi: torch.Tensor, out: torch.Tensor):
 
 def pauli_expectation(H: PauliSum, psi: torch.Tensor) -> torch.Tensor:
     """<psi|H|psi> per state (float64, FP64 accumulation)."""
+    psi = _core.dense(psi)
     lam = torch.empty_like(psi)
-    _pauli_apply(H, psi.contiguous(), lam)
+    _pauli_apply(H, psi, lam)
     return _real_inner(psi, lam)
 
 
@@ -404,7 +405,7 @@ def _backward_sweep(pc, params, H, psi_L, saved, dtype):
     fixed = [op for op in pc.ops if op[0] == "fixed"]
     dag = {}
     if fixed:
-        flat = [op[1].conj().T.contiguous().reshape(-1) for op in fixed]
+        flat = [_core.dense(op[1].conj().T).reshape(-1) for op in fixed]
         host = torch.cat(flat).to(dtype)
         if dev.type == "cuda":
             host = host.pin_memory()
@@ -840,7 +841,7 @@ def _backward_fused(pc, params, H, psi_L, saved, dtype, lam=None):
                 _lib.check(rc, "adjoint_rotation_step")
             else:
                 _, m_, qs, _k = entry[1]
-                md = m_.conj().T.contiguous().to(device=dev, dtype=dtype)
+                md = _core.dense(m_.conj().T).to(device=dev, dtype=dtype)
                 wide = not _core.inplace_ok(dtype, len(qs), n)
                 dst = torch.empty_like(both) if wide else both
                 rc = L.gbsv_apply_operator(

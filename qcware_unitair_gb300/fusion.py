@@ -442,7 +442,8 @@ def _circuit_desc(gates: Sequence[CircuitGate]):
     parts = []
     off = 0
     for i, g in enumerate(gates):
-        mat = g.matrix.detach().numpy().astype(np.complex128, copy=False)
+        mat = _core.dense(g.matrix.detach()).numpy().astype(np.complex128,
+                                                        copy=False)
         d = mat.shape[-1]
         desc[i] = (_KIND_CODE[g.kind], len(g.qubits), g.qubits[0],
                    g.qubits[1] if len(g.qubits) > 1 else 0, off,
@@ -584,7 +585,7 @@ class Program:
                                   int(op["first"]), int(op["count"]))
             if t == 0:
                 g = gates[first]
-                mat = g.matrix.to(dtype=dt).contiguous()
+                mat = _core.dense(g.matrix.to(dtype=dt))
                 if dev.type == "cuda":
                     mat = mat.pin_memory()
                 self.ops.append(("plain", mat.to(dev, non_blocking=True),
@@ -612,7 +613,7 @@ class Program:
 
     # -- packing ---------------------------------------------------------
     def _plain_op(self, g):
-        mat = g.matrix.to(dtype=self.dtype).contiguous()
+        mat = _core.dense(g.matrix.to(dtype=self.dtype))
         if self.device.type == "cuda" and not mat.is_cuda:
             mat = mat.pin_memory()
         return ("plain", mat.to(self.device, non_blocking=True), g.qubits)
@@ -661,7 +662,7 @@ class Program:
             """values (nv,) or (B, nv) -> (offset, bstride).  Host values
             stay on the host until one transfer at the end."""
             nonlocal pool_len
-            v = values.to(dtype=dt)
+            v = values.to(dtype=dt).resolve_conj()
             off = pool_len
             pool_parts.append(v.reshape(-1))
             pool_len += v.numel()
@@ -673,7 +674,7 @@ class Program:
         for kind, item in raw:
             if kind == "plain":
                 g = item
-                mat = g.matrix.to(dtype=dt).contiguous()
+                mat = _core.dense(g.matrix.to(dtype=dt))
                 if dev.type == "cuda" and not mat.is_cuda:
                     mat = mat.pin_memory()
                 mat = mat.to(dev, non_blocking=True)
@@ -761,10 +762,12 @@ class Program:
         if inplace:
             if not state.is_contiguous():
                 raise ValueError("in-place run needs a contiguous state")
+            if _core.lazy(state):
+                return state.copy_(self.run(state, False, renorm_every))
             out = state
         else:
             out = torch.empty_like(state, memory_format=torch.contiguous_format)
-        src = state.contiguous()
+        src = _core.dense(state)
         if B == 0:
             return out
         L = _lib.load()

@@ -24,7 +24,7 @@ def sample(state: torch.Tensor, num_samples: int,
         raise ValueError("measure samples one state; index the batch first")
     if seed is None:
         seed = int(torch.randint(0, 2 ** 62, (1,)).item())
-    s = state.contiguous()
+    s = _core.dense(state)
     if s.data_ptr() % 16:  # a view at an odd offset: vector loads need 16
         s = s.clone()
     out = torch.empty(int(num_samples), dtype=torch.int64, device=s.device)

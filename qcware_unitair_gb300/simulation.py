@@ -77,7 +77,7 @@ class _BatchPlan:
             self.out_batch = op_batch
             self.in_stride = 0
             self.state_expanded = True
-            self.ops = operator.contiguous()
+            self.ops = _core.dense(operator)
             self.op_stride = d * d if _prod(op_batch) > 1 else 0
         else:
             extra = len(op_batch) - len(state_batch)
@@ -98,13 +98,13 @@ class _BatchPlan:
             self.out_batch = state_batch
             self.in_stride = N
             if _prod(op_batch) == 1:
-                self.ops = operator.reshape(d, d).contiguous()
+                self.ops = _core.dense(operator.reshape(d, d))
                 self.op_stride = 0
             elif tuple(op_batch) == state_batch:
-                self.ops = operator.contiguous()
+                self.ops = _core.dense(operator)
                 self.op_stride = d * d
             else:
-                self.ops = operator.expand(state_batch + (d, d)).contiguous()
+                self.ops = _core.dense(operator.expand(state_batch + (d, d)))
                 self.op_stride = d * d
         self.num_states = _prod(self.out_batch)
 
@@ -157,13 +157,13 @@ def _op_grad(gop, plan, tail, target):
 
 
 def _dagger(ops: torch.Tensor) -> torch.Tensor:
-    return ops.conj().transpose(-1, -2).resolve_conj().contiguous()
+    return _core.dense(ops.conj().transpose(-1, -2))
 
 
 def _apply_forward(operator, state, qubits, n, k):
     """The forward launch; returns (out, plan, contiguous state)."""
     plan = _BatchPlan(operator, state, n, k)
-    state_c = state.contiguous()
+    state_c = _core.dense(state)
     out = torch.empty(plan.out_batch + (2 ** n,), dtype=state.dtype,
                       device=state.device)
     if plan.num_states:
@@ -187,7 +187,7 @@ class _ApplyOperator(torch.autograd.Function):
     def backward(ctx, g):
         (state_c,) = ctx.saved_tensors
         plan, n, k, qubits = ctx.plan, ctx.n, ctx.k, ctx.qubits
-        g = g.contiguous()
+        g = _core.dense(g)
         grad_op = grad_state = None
         if plan.num_states == 0:
             return (torch.zeros(ctx.op_shape, dtype=g.dtype, device=g.device),
@@ -264,10 +264,12 @@ def apply_operator_(operator: torch.Tensor, qubits: Iterable[int],
         raise ValueError("apply_operator_ cannot broadcast an unbatched "
                          "state over an operator batch")
     if plan.num_states:
-        wide = not _core.inplace_ok(state.dtype, k, n, plan.op_stride != 0)
-        if wide:  # this operator is not applied in place
-            out = torch.empty_like(state)
-            _launch_apply(plan.ops, plan.op_stride, state, 2 ** n, out, n,
+        wide = _core.lazy(state) or not _core.inplace_ok(
+            state.dtype, k, n, plan.op_stride != 0)
+        if wide:  # this operator, or this view, is not applied in place
+            src = _core.dense(state)
+            out = torch.empty_like(src)
+            _launch_apply(plan.ops, plan.op_stride, src, 2 ** n, out, n,
                           qubits, plan.num_states)
             state.copy_(out)
         else:
@@ -296,9 +298,9 @@ def _all_qubits_plan(operator, state, n, each):
     if not each:
         return plan, plan.ops, plan.op_stride, 0
     if plan.op_stride:
-        ops = operator.expand(plan.out_batch + (n, 2, 2)).contiguous()
+        ops = _core.dense(operator.expand(plan.out_batch + (n, 2, 2)))
         return plan, ops, n * 4, 4
-    return plan, operator.reshape(n, 2, 2).contiguous(), 0, 4
+    return plan, _core.dense(operator.reshape(n, 2, 2)), 0, 4
 
 
 def _apply_all_qubits_kernel(operator, state, n, each):
@@ -306,7 +308,7 @@ def _apply_all_qubits_kernel(operator, state, n, each):
     (complex64; one launch per qubit otherwise)."""
     plan, ops, op_stride, op_qubit_stride = _all_qubits_plan(operator, state,
                                                              n, each)
-    state_c = state.contiguous()
+    state_c = _core.dense(state)
     out = torch.empty(plan.out_batch + (2 ** n,), dtype=state.dtype,
                       device=state.device)
     if plan.num_states:
@@ -328,7 +330,7 @@ class _ApplyAllQubits(torch.autograd.Function):
     def forward(ctx, operator, state, n, each, passes):
         plan, ops, op_stride, op_qubit_stride = _all_qubits_plan(
             operator, state, n, each)
-        state_c = state.contiguous()
+        state_c = _core.dense(state)
         shape = plan.out_batch + (2 ** n,)
         outs = [torch.empty(shape, dtype=state.dtype, device=state.device)
                 for _ in range(passes)]
@@ -349,7 +351,7 @@ class _ApplyAllQubits(torch.autograd.Function):
         entered = ctx.saved_tensors
         plan, n, each, ops = ctx.plan, ctx.n, ctx.each, ctx.ops
         op_stride, op_qubit_stride = ctx.strides
-        g = g.contiguous()
+        g = _core.dense(g)
         need_op, need_state = ctx.needs_input_grad[:2]
         grad_op = gs = None
         L = _lib.load()
@@ -474,7 +476,7 @@ class _ApplyPhase(torch.autograd.Function):
         if torch.is_grad_enabled():  # create_graph: keep ga differentiable
             ga = gs = None
             if need_state:
-                gs = _phase_kernel(-angles, g.contiguous())
+                gs = _phase_kernel(-angles, g)
                 gs = gs.to(state.dtype).sum_to_size(state.shape)
             if need_angles:
                 ga = (1j * g * out.conj()).real.to(angles.dtype)
@@ -482,8 +484,8 @@ class _ApplyPhase(torch.autograd.Function):
             return ga, gs
         # out = exp(-i a) psi  =>  dL/dpsi = exp(i a) g and
         # dL/da = Re(i * g * conj(out)), both from one read of g
-        a = _phase_angles(angles).contiguous()
-        g = g.contiguous()
+        a = _core.dense(_phase_angles(angles))
+        g = _core.dense(g)
         gs = torch.empty_like(g) if need_state else None
         ga = torch.empty(g.shape, dtype=_core.real_of(g.dtype),
                          device=g.device) if need_angles else None
@@ -521,8 +523,8 @@ def _phase_kernel(angles: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
     out_dtype = torch.complex128 if (angles.dtype == torch.float64 or
                                      state.dtype == torch.complex128) \
         else torch.complex64
-    a = angles.contiguous()
-    s = state.contiguous()
+    a = _core.dense(angles)
+    s = _core.dense(state)
     out_shape = torch.broadcast_shapes(a.shape, s.shape)
     out = torch.empty(out_shape, dtype=out_dtype, device=dev)
     if out.numel() == 0:
@@ -550,7 +552,7 @@ def apply_phase(angles: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
 def _permute(state: torch.Tensor, perm, n: int) -> torch.Tensor:
     _core.require_cuda(state)
     code = _core.complex_code(state.dtype)
-    s = state.contiguous()
+    s = _core.dense(state)
     out = torch.empty_like(s)
     if s.numel():
         rc = _lib.load().gbsv_permute_qubits(
@@ -666,7 +668,7 @@ def _phase_flip(state: torch.Tensor, masks) -> torch.Tensor:
     n = count_qubits(state)
     _core.require_cuda(state)
     code = _core.complex_code(state.dtype)
-    s = state.contiguous()
+    s = _core.dense(state)
     out = torch.empty_like(s)
     if s.numel() == 0:
         return out
@@ -730,7 +732,7 @@ def multi_controlled_x(state_vector: torch.Tensor, controls: Iterable[int],
                          f"{n} qubits")
     _core.require_cuda(state_vector)
     code = _core.complex_code(state_vector.dtype)
-    s = state_vector.contiguous()
+    s = _core.dense(state_vector)
     out = torch.empty_like(s)
     if s.numel():
         rc = _lib.load().gbsv_multi_controlled_x(

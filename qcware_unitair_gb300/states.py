@@ -143,7 +143,7 @@ def _scratch(rows: int, dim: int, device) -> tuple:
 def _norm_squared_kernel(state: torch.Tensor, out_dtype=None) -> torch.Tensor:
     dev = _core.require_cuda(state)
     code = _core.complex_code(state.dtype)
-    s = state.contiguous()
+    s = _core.dense(state)
     rows = s.numel() // s.shape[-1] if s.shape[-1] else 0
     real = _core.real_of(state.dtype) if out_dtype is None else out_dtype
     out = torch.empty(s.shape[:-1], dtype=real, device=dev)
@@ -163,7 +163,7 @@ def _norm_squared_kernel(state: torch.Tensor, out_dtype=None) -> torch.Tensor:
 def _abs_squared_kernel(state: torch.Tensor) -> torch.Tensor:
     dev = _core.require_cuda(state)
     code = _core.complex_code(state.dtype)
-    s = state.contiguous()
+    s = _core.dense(state)
     out = torch.empty(s.shape, dtype=_core.real_of(state.dtype), device=dev)
     if s.numel() == 0:
         return out
@@ -194,8 +194,8 @@ def _inner_product_kernel(a: torch.Tensor, b: torch.Tensor,
             f"expected both states to have one dtype, got {a.dtype} and "
             f"{b.dtype}")
     code = _core.complex_code(a.dtype)
-    a = a.contiguous()
-    b = b.contiguous()
+    a = _core.dense(a)
+    b = _core.dense(b)
     rows_shape, desc, dim, ia, ib = _row_broadcast(a, b)
     out_dtype = a.dtype if out_dtype is None else out_dtype
     out = torch.empty(rows_shape, dtype=out_dtype, device=dev)
@@ -221,8 +221,8 @@ def _diag_expectation_kernel(diag: torch.Tensor,
                                   "pass the real diagonal")
     dcode = _core.real_code(diag.dtype)
     out_dtype = torch.promote_types(_core.real_of(state.dtype), diag.dtype)
-    d = diag.contiguous()
-    s = state.contiguous()
+    d = _core.dense(diag)
+    s = _core.dense(state)
     rows_shape, desc, dim, ia, ib = _row_broadcast(d, s)
     out = torch.empty(rows_shape, dtype=out_dtype, device=dev)
     rows = out.numel()
