@@ -73,6 +73,37 @@ def stream_of(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+class Uploads:
+    """Device tensors that a plan fills once, without waiting, and that any
+    stream may read afterwards: a stream's first use waits for the copies and
+    tells the allocator of it."""
+
+    def __init__(self, tensors, device: torch.device):
+        self.tensors = [t for t in tensors if t.is_cuda]
+        self.streams = set()
+        self.ready = None
+        if self.tensors and not torch.cuda.is_current_stream_capturing():
+            stream = torch.cuda.current_stream(device)
+            self.streams.add(stream.cuda_stream)
+            self.ready = torch.cuda.Event()
+            self.ready.record(stream)
+
+    def use(self, device: torch.device, stream: int) -> None:
+        """Before work that reads the tensors goes to ``stream``, the current
+        one of ``device``.  A capture starts after what it reads is there
+        (torch.cuda.graph waits for the device), and cannot wait for an event
+        from outside."""
+        if self.ready is None or stream in self.streams:
+            return
+        current = torch.cuda.current_stream(device)
+        for t in self.tensors:
+            t.record_stream(current)
+        if torch.cuda.is_current_stream_capturing():
+            return
+        current.wait_event(self.ready)
+        self.streams.add(stream)
+
+
 def ptr(t: torch.Tensor) -> int:
     return t.data_ptr()
 

@@ -221,9 +221,9 @@ _PLACEHOLDER = {
 
 def _forward_program(pc: ParamCircuit, a: int, b: int, B: int, dtype, dev,
                      fuse: bool):
-    """(Program, scatter index, rotation index) for ops [a, b) with B
-    states, planned once per structure.  Each call only writes the rotation
-    values into the program's pool."""
+    """(Program, its rotations, their gates) for ops [a, b) with B states,
+    planned once per structure.  Each call only writes the rotation values
+    into the program's pool."""
     key = (a, b, B, dtype, str(dev), fuse)
     cache = pc.__dict__.setdefault("_fwd_cache", {})
     if key in cache:
@@ -247,6 +247,8 @@ def _forward_program(pc: ParamCircuit, a: int, b: int, B: int, dtype, dev,
         else:
             off, nv = None, 4
         which.append((op[1], op[3], op[4], off, nv))
+    if fuse and which:
+        _rotation_records(prog, which)
     cache[key] = (prog, which, rots)
     return cache[key]
 
@@ -298,21 +300,27 @@ def _real_params(params: torch.Tensor) -> torch.Tensor:
     return p
 
 
+def _rotation_records(prog, which):
+    """The program's rotations as gbsv_rotation_values reads them, on the
+    device."""
+    from .fusion import _to_device
+    recs = [(GEN[gen], nv, pi, 0, off, 0.5 * scale)
+            for gen, pi, scale, off, nv in which]
+    prog._rot_recs = _to_device(np.array(recs, ROT_DTYPE).view(np.uint8),
+                                prog.pool.device)
+    prog._rot_uploads = _core.Uploads([prog._rot_recs], prog.pool.device)
+
+
 def _write_rotations(prog, which, p):
     """Every rotation's matrices written into the program's pool by one
     kernel (sin and cos in FP64)."""
-    from .fusion import _to_device
-    recs = prog.__dict__.get("_rot_recs")
-    if recs is None:
-        host = np.zeros(len(which), dtype=ROT_DTYPE)
-        for i, (gen, pi, scale, off, nv) in enumerate(which):
-            host[i] = (GEN[gen], nv, pi, 0, off, 0.5 * scale)
-        recs = prog._rot_recs = _to_device(host.view(np.uint8),
-                                           prog.pool.device)
+    dev, stream = p.device, _core.stream_of(p.device)
+    prog._rot_uploads.use(dev, stream)
+    prog._uploads.use(dev, stream)
     rc = _lib.load().gbsv_rotation_values(
         p.data_ptr(), _core.real_code(p.dtype), p.shape[1], p.shape[0],
-        recs.data_ptr(), len(which), prog.pool.data_ptr(),
-        _core.complex_code(prog.dtype), _core.stream_of(p.device))
+        prog._rot_recs.data_ptr(), len(which), prog.pool.data_ptr(),
+        _core.complex_code(prog.dtype), stream)
     _lib.check(rc, "rotation_values")
 
 
@@ -723,8 +731,9 @@ _PARTIAL_BYTES = 64 << 20
 
 
 def _segment_plan(pc, a, b, dtype, dev, m):
-    """Entries of the backward sweep over ops [a, b) and their register
-    plan (None: not all of them have one), made once per circuit."""
+    """Entries of the backward sweep over ops [a, b), their register plan
+    (None: not all of them have one) and what of them is on the device, made
+    once per circuit."""
     cache = pc.__dict__.setdefault("_adj_cache", {})
     key = (a, b, dtype, str(dev), m)
     if key not in cache:
@@ -732,11 +741,15 @@ def _segment_plan(pc, a, b, dtype, dev, m):
         plan = (_plan_backward_native if host else _plan_backward)(
             pc, a, b, dtype, dev, m, device_ops=False)
         regs = _register_plan(plan, m, dtype, dev)
+        stages = [st for kind, st in plan if kind == "stage"]
         if regs is None:
-            for kind, st in plan:
-                if kind == "stage":
-                    _device_stage(st, dev)
-        cache[key] = (plan, regs)
+            for st in stages:
+                _device_stage(st, dev)
+        held = {id(t): t for st in stages for t in st.values()
+                if isinstance(t, torch.Tensor)}
+        uploads = _core.Uploads([*held.values()] + (
+            [regs["buf"]] if regs is not None else []), dev)
+        cache[key] = (plan, regs, uploads)
     return cache[key]
 
 
@@ -753,7 +766,7 @@ def _backward_fused(pc, params, H, psi_L, saved, dtype, lam=None):
     plans = [_segment_plan(pc, a, b, dtype, dev, m) for a, b in segs]
     # gates outside the stages run on psi and lambda as one batch
     owned = lam is not None and all(
-        entry[0] in ("stage", "rot") for plan, _ in plans for entry in plan)
+        entry[0] in ("stage", "rot") for plan, *_ in plans for entry in plan)
     if owned:
         psi = psi_L
     else:
@@ -771,7 +784,8 @@ def _backward_fused(pc, params, H, psi_L, saved, dtype, lam=None):
     tiles = B << (n - m)
     scratch = partial = None
     for si in range(len(segs) - 1, -1, -1):
-        entries, regs = plans[si]
+        entries, regs, uploads = plans[si]
+        uploads.use(dev, stream)
         if regs is not None and regs["total"]:
             buf0, at = regs["buf"].data_ptr(), regs["at"]
             total = regs["total"]

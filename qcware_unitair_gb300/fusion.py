@@ -607,9 +607,8 @@ class Program:
             pool = pool.pin_memory()
         self._staging = pool
         self.pool = pool.to(dev, non_blocking=True)
-        self.num_stages = sum(1 for o in self.ops if o[0] != "plain")
-        self.num_plain = sum(1 for o in self.ops if o[0] == "plain")
         self.native = True
+        self._finish()
 
     # -- packing ---------------------------------------------------------
     def _plain_op(self, g):
@@ -645,9 +644,9 @@ class Program:
         self.gate_records = self.layout_records = _to_device(None, dev)
         self.num_layouts = 0
         self.pool = torch.zeros(1, dtype=self.dtype, device=dev)
-        self.num_stages = sum(1 for o in self.ops if o[0] != "plain")
-        self.num_plain = sum(1 for o in self.ops if o[0] == "plain")
         self.tensor_cores = True
+        self._finish(self.tc_blocks, self.tc_diags, self.tc_images,
+                     self.tc_factors)
 
     def _build(self, raw):
         n, dev, dt = self.n, self.device, self.dtype
@@ -728,8 +727,15 @@ class Program:
             self._staging = host  # alive until the copy has run
         else:
             self.pool = torch.cat([p.to(dev) for p in pool_parts])
-        self.num_stages = sum(1 for o in self.ops if o[0] != "plain")
-        self.num_plain = sum(1 for o in self.ops if o[0] == "plain")
+        self._finish()
+
+    def _finish(self, *tensors):
+        plain = [o[1] for o in self.ops if o[0] == "plain"]
+        self.num_plain = len(plain)
+        self.num_stages = len(self.ops) - len(plain)
+        self._uploads = _core.Uploads(
+            [self.gate_records, self.layout_records, self.pool, *plain,
+             *tensors], self.device)
 
     @property
     def num_passes(self) -> int:
@@ -772,6 +778,7 @@ class Program:
             return out
         L = _lib.load()
         stream = _core.stream_of(state.device)
+        self._uploads.use(state.device, stream)
         N = 2 ** self.n
         cur = src
         if not self.ops and cur is not out:
@@ -810,8 +817,9 @@ class Program:
         """One pass of the program (an entry of ``ops``), in place on a
         contiguous state: for timing the stages one at a time."""
         B = state.numel() >> self.n
-        self._run_op(op, state, state, B, 2 ** self.n, _lib.load(),
-                     _core.stream_of(state.device))
+        stream = _core.stream_of(state.device)
+        self._uploads.use(state.device, stream)
+        self._run_op(op, state, state, B, 2 ** self.n, _lib.load(), stream)
 
     def _run_op(self, op, cur, out, B, N, L, stream):
         gp = self.gate_records.data_ptr()
