@@ -552,6 +552,15 @@ int gbsv_rotation_values(const void* params, int params_dtype,
                          const void* rots, int64_t num_rots, void* pool,
                          int dtype, void* stream);
 
+/* The same into a pool of the call's own: records of gen 3 copy nv entries
+ * at off from `base` (their pidx and half are not looked at), so that the
+ * records together fill the pool.  Calls that run at the same time, on
+ * streams or threads of their own, then share only what nobody writes. */
+int gbsv_rotation_pool(const void* params, int params_dtype,
+                       int64_t num_params, int64_t num_states,
+                       const void* rots, int64_t num_rots, const void* base,
+                       void* pool, int dtype, void* stream);
+
 /* Scratch bytes gbsv_adjoint_rotation_step needs. */
 size_t gbsv_adjoint_scratch_bytes(int64_t num_states, int num_qubits);
 

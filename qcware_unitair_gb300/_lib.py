@@ -126,6 +126,8 @@ SIGNATURES = {
     "gbsv_pauli_sum_apply_host": (_I, [_P, _P, _I, _I, _I64, _P, _I, _P]),
     "gbsv_rotation_values": (_I, [_P, _I, _I64, _I64, _P, _I64, _P, _I,
                                   _P]),
+    "gbsv_rotation_pool": (_I, [_P, _I, _I64, _I64, _P, _I64, _P, _P, _I,
+                                _P]),
     "gbsv_adjoint_scratch_bytes": (_SZ, [_I64, _I]),
     "gbsv_adjoint_rotation_step": (_I, [_P, _P, _I, _I, _I64, _I, _I, _P, _I,
                                         _I64, ctypes.c_double, _P, _I64,

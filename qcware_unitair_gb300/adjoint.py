@@ -222,8 +222,8 @@ _PLACEHOLDER = {
 def _forward_program(pc: ParamCircuit, a: int, b: int, B: int, dtype, dev,
                      fuse: bool):
     """(Program, its rotations, their gates) for ops [a, b) with B states,
-    planned once per structure.  Each call only writes the rotation values
-    into the program's pool."""
+    planned once per structure.  Each call only fills a pool of gate values
+    (_call_pool)."""
     key = (a, b, B, dtype, str(dev), fuse)
     cache = pc.__dict__.setdefault("_fwd_cache", {})
     if key in cache:
@@ -248,7 +248,7 @@ def _forward_program(pc: ParamCircuit, a: int, b: int, B: int, dtype, dev,
             off, nv = None, 4
         which.append((op[1], op[3], op[4], off, nv))
     if fuse and which:
-        _rotation_records(prog, which)
+        _rotation_records(prog, which, B)
     cache[key] = (prog, which, rots)
     return cache[key]
 
@@ -300,28 +300,52 @@ def _real_params(params: torch.Tensor) -> torch.Tensor:
     return p
 
 
-def _rotation_records(prog, which):
-    """The program's rotations as gbsv_rotation_values reads them, on the
-    device."""
+def _rotation_records(prog, which, B):
+    """The records that fill a pool for this program, on the device: its
+    rotations, then copies of what lies between them, four entries a
+    thread."""
     from .fusion import _to_device
     recs = [(GEN[gen], nv, pi, 0, off, 0.5 * scale)
             for gen, pi, scale, off, nv in which]
+    at = 0
+    for off, end in sorted((off, off + B * nv) for *_, off, nv in which) + [
+            (prog.pool.numel(), 0)]:
+        while at < off:
+            n = min(off - at, 4 * B)
+            recs.append((3, n, 0, 0, at, 0.0))
+            at += n
+        at = max(at, end)
     prog._rot_recs = _to_device(np.array(recs, ROT_DTYPE).view(np.uint8),
                                 prog.pool.device)
+    prog._rot_count = len(recs)
     prog._rot_uploads = _core.Uploads([prog._rot_recs], prog.pool.device)
 
 
-def _write_rotations(prog, which, p):
-    """Every rotation's matrices written into the program's pool by one
-    kernel (sin and cos in FP64)."""
+def _write_rotations(prog, which, p, pool=None):
+    """Every rotation's matrices written by one kernel (sin and cos in FP64):
+    into the program's own pool, or all of ``pool``."""
     dev, stream = p.device, _core.stream_of(p.device)
     prog._rot_uploads.use(dev, stream)
     prog._uploads.use(dev, stream)
-    rc = _lib.load().gbsv_rotation_values(
+    own = pool is None
+    rc = _lib.load().gbsv_rotation_pool(
         p.data_ptr(), _core.real_code(p.dtype), p.shape[1], p.shape[0],
-        prog._rot_recs.data_ptr(), len(which), prog.pool.data_ptr(),
+        prog._rot_recs.data_ptr(), len(which) if own else prog._rot_count,
+        None if own else prog.pool.data_ptr(),
+        (prog.pool if own else pool).data_ptr(),
         _core.complex_code(prog.dtype), stream)
     _lib.check(rc, "rotation_values")
+
+
+def _call_pool(prog, which, p):
+    """The gate values of one evaluation.  The program is shared by every
+    evaluation of its circuit, on whatever stream or thread, so what depends
+    on the parameters is not kept in it."""
+    if not which:
+        return prog.pool
+    pool = torch.empty_like(prog.pool)
+    _write_rotations(prog, which, p, pool)
+    return pool
 
 
 def _initial_state(n, B, dtype, device, psi0):
@@ -360,9 +384,7 @@ def _forward(pc: ParamCircuit, params, dtype, psi0, checkpoints: bool,
             prog.run(psi, inplace=True)
             continue
         prog, which, _ = _forward_program(pc, a, b, B, dtype, dev, fuse)
-        if which:
-            _write_rotations(prog, which, p)
-        psi = prog.run(psi, inplace=not keep)
+        psi = prog._run(psi, not keep, None, _call_pool(prog, which, p))
     return psi, saved
 
 

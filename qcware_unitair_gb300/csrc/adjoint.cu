@@ -244,9 +244,10 @@ __global__ void __launch_bounds__(256)
 // Entries of parameterised rotations, written into a program's matrix pool:
 // rotation k of state b with angle theta = 2 half * params[b, pidx] fills
 // pool[off + b nv ..] with its 2x2 (nv = 4) or diagonal (nv = 2), sin and
-// cos in FP64.
+// cos in FP64.  A record of kind 3 copies nv entries of `base`, the pool that
+// the program was made with: a call then has a pool of its own.
 struct RotRec {
-  int32_t gen;   // 0 X, 1 Y, 2 Z
+  int32_t gen;   // 0 X, 1 Y, 2 Z, 3 a copy
   int32_t nv;
   int32_t pidx;
   int32_t pad_;
@@ -258,12 +259,19 @@ template <typename R, typename P>
 __global__ void __launch_bounds__(256)
     rotation_values_kernel(const P* params, int64_t num_params,
                            int64_t num_states, const RotRec* recs,
-                           int64_t num_rots, Cx<R>* pool) {
+                           int64_t num_rots, const Cx<R>* base,
+                           Cx<R>* pool) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= num_states * num_rots) return;
   // states fastest: neighbouring threads write neighbouring pool entries
   const int64_t b = i % num_states;
   const RotRec r = recs[i / num_states];
+  if (r.gen == 3) {
+    if (base)
+      for (int64_t k = b; k < r.nv; k += num_states)
+        pool[r.off + k] = base[r.off + k];
+    return;
+  }
   double sn, cs;
   sincos((double)params[b * num_params + r.pidx] * r.half, &sn, &cs);
   const R c = (R)cs, s = (R)sn;
@@ -519,6 +527,15 @@ extern "C" int gbsv_rotation_values(const void* params, int params_dtype,
                                     int64_t num_params, int64_t num_states,
                                     const void* rots, int64_t num_rots,
                                     void* pool, int dtype, void* stream) {
+  return gbsv_rotation_pool(params, params_dtype, num_params, num_states,
+                            rots, num_rots, nullptr, pool, dtype, stream);
+}
+
+extern "C" int gbsv_rotation_pool(const void* params, int params_dtype,
+                                  int64_t num_params, int64_t num_states,
+                                  const void* rots, int64_t num_rots,
+                                  const void* base, void* pool, int dtype,
+                                  void* stream) {
   if ((dtype != GBSV_C64 && dtype != GBSV_C128) ||
       (params_dtype != GBSV_F32 && params_dtype != GBSV_F64))
     return set_error(GBSV_ERR_INVALID_ARG, "bad dtype");
@@ -534,7 +551,8 @@ extern "C" int gbsv_rotation_values(const void* params, int params_dtype,
 #define GBSV_ROT(R, P)                                                     \
   rotation_values_kernel<R, P><<<(unsigned)grid, 256, 0, st>>>(            \
       static_cast<const P*>(params), num_params, num_states,               \
-      static_cast<const RotRec*>(rots), num_rots, static_cast<Cx<R>*>(pool))
+      static_cast<const RotRec*>(rots), num_rots,                          \
+      static_cast<const Cx<R>*>(base), static_cast<Cx<R>*>(pool))
   if (dtype == GBSV_C64) {
     if (params_dtype == GBSV_F32) GBSV_ROT(float, float);
     else GBSV_ROT(float, double);

@@ -754,6 +754,10 @@ class Program:
         unitary circuit preserves the norm; rounding over thousands of gates
         drifts it.  ``renorm_drift()`` reports the largest relative drift
         the checkpoints removed."""
+        return self._run(state, inplace, renorm_every, self.pool)
+
+    def _run(self, state, inplace, renorm_every, pool):
+        """``run`` with the gates' values in ``pool``."""
         _core.require_cuda(state)
         if state.dtype != self.dtype:
             raise RuntimeError(f"program compiled for {self.dtype}, state is "
@@ -769,7 +773,8 @@ class Program:
             if not state.is_contiguous():
                 raise ValueError("in-place run needs a contiguous state")
             if _core.lazy(state):
-                return state.copy_(self.run(state, False, renorm_every))
+                return state.copy_(self._run(state, False, renorm_every,
+                                             pool))
             out = state
         else:
             out = torch.empty_like(state, memory_format=torch.contiguous_format)
@@ -791,7 +796,7 @@ class Program:
             scratch = torch.empty(max(nbytes, 16), dtype=torch.uint8,
                                   device=state.device)
         for i, op in enumerate(self.ops):
-            self._run_op(op, cur, out, B, N, L, stream)
+            self._run_op(op, cur, out, B, N, L, stream, pool)
             cur = out
             if (renorm_every and (i + 1) % int(renorm_every) == 0
                     and i + 1 < len(self.ops)):
@@ -819,12 +824,13 @@ class Program:
         B = state.numel() >> self.n
         stream = _core.stream_of(state.device)
         self._uploads.use(state.device, stream)
-        self._run_op(op, state, state, B, 2 ** self.n, _lib.load(), stream)
+        self._run_op(op, state, state, B, 2 ** self.n, _lib.load(), stream,
+                     self.pool)
 
-    def _run_op(self, op, cur, out, B, N, L, stream):
+    def _run_op(self, op, cur, out, B, N, L, stream, pool):
         gp = self.gate_records.data_ptr()
         lp = self.layout_records.data_ptr()
-        pool = self.pool.data_ptr()
+        pool = pool.data_ptr()
         if op[0] == "stage":
             _, c, positions, first, count = op
             rc = L.gbsv_run_stage(cur.data_ptr(), out.data_ptr(),

@@ -1,6 +1,9 @@
-"""One circuit or program used on several streams: what is cached on it is
-uploaded before another stream reads it.  Against the same calls one after another,
+"""One circuit evaluated on several streams and threads at once: each call's
+rotation values are its own, and what is cached on the circuit is uploaded
+before another stream reads it.  Against the same calls one after another,
 bit for bit (the same kernels on the same values)."""
+import threading
+
 import pytest
 import torch
 
@@ -42,6 +45,67 @@ def same(got, want):
     for g, w in zip(got, want):
         for a, b in zip(g, w):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n,layers,batch", [(6, 3, 4), (14, 4, 8)])
+def test_streams(n, layers, batch):
+    pc, H = circuit(n, layers)
+    params = inputs(pc, batch)
+    want = [evaluate(pc, H, p) for p in params]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(CALLS)]
+    for _ in range(3):
+        got = []
+        for s, p in zip(streams, params):
+            with torch.cuda.stream(s):
+                got.append(evaluate(pc, H, p))
+        torch.cuda.synchronize()
+        same(got, want)
+
+
+@pytest.mark.parametrize("n,layers,batch", [(6, 3, 4), (12, 4, 8)])
+def test_threads_on_one_stream(n, layers, batch):
+    pc, H = circuit(n, layers)
+    params = inputs(pc, batch)
+    want = [evaluate(pc, H, p) for p in params]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        got = [None] * CALLS
+        start = threading.Barrier(CALLS)
+
+        def run(i):
+            start.wait()
+            got[i] = evaluate(pc, H, params[i])
+
+        threads = [threading.Thread(target=run, args=(i,))
+                   for i in range(CALLS)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        same(got, want)
+
+
+@pytest.mark.parametrize("first", [0, 1])
+def test_cached_uploads_behind_other_work(first):
+    """The first call, on a stream that is behind, plans and uploads; the
+    second, on an idle stream, must not read before the copies."""
+    pc, H = circuit(13, 4)
+    params = inputs(pc, 4)
+    want = evaluate(*circuit(13, 4), params[1])
+    torch.cuda.synchronize()
+    late, idle = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(late):
+        busy(30)
+        if first:
+            evaluate(pc, H, params[0])
+        else:
+            ad.expectation(pc, params[0], H)
+    with torch.cuda.stream(idle):
+        got = evaluate(pc, H, params[1])
+    torch.cuda.synchronize()
+    same([got], [want])
 
 
 @pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
