@@ -78,12 +78,29 @@ bool plain(const Tensor& t) {
 }
 
 // The tensor of a Python argument, if it is exactly a Tensor or Parameter.
-const Tensor* unpack(PyObject* o) {
+Tensor unpack(PyObject* o) {
   if (!THPVariable_CheckExact(o) &&
       reinterpret_cast<PyObject*>(Py_TYPE(o)) != ParameterClass)
-    return nullptr;
+    return Tensor();
   const Tensor& t = THPVariable_Unpack(o);
-  return plain(t) ? &t : nullptr;
+  return plain(t) ? t : Tensor();
+}
+
+// Other Python threads run while a call allocates and launches: both can
+// wait for the device (a full allocator, a full queue, behind which a host
+// callback may need the interpreter).  The same calls through ctypes do so.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+template <typename F>
+PyObject* without_gil(F f) {
+  Tensor out;
+  {
+    const WithoutGil w;
+    out = f();
+  }
+  return THPVariable_Wrap(std::move(out));
 }
 
 bool needs_grad(const Tensor& a, const Tensor& b) {
@@ -299,22 +316,22 @@ PyObject* none() { Py_RETURN_NONE; }
 PyObject* py_apply_operator(PyObject*, PyObject* const* args, Py_ssize_t na) {
   GBSV_CALL
   if (na != 3 || !plain_context()) return none();
-  const Tensor* op = unpack(args[0]);
-  const Tensor* state = unpack(args[2]);
-  if (!op || !state || op->scalar_type() != state->scalar_type() ||
-      complex_code(state->scalar_type()) < 0 ||
-      op->device() != state->device() || op->dim() < 2 || state->dim() < 1)
+  const Tensor op = unpack(args[0]), state = unpack(args[2]);
+  if (!op.defined() || !state.defined() ||
+      op.scalar_type() != state.scalar_type() ||
+      complex_code(state.scalar_type()) < 0 ||
+      op.device() != state.device() || op.dim() < 2 || state.dim() < 1)
     return none();
   Gate g;
-  g.n = log2_exact(state->size(-1));
+  g.n = log2_exact(state.size(-1));
   if (g.n < 0 || g.n > 62 || !parse_qubits(args[1], g.n, g.q.data(), &g.k) ||
-      op->size(-1) != (int64_t(1) << g.k) || op->size(-2) != op->size(-1) ||
-      !plan(*op, 2, int64_t(1) << (2 * g.k), *state, g.n, &g.b))
+      op.size(-1) != (int64_t(1) << g.k) || op.size(-2) != op.size(-1) ||
+      !plan(op, 2, int64_t(1) << (2 * g.k), state, g.n, &g.b))
     return none();
-  if (needs_grad(*op, *state))
-    return THPVariable_Wrap(ApplyOperator::apply(*op, *state, g));
-  return THPVariable_Wrap(
-      run_gate(op->contiguous(), state->contiguous(), g));
+  return without_gil([&]() -> Tensor {
+    if (needs_grad(op, state)) return ApplyOperator::apply(op, state, g);
+    return run_gate(op.contiguous(), state.contiguous(), g);
+  });
   GBSV_END_CALL
 }
 
@@ -404,44 +421,51 @@ struct ApplyLayer : public Function<ApplyLayer> {
 PyObject* py_apply_layer(PyObject*, PyObject* const* args, Py_ssize_t na) {
   GBSV_CALL
   if (na != 3 || !plain_context()) return none();
-  const Tensor* op = unpack(args[0]);
-  const Tensor* state = unpack(args[1]);
+  const Tensor op = unpack(args[0]), state = unpack(args[1]);
   const bool each = args[2] == Py_True;
   const int tail = each ? 3 : 2;
-  if (!op || !state || op->scalar_type() != state->scalar_type() ||
-      complex_code(state->scalar_type()) < 0 ||
-      op->device() != state->device() || op->dim() < tail ||
-      state->dim() < 1 || op->size(-1) != 2 || op->size(-2) != 2)
+  if (!op.defined() || !state.defined() ||
+      op.scalar_type() != state.scalar_type() ||
+      complex_code(state.scalar_type()) < 0 ||
+      op.device() != state.device() || op.dim() < tail || state.dim() < 1 ||
+      op.size(-1) != 2 || op.size(-2) != 2)
     return none();
   Layer l;
-  l.n = log2_exact(state->size(-1));
-  if (l.n < 1 || l.n > 62 || (each && op->size(-3) != l.n) ||
-      !plan(*op, tail, each ? 4 * l.n : 4, *state, l.n, &l.b))
+  l.n = log2_exact(state.size(-1));
+  if (l.n < 1 || l.n > 62 || (each && op.size(-3) != l.n) ||
+      !plan(op, tail, each ? 4 * l.n : 4, state, l.n, &l.b))
     return none();
   l.op_qstride = each ? 4 : 0;
-  const int code = complex_code(state->scalar_type());
-  if (needs_grad(*op, *state)) {
-    const int passes = gbsv_all_qubits_passes(code, l.n);
-    if (!passes) return none();  // one node per qubit, in Python
-    return THPVariable_Wrap(ApplyLayer::apply(*op, *state, l, passes));
-  }
-  const Tensor ops = op->contiguous(), sc = state->contiguous();
-  Tensor out = at::empty(l.b.out, state->options());
-  check(gbsv_apply_all_qubits(sc.data_ptr(), out.data_ptr(), code, l.n,
-                              l.b.num_states, l.b.in_stride, ops.data_ptr(),
-                              l.b.op_stride, l.op_qstride, stream_of(sc)),
-        "apply_all_qubits");
-  return THPVariable_Wrap(out);
+  const int code = complex_code(state.scalar_type());
+  const bool grad = needs_grad(op, state);
+  const int passes = grad ? gbsv_all_qubits_passes(code, l.n) : 0;
+  if (grad && !passes) return none();  // one node per qubit, in Python
+  return without_gil([&]() -> Tensor {
+    if (grad) return ApplyLayer::apply(op, state, l, passes);
+    const Tensor ops = op.contiguous(), sc = state.contiguous();
+    Tensor out = at::empty(l.b.out, state.options());
+    check(gbsv_apply_all_qubits(sc.data_ptr(), out.data_ptr(), code, l.n,
+                                l.b.num_states, l.b.in_stride, ops.data_ptr(),
+                                l.b.op_stride, l.op_qstride, stream_of(sc)),
+          "apply_all_qubits");
+    return out;
+  });
   GBSV_END_CALL
 }
 
 // ------------------------------------------------------- broadcasting ----
-// Element strides of a contiguous tensor broadcast to `shape`.
+// Element strides of t, made contiguous, broadcast to `shape`.
 Sizes bcast_strides(const Tensor& t, c10::IntArrayRef shape) {
   const int64_t nd = (int64_t)shape.size(), off = nd - t.dim();
   Sizes s(nd, 0);
-  for (int64_t i = 0; i < t.dim(); ++i)
-    s[off + i] = t.size(i) == 1 && shape[off + i] != 1 ? 0 : t.stride(i);
+  const bool dense = t.is_contiguous();
+  int64_t stride = 1;
+  for (int64_t i = t.dim() - 1; i >= 0; --i) {
+    s[off + i] = t.size(i) == 1 && shape[off + i] != 1 ? 0
+                 : dense                               ? t.stride(i)
+                                                       : stride;
+    stride *= t.size(i);
+  }
   return s;
 }
 
@@ -557,22 +581,20 @@ struct ApplyPhase : public Function<ApplyPhase> {
 PyObject* py_apply_phase(PyObject*, PyObject* const* args, Py_ssize_t na) {
   GBSV_CALL
   if (na != 2 || !plain_context()) return none();
-  const Tensor* a = unpack(args[0]);
-  const Tensor* s = unpack(args[1]);
-  if (!a || !s || a->device() != s->device() ||
-      real_code(a->scalar_type()) < 0 || complex_code(s->scalar_type()) < 0 ||
-      a->numel() == 0 || s->numel() == 0)
+  const Tensor a = unpack(args[0]), s = unpack(args[1]);
+  if (!a.defined() || !s.defined() || a.device() != s.device() ||
+      real_code(a.scalar_type()) < 0 || complex_code(s.scalar_type()) < 0 ||
+      a.numel() == 0 || s.numel() == 0)
     return none();
-  const auto shape = broadcast(*a, *s);
-  if (!shape) return none();
-  const Tensor ac = a->contiguous(), sc = s->contiguous();
+  const auto shape = broadcast(a, s);
   gbsv_bcast_t d;
-  if (!bcast_desc(*shape, bcast_strides(ac, *shape),
-                  bcast_strides(sc, *shape), &d))
+  if (!shape || !bcast_desc(*shape, bcast_strides(a, *shape),
+                            bcast_strides(s, *shape), &d))
     return none();
-  if (needs_grad(*a, *s))
-    return THPVariable_Wrap(ApplyPhase::apply(*a, *s, *shape, d));
-  return THPVariable_Wrap(run_phase(ac, sc, *shape, d));
+  return without_gil([&]() -> Tensor {
+    if (needs_grad(a, s)) return ApplyPhase::apply(a, s, *shape, d);
+    return run_phase(a.contiguous(), s.contiguous(), *shape, d);
+  });
   GBSV_END_CALL
 }
 
@@ -625,33 +647,37 @@ struct AbsSquared : public Function<AbsSquared> {
 };
 
 // A complex state of at least one amplitude.
-const Tensor* state_arg(PyObject* o) {
-  const Tensor* s = unpack(o);
-  return s && s->dim() >= 1 && s->numel() > 0 &&
-                 complex_code(s->scalar_type()) >= 0
+Tensor state_arg(PyObject* o) {
+  const Tensor s = unpack(o);
+  return s.defined() && s.dim() >= 1 && s.numel() > 0 &&
+                 complex_code(s.scalar_type()) >= 0
              ? s
-             : nullptr;
+             : Tensor();
 }
 
 PyObject* py_norm_squared(PyObject*, PyObject* const* args, Py_ssize_t na) {
   GBSV_CALL
-  const Tensor* s = na == 1 && plain_context() ? state_arg(args[0]) : nullptr;
-  if (!s) return none();
-  return THPVariable_Wrap(needs_grad(*s) ? NormSquared::apply(*s)
-                                         : run_norm(*s));
+  const Tensor s =
+      na == 1 && plain_context() ? state_arg(args[0]) : Tensor();
+  if (!s.defined()) return none();
+  return without_gil([&]() -> Tensor {
+    return needs_grad(s) ? NormSquared::apply(s) : run_norm(s);
+  });
   GBSV_END_CALL
 }
 
 PyObject* py_abs_squared(PyObject*, PyObject* const* args, Py_ssize_t na) {
   GBSV_CALL
-  const Tensor* s = na == 1 && plain_context() ? state_arg(args[0]) : nullptr;
-  if (!s) return none();
-  return THPVariable_Wrap(needs_grad(*s) ? AbsSquared::apply(*s)
-                                         : run_abs(*s));
+  const Tensor s =
+      na == 1 && plain_context() ? state_arg(args[0]) : Tensor();
+  if (!s.defined()) return none();
+  return without_gil([&]() -> Tensor {
+    return needs_grad(s) ? AbsSquared::apply(s) : run_abs(s);
+  });
   GBSV_END_CALL
 }
 
-// Rows of two broadcast (*batch, dim) tensors.
+// Rows of two broadcast (*batch, dim) tensors, made contiguous.
 struct Rows {
   Sizes shape;  // without the inner dim
   gbsv_bcast_t d;
@@ -703,17 +729,16 @@ struct InnerProduct : public Function<InnerProduct> {
 PyObject* py_inner_product(PyObject*, PyObject* const* args, Py_ssize_t na) {
   GBSV_CALL
   if (na != 2 || !plain_context()) return none();
-  const Tensor* a = state_arg(args[0]);
-  const Tensor* b = state_arg(args[1]);
-  if (!a || !b || a->scalar_type() != b->scalar_type() ||
-      a->device() != b->device())
+  const Tensor a = state_arg(args[0]), b = state_arg(args[1]);
+  if (!a.defined() || !b.defined() || a.scalar_type() != b.scalar_type() ||
+      a.device() != b.device())
     return none();
-  const Tensor ac = a->contiguous(), bc = b->contiguous();
   Rows r;
-  if (!plan_rows(ac, bc, &r)) return none();
-  if (needs_grad(*a, *b))
-    return THPVariable_Wrap(InnerProduct::apply(*a, *b, r));
-  return THPVariable_Wrap(run_inner(ac, bc, r));
+  if (!plan_rows(a, b, &r)) return none();
+  return without_gil([&]() -> Tensor {
+    if (needs_grad(a, b)) return InnerProduct::apply(a, b, r);
+    return run_inner(a.contiguous(), b.contiguous(), r);
+  });
   GBSV_END_CALL
 }
 
@@ -754,17 +779,16 @@ struct DiagExpectation : public Function<DiagExpectation> {
 PyObject* py_diag(PyObject*, PyObject* const* args, Py_ssize_t na) {
   GBSV_CALL
   if (na != 2 || !plain_context()) return none();
-  const Tensor* d = unpack(args[0]);
-  const Tensor* s = state_arg(args[1]);
-  if (!d || !s || d->dim() < 1 || d->numel() == 0 ||
-      real_code(d->scalar_type()) < 0 || d->device() != s->device())
+  const Tensor d = unpack(args[0]), s = state_arg(args[1]);
+  if (!d.defined() || !s.defined() || d.dim() < 1 || d.numel() == 0 ||
+      real_code(d.scalar_type()) < 0 || d.device() != s.device())
     return none();
-  const Tensor dc = d->contiguous(), sc = s->contiguous();
   Rows r;
-  if (!plan_rows(dc, sc, &r)) return none();
-  if (needs_grad(*d, *s))
-    return THPVariable_Wrap(DiagExpectation::apply(*d, *s, r));
-  return THPVariable_Wrap(run_diag(dc, sc, r));
+  if (!plan_rows(d, s, &r)) return none();
+  return without_gil([&]() -> Tensor {
+    if (needs_grad(d, s)) return DiagExpectation::apply(d, s, r);
+    return run_diag(d.contiguous(), s.contiguous(), r);
+  });
   GBSV_END_CALL
 }
 
@@ -831,13 +855,14 @@ PyObject* py_rotation(PyObject*, PyObject* const* args, Py_ssize_t na) {
   if (na != 2 || !PyLong_CheckExact(args[0]) || !plain_context())
     return none();
   const long axis = PyLong_AsLong(args[0]);
-  const Tensor* a = unpack(args[1]);
-  if (!a || axis < 0 || axis > 2 || real_code(a->scalar_type()) < 0 ||
-      a->numel() == 0)
+  const Tensor a = unpack(args[1]);
+  if (!a.defined() || axis < 0 || axis > 2 || real_code(a.scalar_type()) < 0 ||
+      a.numel() == 0)
     return none();
-  return THPVariable_Wrap(needs_grad(*a)
-                              ? Rotation::apply(*a, (int64_t)axis)
-                              : run_rotation(angles_of(*a), (int)axis));
+  return without_gil([&]() -> Tensor {
+    return needs_grad(a) ? Rotation::apply(a, (int64_t)axis)
+                         : run_rotation(angles_of(a), (int)axis);
+  });
   GBSV_END_CALL
 }
 
