@@ -237,7 +237,6 @@ struct ApplyOperator : public Function<ApplyOperator> {
                           const Variable& state, const Gate& g) {
     const Tensor ops = op.contiguous(), sc = state.contiguous();
     Tensor out = run_gate(ops, sc, g);
-    ctx->saved_data["ops"] = ops.detach();
     ctx->saved_data["op_shape"] = op.sizes().vec();
     ctx->saved_data["shape"] = state.sizes().vec();
     ctx->saved_data["out"] = g.b.out;
@@ -245,13 +244,14 @@ struct ApplyOperator : public Function<ApplyOperator> {
         Sizes{g.b.num_states, g.b.in_stride, g.b.op_stride, g.b.expanded,
               g.n, g.k};
     ctx->saved_data["q"] = Sizes(g.q.begin(), g.q.begin() + g.k);
-    ctx->save_for_backward({sc});
+    // the operator enters the state's gradient only
+    ctx->save_for_backward({sc, state.requires_grad() ? ops : Tensor()});
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list gout) {
     at::NoGradGuard no_grad;
-    const Tensor sc = ctx->get_saved_variables()[0];
-    const Tensor ops = ctx->saved_data["ops"].toTensor();
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &sc = saved[0], &ops = saved[1];
     Gate g;
     const auto ints = ctx->saved_data["ints"].toIntVector();
     const auto q = ctx->saved_data["q"].toIntVector();
@@ -290,8 +290,8 @@ struct ApplyOperator : public Function<ApplyOperator> {
                       go.options());
       check(gbsv_apply_operator_grad(
                 go.data_ptr(), sc.data_ptr(), code, g.n, g.b.num_states,
-                g.b.in_stride, ops.data_ptr(), g.b.op_stride, g.q.data(),
-                g.k, both ? gs.data_ptr() : nullptr, gop.data_ptr(), shared,
+                g.b.in_stride, ptr(ops), g.b.op_stride, g.q.data(), g.k,
+                both ? gs.data_ptr() : nullptr, gop.data_ptr(), shared,
                 ptr(sp), bytes, stream_of(go)),
             "operator_grad");
     }
@@ -359,19 +359,20 @@ struct ApplyLayer : public Function<ApplyLayer> {
               l.n, l.b.num_states, l.b.in_stride, ops.data_ptr(),
               l.b.op_stride, l.op_qstride, stream_of(sc)),
           "apply_all_qubits");
-    ctx->saved_data["ops"] = ops.detach();
     ctx->saved_data["op_shape"] = op.sizes().vec();
     ctx->saved_data["shape"] = state.sizes().vec();
     ctx->saved_data["ints"] =
         Sizes{l.b.num_states, l.b.in_stride, l.b.op_stride, l.b.expanded, l.n,
               l.op_qstride};
+    kept.push_back(ops);
     ctx->save_for_backward(kept);
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list gout) {
     at::NoGradGuard no_grad;
-    const variable_list kept = ctx->get_saved_variables();
-    const Tensor ops = ctx->saved_data["ops"].toTensor();
+    variable_list kept = ctx->get_saved_variables();
+    const Tensor ops = kept.back();
+    kept.pop_back();
     const auto ints = ctx->saved_data["ints"].toIntVector();
     Batch b;
     b.num_states = ints[0];

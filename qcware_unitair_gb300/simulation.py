@@ -51,6 +51,12 @@ def _prod(shape) -> int:
     return p
 
 
+def _shaped(t: torch.Tensor, shape: tuple) -> torch.Tensor:
+    """reshape, but t itself where it has the shape: autograd keeps it, and a
+    view made inside a node is harder on later in-place changes."""
+    return t if tuple(t.shape) == shape else t.reshape(shape)
+
+
 class _BatchPlan:
     """How a (operator, state) pair maps onto the C ABI's two strides."""
 
@@ -98,7 +104,7 @@ class _BatchPlan:
             self.out_batch = state_batch
             self.in_stride = N
             if _prod(op_batch) == 1:
-                self.ops = _core.dense(operator.reshape(d, d))
+                self.ops = _core.dense(_shaped(operator, (d, d)))
                 self.op_stride = 0
             elif tuple(op_batch) == state_batch:
                 self.ops = _core.dense(operator)
@@ -180,12 +186,15 @@ class _ApplyOperator(torch.autograd.Function):
         ctx.plan = plan
         ctx.op_shape = operator.shape
         ctx.state_shape = state.shape
-        ctx.save_for_backward(state_c)
+        # the operator enters the state's gradient only
+        ops, plan.ops = plan.ops, None
+        ctx.save_for_backward(state_c, ops if ctx.needs_input_grad[1]
+                              else None)
         return out
 
     @staticmethod
     def backward(ctx, g):
-        (state_c,) = ctx.saved_tensors
+        state_c, ops = ctx.saved_tensors
         plan, n, k, qubits = ctx.plan, ctx.n, ctx.k, ctx.qubits
         g = _core.dense(g)
         grad_op = grad_state = None
@@ -198,7 +207,7 @@ class _ApplyOperator(torch.autograd.Function):
         both = (all(ctx.needs_input_grad[:2]) and k in (1, 2) and
                 g.dtype == torch.complex64)
         if gs is not None and not both:
-            _launch_apply(_dagger(plan.ops), plan.op_stride, g, 2 ** n, gs, n,
+            _launch_apply(_dagger(ops), plan.op_stride, g, 2 ** n, gs, n,
                           qubits, plan.num_states)
         if ctx.needs_input_grad[0]:
             shared = plan.op_stride == 0
@@ -213,8 +222,8 @@ class _ApplyOperator(torch.autograd.Function):
             rc = L.gbsv_apply_operator_grad(
                 g.data_ptr(), state_c.data_ptr(),
                 _core.complex_code(g.dtype), n, plan.num_states,
-                plan.in_stride, plan.ops.data_ptr(), plan.op_stride,
-                _lib.qubit_array(qubits), k,
+                plan.in_stride, ops.data_ptr() if both else None,
+                plan.op_stride, _lib.qubit_array(qubits), k,
                 gs.data_ptr() if both else None, gop.data_ptr(),
                 int(shared), scratch.data_ptr() if scratch is not None else
                 None, nbytes, _core.stream_of(g.device))
@@ -300,7 +309,7 @@ def _all_qubits_plan(operator, state, n, each):
     if plan.op_stride:
         ops = _core.dense(operator.expand(plan.out_batch + (n, 2, 2)))
         return plan, ops, n * 4, 4
-    return plan, _core.dense(operator.reshape(n, 2, 2)), 0, 4
+    return plan, _core.dense(_shaped(operator, (n, 2, 2))), 0, 4
 
 
 def _apply_all_qubits_kernel(operator, state, n, each):
@@ -341,15 +350,16 @@ class _ApplyAllQubits(torch.autograd.Function):
             _core.stream_of(state.device))
         _lib.check(rc, "apply_all_qubits")
         ctx.plan, ctx.n, ctx.each = plan, n, each
-        ctx.ops, ctx.strides = ops, (op_stride, op_qubit_stride)
+        ctx.strides = op_stride, op_qubit_stride
+        plan.ops = None
         ctx.op_shape, ctx.state_shape = operator.shape, state.shape
-        ctx.save_for_backward(state_c, *outs[:-1])
+        ctx.save_for_backward(ops, state_c, *outs[:-1])
         return outs[-1]
 
     @staticmethod
     def backward(ctx, g):
-        entered = ctx.saved_tensors
-        plan, n, each, ops = ctx.plan, ctx.n, ctx.each, ctx.ops
+        ops, *entered = ctx.saved_tensors
+        plan, n, each = ctx.plan, ctx.n, ctx.each
         op_stride, op_qubit_stride = ctx.strides
         g = _core.dense(g)
         need_op, need_state = ctx.needs_input_grad[:2]
