@@ -1166,24 +1166,18 @@ extern "C" int gbsv_adjoint_stage(
     }
   }
   if (dtype == GBSV_C64) {
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(adjoint_stage_kernel<float>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           200 * 1024);
-      attr = true;
-    }
+    static OncePerDevice once;
+    const int rc = allow_smem(once, adjoint_stage_kernel<float>, 200 * 1024,
+                              "adjoint_stage_kernel");
+    if (rc) return rc;
     adjoint_stage_kernel<float><<<(unsigned)tiles, threads, smem, st>>>(
         static_cast<float2*>(psi), static_cast<float2*>(lam),
         static_cast<const float2*>(pool), a, partial);
   } else {
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(adjoint_stage_kernel<double>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           200 * 1024);
-      attr = true;
-    }
+    static OncePerDevice once;
+    const int rc = allow_smem(once, adjoint_stage_kernel<double>, 200 * 1024,
+                              "adjoint_stage_kernel");
+    if (rc) return rc;
     adjoint_stage_kernel<double><<<(unsigned)tiles, threads, smem, st>>>(
         static_cast<double2*>(psi), static_cast<double2*>(lam),
         static_cast<const double2*>(pool), a, partial);

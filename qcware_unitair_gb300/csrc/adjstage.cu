@@ -12,7 +12,6 @@
 // intermediate state of its gates
 // (src/unitair/simulation/operations.py:45-148).
 #include <algorithm>
-#include <atomic>
 
 #include "common.cuh"
 
@@ -499,20 +498,10 @@ static int ar_launch(void* psi, void* lam, const void* pool,
     return set_error(GBSV_ERR_UNSUPPORTED,
                      "adjoint stage with %d rotations needs %zu bytes of "
                      "shared memory", a.num_slots, smem);
-  // the shared-memory opt-in, once per device (a race only repeats it)
-  static std::atomic<uint64_t> attr_set;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const uint64_t bit = uint64_t(1) << (dev & 63);
-  if (!(attr_set.load(std::memory_order_relaxed) & bit)) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        adjoint_reg_kernel<R, RB>,
-        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
-    if (e != cudaSuccess)
-      return set_error(GBSV_ERR_CUDA, "adjoint_reg_kernel: %s",
-                       cudaGetErrorString(e));
-    attr_set.fetch_or(bit, std::memory_order_relaxed);
-  }
+  static OncePerDevice once;
+  const int rc = allow_smem(once, adjoint_reg_kernel<R, RB>, (int)kMost,
+                            "adjoint_reg_kernel");
+  if (rc) return rc;
   adjoint_reg_kernel<R, RB><<<(unsigned)a.tiles, T, smem, st>>>(
       static_cast<Cx<R>*>(psi), static_cast<Cx<R>*>(lam),
       static_cast<const Cx<R>*>(pool), a);

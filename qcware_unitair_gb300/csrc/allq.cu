@@ -7,7 +7,6 @@
 // write of the state: a pass takes a tile of 2^12 amplitudes, applies the
 // operators of up to 12 of its index bits, and writes it back.
 #include <algorithm>
-#include <atomic>
 
 #include "common.cuh"
 
@@ -778,20 +777,10 @@ template <int M>
 static int aq_grad_launch(const float2* psi, const float2* gin, float2* gout,
                           const float2* ops, const AllqGradArgs& ga,
                           uint64_t ctas, cudaStream_t st) {
-  // the shared-memory opt-in, once per device (a race only repeats it)
-  static std::atomic<uint64_t> attr_set;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const uint64_t bit = uint64_t(1) << (dev & 63);
-  if (!(attr_set.load(std::memory_order_relaxed) & bit)) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        allq_grad_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        (int)AQ_GRAD_SMEM);
-    if (e != cudaSuccess)
-      return set_error(GBSV_ERR_CUDA, "allq_grad_kernel: %s",
-                       cudaGetErrorString(e));
-    attr_set.fetch_or(bit, std::memory_order_relaxed);
-  }
+  static OncePerDevice once;
+  const int rc = allow_smem(once, allq_grad_kernel<M>, (int)AQ_GRAD_SMEM,
+                            "allq_grad_kernel");
+  if (rc) return rc;
   allq_grad_kernel<M><<<(unsigned)ctas, AQ_THREADS, AQ_GRAD_SMEM, st>>>(
       psi, gin, gout, ops, ga);
   return after_launch("allq_grad_kernel");

@@ -1249,20 +1249,10 @@ static int launch_c128_stream(const void* in, void* out, int n,
                           C128_BLOCK * sizeof(double2);
   const void* fn = k == 1 ? (const void*)dense_c128_stream_kernel<1>
                           : (const void*)dense_c128_stream_kernel<2>;
-  // the shared-memory opt-in, once per device and kernel (a race only
-  // repeats it)
-  static std::atomic<uint64_t> attr_set[2];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const uint64_t bit = uint64_t(1) << (dev & 63);
-  if (!(attr_set[k - 1].load(std::memory_order_relaxed) & bit)) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess)
-      return set_error(GBSV_ERR_CUDA, "dense_c128_stream_kernel: %s",
-                       cudaGetErrorString(e));
-    attr_set[k - 1].fetch_or(bit, std::memory_order_relaxed);
-  }
+  static OncePerDevice once[2];
+  const int rc =
+      allow_smem(once[k - 1], fn, (int)smem, "dense_c128_stream_kernel");
+  if (rc) return rc;
   const uint64_t warps = C128_THREADS / 32;
   uint64_t blocks = (a.total_steps + warps - 1) / warps;
   const uint64_t cap = (uint64_t)sm_count() * 2;

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "gbsv.h"
+#include "once.h"
 
 namespace gbsv {
 
@@ -162,6 +163,22 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // Records a launch and converts a pending CUDA error into a status.
 int after_launch(const char* what);
 int set_error(int status, const char* fmt, ...);
+// Lets a kernel use `bytes` of dynamic shared memory beside its static; above
+// 48 KB that is to be allowed for each kernel and device.  `once` is a static
+// of the kernel's launch.
+template <typename Kernel>
+int allow_smem(OncePerDevice& once, Kernel kernel, int bytes,
+               const char* what) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return once(dev, [&]() -> int {
+    const cudaError_t e = cudaFuncSetAttribute(
+        kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) return GBSV_OK;
+    (void)cudaGetLastError();
+    return set_error(GBSV_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  });
+}
 // GBSV_C128_PAIRS or GBSV_C128_FP64 (gbsv_set_c128_arith)
 int c128_arith();
 // apply_all_qubits for complex64 states of n >= 4 qubits (allq.cu)

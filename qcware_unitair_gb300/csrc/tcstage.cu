@@ -1178,12 +1178,10 @@ extern "C" int gbsv_run_stage_tc(const void* state_in, void* state_out,
   // up to TW_BLOCKS images stay in shared memory beside three tile buffers;
   // longer stages stream them
   if (num_blocks <= TW_BLOCKS) {
-    static const cudaError_t attr = cudaFuncSetAttribute(
-        tc_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        TW_SMEM_BYTES);
-    if (attr != cudaSuccess)
-      return set_error(GBSV_ERR_CUDA, "tc_wide_kernel: %s",
-                       cudaGetErrorString(attr));
+    static OncePerDevice once;
+    const int rc =
+        allow_smem(once, tc_wide_kernel, TW_SMEM_BYTES, "tc_wide_kernel");
+    if (rc) return rc;
     const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)sm_count());
     tc_wide_kernel<<<(unsigned)grid, TW_THREADS, TW_SMEM_BYTES,
                      static_cast<cudaStream_t>(stream)>>>(
@@ -1191,13 +1189,10 @@ extern "C" int gbsv_run_stage_tc(const void* state_in, void* state_out,
         static_cast<float2*>(state_out), a);
     return after_launch("tc_wide_kernel");
   }
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(tc_stage_kernel,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         TC_SMEM_BYTES);
-    attr_set = true;
-  }
+  static OncePerDevice once;
+  const int rc =
+      allow_smem(once, tc_stage_kernel, TC_SMEM_BYTES, "tc_stage_kernel");
+  if (rc) return rc;
   const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)sm_count() * 2);
   tc_stage_kernel<<<(unsigned)grid, TC_ROLE_THREADS, TC_SMEM_BYTES,
                     static_cast<cudaStream_t>(stream)>>>(
