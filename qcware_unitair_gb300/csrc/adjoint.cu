@@ -94,6 +94,22 @@ __device__ __forceinline__ double pauli_sign<double>(double v, int neg) {
                           __double2loint(v));
 }
 
+// By integers: a comparison of doubles is FP64 work.
+__device__ __forceinline__ uint32_t pauli_top(float v) {
+  return __float_as_uint(v) & 0x7f800000u;
+}
+__device__ __forceinline__ uint32_t pauli_top(double v) {
+  return (uint32_t)__double2hiint(v) & 0x7ff00000u;
+}
+template <typename R, int V>
+__device__ __forceinline__ bool pauli_finite(const R* a, const R* b) {
+  uint32_t top = 0;
+#pragma unroll
+  for (int e = 0; e < V; ++e)
+    top = max(top, max(pauli_top(a[e]), pauli_top(b[e])));
+  return top < (sizeof(R) == 4 ? 0x7f800000u : 0x7ff00000u);
+}
+
 // Parity of e & (low bits of zm) for the V amplitudes of a block.
 __device__ __forceinline__ int pauli_low(int e, int zm) {
   return (e & 1 & zm) ^ ((e >> 1) & (zm >> 1) & 1);
@@ -126,8 +142,10 @@ __device__ __forceinline__ void pauli_swap(C* b, int xm) {
 // for each term the partner amplitudes y = x ^ xmask of the block are again
 // one 32-byte block, read with vector loads, their order permuted by the
 // low bits of xmask.  Z strings use the thread's own block, and X strings
-// need no signs; the terms are summed in the order given (products with a
-// zero imaginary part left out, which changes no finite sum).
+// need no signs; the terms are summed in the order given.  Products with a
+// zero imaginary part are left out, which changes no finite sum; where one is
+// not finite, every term is taken as a complex one (what is not finite stays
+// so, so a look at the sums is enough).
 template <typename R, int V>
 __device__ __forceinline__ void pauli_block_body(const Cx<R>* psi,
                                                  Cx<R>* out, uint64_t total,
@@ -156,54 +174,59 @@ __device__ __forceinline__ void pauli_block_body(const Cx<R>* psi,
     C own[V];
     load_chunk<V>(p + x, own);
     R ar[V], ai[V];
+#pragma unroll 1
+    for (bool again = false;; again = true) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) ar[e] = ai[e] = 0;
-    for (int k = 0; k < num_terms;) {
-      const int end = st[k].end;
-      if (st[k].kind == 0) {
+      for (int e = 0; e < V; ++e) ar[e] = ai[e] = 0;
+      for (int k = 0; k < num_terms;) {
+        const int end = again ? num_terms : st[k].end;
+        const int kind = again ? 2 : st[k].kind;
+        if (kind == 0) {
 #pragma unroll 2
-        for (; k < end; ++k) {
-          const uint64_t zm = st[k].zmask;
-          const int par = __popcll(x & zm) & 1;
+          for (; k < end; ++k) {
+            const uint64_t zm = st[k].zmask;
+            const int par = __popcll(x & zm) & 1;
 #pragma unroll
-          for (int e = 0; e < V; ++e) {
-            const R cr = pauli_sign(st[k].re, par ^ pauli_low(e, (int)zm));
-            ar[e] = fma(cr, own[e].x, ar[e]);
-            ai[e] = fma(cr, own[e].y, ai[e]);
+            for (int e = 0; e < V; ++e) {
+              const R cr = pauli_sign(st[k].re, par ^ pauli_low(e, (int)zm));
+              ar[e] = fma(cr, own[e].x, ar[e]);
+              ai[e] = fma(cr, own[e].y, ai[e]);
+            }
           }
-        }
-      } else if (st[k].kind == 1) {
+        } else if (kind == 1) {
 #pragma unroll 4
-        for (; k < end; ++k) {
-          const uint64_t xm = st[k].xmask;
-          C b[V];
-          load_chunk<V>(p + ((x ^ xm) & ~uint64_t(V - 1)), b);
-          pauli_swap<C, V>(b, (int)xm);
-          const R re = st[k].re;
+          for (; k < end; ++k) {
+            const uint64_t xm = st[k].xmask;
+            C b[V];
+            load_chunk<V>(p + ((x ^ xm) & ~uint64_t(V - 1)), b);
+            pauli_swap<C, V>(b, (int)xm);
+            const R re = st[k].re;
 #pragma unroll
-          for (int e = 0; e < V; ++e) {
-            ar[e] = fma(re, b[e].x, ar[e]);
-            ai[e] = fma(re, b[e].y, ai[e]);
+            for (int e = 0; e < V; ++e) {
+              ar[e] = fma(re, b[e].x, ar[e]);
+              ai[e] = fma(re, b[e].y, ai[e]);
+            }
           }
-        }
-      } else {
-        for (; k < end; ++k) {
-          const uint64_t xm = st[k].xmask, zm = st[k].zmask;
-          C b[V];
-          load_chunk<V>(p + ((x ^ xm) & ~uint64_t(V - 1)), b);
-          pauli_swap<C, V>(b, (int)xm);
-          // the sign of amplitude e's partner y = (x + e) ^ xm
-          const int par = __popcll((x ^ xm) & zm) & 1;
+        } else {
+          for (; k < end; ++k) {
+            const uint64_t xm = st[k].xmask, zm = st[k].zmask;
+            C b[V];
+            load_chunk<V>(p + ((x ^ xm) & ~uint64_t(V - 1)), b);
+            pauli_swap<C, V>(b, (int)xm);
+            // the sign of amplitude e's partner y = (x + e) ^ xm
+            const int par = __popcll((x ^ xm) & zm) & 1;
 #pragma unroll
-          for (int e = 0; e < V; ++e) {
-            const int neg = par ^ pauli_low(e, (int)zm);
-            const R cr = pauli_sign(st[k].re, neg);
-            const R ci = pauli_sign(st[k].im, neg);
-            ar[e] = fma(cr, b[e].x, fma(-ci, b[e].y, ar[e]));
-            ai[e] = fma(cr, b[e].y, fma(ci, b[e].x, ai[e]));
+            for (int e = 0; e < V; ++e) {
+              const int neg = par ^ pauli_low(e, (int)zm);
+              const R cr = pauli_sign(st[k].re, neg);
+              const R ci = pauli_sign(st[k].im, neg);
+              ar[e] = fma(cr, b[e].x, fma(-ci, b[e].y, ar[e]));
+              ai[e] = fma(cr, b[e].y, fma(ci, b[e].x, ai[e]));
+            }
           }
         }
       }
+      if (again || pauli_finite<R, V>(ar, ai)) break;
     }
     C o[V];
 #pragma unroll

@@ -1,5 +1,7 @@
-"""Amplitudes that overflow on the way through a layer or its gradient: the same infinities and NaNs as gate by gate (in the order of the
-qubits, which is the order inside a pass).  Exact."""
+"""Amplitudes that overflow on the way through a layer or its gradient, or
+that enter a Pauli sum infinite: the same infinities and NaNs as gate by gate
+(in the order of the qubits, which is the order inside a pass), or as the
+terms' complex products.  Exact where not finite."""
 import numpy as np
 import pytest
 import torch
@@ -73,3 +75,37 @@ def test_layer_state_gradients(n, operator, name):
     for q in range(n):
         loop = ug.apply_operator(adj, [q], loop)
     equal(got, loop)
+
+
+@pytest.mark.parametrize("dtype", [torch.complex64, torch.complex128])
+@pytest.mark.parametrize("n", [1, 2, 3, 8, 13])
+def test_pauli_sums(n, dtype):
+    """A real coefficient is multiplied as the complex number it is: an
+    infinite partner gives NaN in the other component."""
+    from qcware_unitair_gb300.adjoint import PauliSum, _pauli_apply
+    rng = np.random.default_rng(n)
+    psi = torch.from_numpy(rng.normal(size=(3, 2 ** n, 2)) @ [1, 1j]).to(
+        dtype).to(DEV)
+    psi[1, 1] = complex(float("inf"), 0.5)
+    psi[2, 0] = complex(0.25, float("nan"))
+    H = PauliSum(n).z(0).add(0.5, {0: "X"}).add(-2.0, {n - 1: "Y"}).z(
+        n - 1, 0.3)
+    got = _pauli_apply(H, psi, torch.empty_like(psi))
+    x = np.arange(2 ** n)
+    re, im = np.zeros((2, 3, 2 ** n))
+    host = psi.cpu().numpy().astype(complex)
+    for t in H.term_array():
+        y = x ^ int(t["x"])
+        sign = 1 - 2 * (np.array([bin(v & int(t["z"])).count("1")
+                                  for v in y]) & 1)
+        a, b = host[:, y].real * sign, host[:, y].imag * sign
+        with np.errstate(invalid="ignore"):
+            re, im = (re + (t["re"] * a - t["im"] * b),
+                      im + (t["re"] * b + t["im"] * a))
+    eps = 1e-5 if dtype == torch.complex64 else 1e-13
+    for g, w in ((got.real, re), (got.imag, im)):
+        g = g.cpu().numpy().astype(float)
+        assert np.array_equal(np.isnan(g), np.isnan(w))
+        fin = np.isfinite(w)
+        assert np.array_equal(g[~fin & ~np.isnan(w)], w[~fin & ~np.isnan(w)])
+        assert np.abs(g[fin] - w[fin]).max(initial=0) < eps
