@@ -670,11 +670,12 @@ __device__ __forceinline__ bool pairs_all_in_range(const C* r) {
 // the zeros halves the FP64 operations, which bound this path.  The choice
 // is per warp (a choice per thread is turned into selects that run every
 // form), and where an amplitude is not finite, so that a product with zero
-// is not zero, the full form runs.
+// is not zero, the full form runs.  Every lane of the warp comes here; one
+// without a unit (not `live`) goes along with any form.
 template <typename C, int NR, int T>
-__device__ __forceinline__ void apply_own_2x2(C* r, const C* m) {
+__device__ __forceinline__ void apply_own_2x2(C* r, const C* m, bool live) {
   constexpr int B = 1 << T;
-  const unsigned lanes = __activemask();
+  constexpr unsigned lanes = 0xffffffffu;
   // by integers: a comparison of doubles is FP64 work
   auto zero = [](double x) {
     return ((df_hiword(x) << 1) | df_loword(x)) == 0;
@@ -683,14 +684,14 @@ __device__ __forceinline__ void apply_own_2x2(C* r, const C* m) {
   const bool im1 = zero(m[1].x) && zero(m[2].x);
   const bool real03 = zero(m[0].y) && zero(m[3].y);
   int form = re1 && im1 ? 3 : !real03 ? 0 : re1 ? 1 : im1 ? 2 : 0;
-  if (__any_sync(lanes, form != 0)) {
+  if (__any_sync(lanes, live && form != 0)) {
 #pragma unroll
     for (int i = 0; i < NR; ++i)
       if ((df_hiword(r[i].x) & 0x7ff00000u) == 0x7ff00000u ||
           (df_hiword(r[i].y) & 0x7ff00000u) == 0x7ff00000u)
         form = 0;
   }
-  if (__all_sync(lanes, form == 1)) {  // real
+  if (__all_sync(lanes, !live || form == 1)) {  // real
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
       if (i & B) continue;
@@ -700,7 +701,7 @@ __device__ __forceinline__ void apply_own_2x2(C* r, const C* m) {
       r[i | B].x = fma(m[3].x, a1.x, m[2].x * a0.x);
       r[i | B].y = fma(m[3].x, a1.y, m[2].x * a0.y);
     }
-  } else if (__all_sync(lanes, form == 2)) {  // real, imaginary off-diagonal
+  } else if (__all_sync(lanes, !live || form == 2)) {  // real, imaginary off-diagonal
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
       if (i & B) continue;
@@ -710,7 +711,7 @@ __device__ __forceinline__ void apply_own_2x2(C* r, const C* m) {
       r[i | B].x = fma(m[3].x, a1.x, -(m[2].y * a0.y));
       r[i | B].y = fma(m[3].x, a1.y, m[2].y * a0.x);
     }
-  } else if (__all_sync(lanes, form == 3)) {  // diagonal
+  } else if (__all_sync(lanes, !live || form == 3)) {  // diagonal
 #pragma unroll
     for (int i = 0; i < NR; ++i) r[i] = cmul(i & B ? m[3] : m[0], r[i]);
   } else {
@@ -802,15 +803,18 @@ __global__ void __launch_bounds__(256, 3)
 #pragma unroll
   for (int u = 0; u < UNROLL; ++u) {
     const uint64_t g = first + (uint64_t)u * blockDim.x;
-    if (g >= a.total_units) break;
+    const bool live = g < a.total_units;
+    if (!live && (shared_op || !(kC128 && K == 1))) break;
     if (!shared_op) {
-      const C* mp = ops + state[u] * a.op_stride;
+      const C* mp = ops + (live ? state[u] * a.op_stride : 0);
 #pragma unroll
       for (int j = 0; j < D * D; ++j) m[j] = __ldg(mp + j);
-      if constexpr (kC128 && K == 1)
-        apply_own_2x2<C, NR, RB0>(reg[u], m);
-      else
+      if constexpr (kC128 && K == 1) {
+        apply_own_2x2<C, NR, RB0>(reg[u], m, live);
+        if (!live) continue;
+      } else {
         apply_regs<C, NR, K, RB0, RB1>(reg[u], m);
+      }
     } else if constexpr (!kC128) {
       apply_regs<C, NR, K, RB0, RB1>(reg[u], m);
     }
