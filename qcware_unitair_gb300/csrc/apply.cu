@@ -185,6 +185,9 @@ enum {
   PAIRS_ZEROS,  // each component is zero or in [2^-40, 2^61),
   PAIRS_FAST    // or in it, and the operator's entries are C128Op::even
 };
+// C128Op::even's bounds, as high words
+constexpr uint32_t PAIRS_LEAST = (1023u - 60) << 20;
+constexpr uint32_t PAIRS_LARGE = (1023u - 38) << 20;
 template <int P, typename C>
 __device__ __forceinline__ void join_pair(const DC& y, C* r) {
   if constexpr (P == PAIRS_ANY) {
@@ -610,14 +613,13 @@ __device__ __forceinline__ void c128_prologue(const C* ops,
     const uint32_t mr = df_hiword(mj.x) & 0x7fffffffu;
     const uint32_t mi = df_hiword(mj.y) & 0x7fffffffu;
     mag = max(mr, mi);
-    constexpr uint32_t LEAST = (1023u - 60) << 20;
-    small = (mr && mr < LEAST) || (mi && mi < LEAST);
+    small = (mr && mr < PAIRS_LEAST) || (mi && mi < PAIRS_LEAST);
   }
   const uint32_t mx = __reduce_max_sync(0xffffffffu, mag);
   const uint32_t p0 = __ballot_sync(0xffffffffu, cls & 1);
   const uint32_t p1 = __ballot_sync(0xffffffffu, cls & 2);
   const uint32_t p2 = __ballot_sync(0xffffffffu, cls & 4);
-  const uint32_t large = __ballot_sync(0xffffffffu, mag >= ((1023u - 38) << 20));
+  const uint32_t large = __ballot_sync(0xffffffffu, mag >= PAIRS_LARGE);
   const uint32_t some = __ballot_sync(0xffffffffu, mag != 0);
   const uint32_t tiny = __ballot_sync(0xffffffffu, small);
   bool even = tiny == 0;
@@ -655,14 +657,34 @@ __device__ __forceinline__ bool pairs_in_range(const C* r) {
 template <typename C, int NR, bool ZEROS = false>
 __device__ __forceinline__ bool pairs_all_in_range(const C* r) {
   constexpr uint32_t LOW = DF_EMIN << 21;  // in units of 2 * hiword
-  auto above = [](double x) {
-    const uint32_t e = df_hiword(x) * 2;
-    return ZEROS && e == 0 ? 0 : e - LOW;
-  };
-  uint32_t mx = 0;
+  constexpr uint32_t SPAN = (DF_EMAX + 1 - DF_EMIN) << 21;
+  uint32_t mx = 0, mn = ~0u;
 #pragma unroll
-  for (int i = 0; i < NR; ++i) mx = max(mx, max(above(r[i].x), above(r[i].y)));
-  return mx < ((DF_EMAX + 1 - DF_EMIN) << 21);
+  for (int i = 0; i < NR; ++i) {
+    const uint32_t x = df_hiword(r[i].x) * 2, y = df_hiword(r[i].y) * 2;
+    if constexpr (ZEROS) {
+      mx = max(mx, max(x, y));
+      mn = min(mn, min(x - 1, y - 1));  // zero: the largest
+    } else {
+      mx = max(mx, max(x - LOW, y - LOW));
+    }
+  }
+  return ZEROS ? mx < LOW + SPAN && mn >= LOW - 1 : mx < SPAN;
+}
+
+// Whether no component's exponent is below DF_EMIN but a zero's (in
+// dense_group_kernel, bound by the ALU pipe, beside pairs_in_range's look).
+template <typename C, int NR>
+__device__ __forceinline__ bool pairs_none_small(const C* r) {
+  auto below = [](double x) {  // zero: the largest
+    uint32_t e;  // a multiply-add, off the ALU pipe
+    asm("mad.lo.u32 %0, %1, 2, -1;" : "=r"(e) : "r"(df_hiword(x)));
+    return e;
+  };
+  uint32_t mn = ~0u;
+#pragma unroll
+  for (int i = 0; i < NR; ++i) mn = min(mn, min(below(r[i].x), below(r[i].y)));
+  return mn >= (DF_EMIN << 21) - 1;
 }
 
 // A 2x2 of its own for each state, FP64.  Rotations have entries that are
@@ -849,9 +871,9 @@ __global__ void __launch_bounds__(256, 3)
 // are the conversions between doubles and pairs (69% busy, DRAM 62%).  Where
 // a whole warp's amplitudes are in the middle of the pairs' range the split
 // has no special cases, and the join is an FP64 addition: 3 states of 24
-// qubits (HBM alone 241 us) H 320 -> 277, RX 315 -> 281, RZ 333 -> 276, a
+// qubits (HBM alone 241 us) H 320 -> 279, RX 315 -> 279, RZ 333 -> 276, a
 // full matrix 397 -> 356 us; gates that only move 262 us as before.  Where
-// amplitudes are zero the split stays general (H 320, RZ 312 us), and only
+// amplitudes are zero the split stays general (H 314, RZ 304 us), and only
 // what is small or uneven goes back through df_join2.
 constexpr int C128_STAGES = 3;    // slots per warp: two in flight, one in use
 constexpr int C128_THREADS = 256;
@@ -1085,17 +1107,22 @@ __global__ void __launch_bounds__(128)
   constexpr bool kC128 = sizeof(R) == 8;
   __shared__ DEC msd[kC128 ? D * D : 1];
   bool bad = false;
+  bool uneven = false;  // C128Op::even, more strictly: a component not zero
+                        // and below 2^-38
   if (shared_op)
     for (int i = tid; i < D * D; i += blockDim.x) {
       const C mv = ops[i];
       msm[i] = mv;
       if constexpr (kC128) {
         msd[i] = df_entry2(mv.x, mv.y);
-        bad |= max(df_hiword(mv.x) & 0x7ff00000u,
-                   df_hiword(mv.y) & 0x7ff00000u) >= ((DF_EMAX + 1) << 20);
+        const uint32_t x = df_hiword(mv.x) & 0x7fffffffu;
+        const uint32_t y = df_hiword(mv.y) & 0x7fffffffu;
+        bad |= max(x, y) >= ((DF_EMAX + 1) << 20);
+        uneven |= (x && x < PAIRS_LARGE) || (y && y < PAIRS_LARGE);
       }
     }
   bad = __syncthreads_or(bad);
+  if constexpr (kC128) uneven = __syncthreads_or(uneven);
   const int n = a.n;
   const uint64_t gps = uint64_t(1) << (n - K);  // groups per state
   const uint64_t total = (a.total >> n) * gps;
@@ -1117,15 +1144,28 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
         for (int b = 0; b < D; ++b) x[b] = src[offs[b]];
         if (pairs_in_range<C, D>(x)) {
+          const bool zeros = !uneven && pairs_none_small<C, D>(x);
           DC xs[D];
 #pragma unroll
           for (int b = 0; b < D; ++b) xs[b] = df_split2(x[b].x, x[b].y);
+          // a loop for each join: a branch in it (df_join2) keeps the rows
+          // from overlapping (24 qubits, k = 3: 282 us, with it 309)
+          if (zeros) {
 #pragma unroll 2
-          for (int r = 0; r < D; ++r) {
-            const DC y = df_rowD<D>(msd + r * D, xs);
-            C o;
-            df_join2(y, &o);
-            dst[offs[r]] = o;
+            for (int r = 0; r < D; ++r) {
+              C o;
+              join_pair<PAIRS_ZEROS>(df_rowD<D>(msd + r * D, xs), &o);
+              dst[offs[r]] = o;
+            }
+          } else {
+#pragma unroll 2
+            for (int r = 0; r < D; ++r) {
+              const DC y = df_rowD<D>(msd + r * D, xs);
+              C o;
+              o.x = df_join(y.re);
+              o.y = df_join(y.im);
+              dst[offs[r]] = o;
+            }
           }
         } else {
 #pragma unroll 2
