@@ -669,15 +669,24 @@ struct TcGate {
 };
 
 constexpr int TCP_BITS = 5, TCP_TILE = 12, TCP_BLOCKS = 64;
+// Gates of a list that is looked through whole when blocks are compared.
+constexpr size_t TCP_WHOLE = 512;
+
+uint64_t tc_dense(const std::vector<TcGate>& g) {
+  uint64_t m = 0;
+  for (const TcGate& x : g) m |= x.diag ? 0 : x.m;
+  return m;
+}
 
 // Walks the gates in order and reports what a block on positions B takes:
 // gates inside B, and diagonals disjoint from B (which commute with the
 // block and cost nothing).  A gate may pass those left behind when it shares
 // no position with them, or when both are diagonal there.  f(index, post).
+// Ends where the dense gates left behind touch all of `all`.
 template <typename F>
 void tc_scan(const std::vector<TcGate>& g, uint64_t B, uint64_t all, F f) {
   uint64_t dense = 0, diag = 0;  // positions of the gates left behind
-  for (size_t i = 0; i < g.size() && dense != all; ++i) {
+  for (size_t i = 0; i < g.size() && (!all || (dense & all) != all); ++i) {
     const TcGate& x = g[i];
     if (!(x.m & (x.diag ? dense : dense | diag))) {
       if (!(x.m & ~B)) {
@@ -719,7 +728,7 @@ uint64_t tc_best(const std::vector<TcGate>& g, uint64_t all, uint64_t tile,
       v.push_back(m);
   };
   uint64_t dense = 0, diag = 0;
-  for (size_t i = 0; i < g.size() && dense != all; ++i) {
+  for (size_t i = 0; i < g.size() && (!all || (dense & all) != all); ++i) {
     if (!(g[i].m & (g[i].diag ? dense : dense | diag))) add(seeds, g[i].m, 24);
     add(grow, g[i].m, 48);
     (g[i].diag ? diag : dense) |= g[i].m;
@@ -788,17 +797,23 @@ extern "C" int gbsv_plan_tc(const uint64_t* masks, const uint8_t* diagonal,
     return GBSV_ERR_INVALID_ARG;
   const uint64_t low = (uint64_t(1) << min_contiguous) - 1;
   std::vector<TcGate> left;
-  uint64_t all = 0;
+  uint64_t touched = 0;
   for (int i = 0; i < num_gates; ++i) {
     const int k = __builtin_popcountll(masks[i]);
     if (k > TCP_BITS || __builtin_popcountll(low | masks[i]) > TCP_TILE)
       return GBSV_ERR_UNSUPPORTED;
     left.push_back(TcGate{masks[i], diagonal[i] != 0, i});
-    all |= masks[i];
+    touched |= masks[i];
   }
   uint64_t tile = low;
   int s = 0, b = 0;  // current stage and its number of blocks
   while (!left.empty()) {
+    // A qubit without dense gates is never left behind, and a long list
+    // would be looked through to its end for every candidate (quadratic:
+    // 10,000 gates 6.6 s, of which a quarter of the gates diagonal on one
+    // such qubit).  What its diagonals add is not counted there then; the
+    // block takes them all the same, below.
+    const uint64_t all = left.size() > TCP_WHOLE ? tc_dense(left) : touched;
     double v = 0, fresh = 0;
     uint64_t B = b < TCP_BLOCKS ? tc_best(left, all, tile, &v) : 0;
     if (b > 0) {
@@ -812,7 +827,7 @@ extern "C" int gbsv_plan_tc(const uint64_t* masks, const uint8_t* diagonal,
     }
     if (!B) B = left[0].m;  // gates on no position, or none found
     std::vector<char> take(left.size(), 0);
-    tc_scan(left, B, all, [&](size_t i, bool p) {
+    tc_scan(left, B, 0, [&](size_t i, bool p) {
       take[i] = 1;
       const int id = left[i].id;
       stage[id] = s;
