@@ -362,29 +362,31 @@ def _initial_state(n, B, dtype, device, psi0):
 def _forward(pc: ParamCircuit, params, dtype, psi0, checkpoints: bool,
              fuse: bool = True):
     """Run the circuit; return (psi_L, [psi at each segment start]), each in
-    memory of its own."""
+    memory of its own but the first, which may be psi0 (a checkpoint that no
+    sweep goes back to, or the result where there is nothing to run)."""
     n, B = pc.num_qubits, params.shape[0]
     dev = params.device
     psi = _initial_state(n, B, dtype, dev, psi0)
     saved = []
     p = _real_params(params)
+    # whether psi's memory is this function's and not the caller's psi0
+    own = psi0 is None or psi.data_ptr() != psi0.data_ptr()
     for a, b in pc.segments():
-        # a segment leaves its checkpoint where it is and writes elsewhere;
-        # a copy is made only of a state that is not this function's or that
-        # no program will replace
-        keep = checkpoints and fuse and b > a and (
-            psi0 is None or bool(saved))
+        # a segment leaves its checkpoint where it is and writes elsewhere
+        keep = checkpoints and fuse and b > a
         if checkpoints:
             saved.append(psi if keep else psi.clone())
         if b <= a:
             continue
+        inplace = own and not keep
+        own = True
         if not fuse:
             prog = pc._segment_circuit(a, b, params, dtype).compile(
                 dtype, dev, fuse=False)
-            prog.run(psi, inplace=True)
+            psi = prog.run(psi, inplace=inplace)
             continue
         prog, which, _ = _forward_program(pc, a, b, B, dtype, dev, fuse)
-        psi = prog._run(psi, not keep, None, _call_pool(prog, which, p))
+        psi = prog._run(psi, inplace, None, _call_pool(prog, which, p))
     return psi, saved
 
 
@@ -904,9 +906,7 @@ def expectation_and_grad(pc: ParamCircuit, params: torch.Tensor,
     lam = _pauli_apply(H, psi_L, torch.empty_like(psi_L))
     values = _real_inner(psi_L, lam)
     if fuse:
-        # psi_L may be the caller's psi0
-        grads = _backward_fused(pc, params, H, psi_L, saved, dtype,
-                                lam if psi0 is None else None)
+        grads = _backward_fused(pc, params, H, psi_L, saved, dtype, lam)
     else:
         grads = _backward_sweep(pc, params, H, psi_L, saved, dtype)
     return values, grads
@@ -919,12 +919,11 @@ class _Expectation(torch.autograd.Function):
         lam = _pauli_apply(H, psi_L, torch.empty_like(psi_L))
         ctx.pc, ctx.H, ctx.dtype = pc, H, dtype
         ctx.psi_L, ctx.saved = psi_L, saved
-        # H psi_L, which starts the backward sweep; kept only where psi_L is
-        # this node's own (it may be the caller's psi0).  The backward pass
-        # then allocates no state: one more is held between the passes, two
-        # fewer during the second, and on 32 states of 16 qubits five copies
-        # (24 us) and an application of H (30 us) are saved.
-        ctx.lam = lam if ctx.needs_input_grad[0] and psi0 is None else None
+        # H psi_L, which starts the backward sweep.  That pass then allocates
+        # no state: one more is held between the passes, two fewer during the
+        # second, and on 32 states of 16 qubits five copies (24 us) and an
+        # application of H (30 us) are saved.
+        ctx.lam = lam if ctx.needs_input_grad[0] else None
         ctx.save_for_backward(params)
         return _real_inner(psi_L, lam)
 
