@@ -292,6 +292,15 @@ ROT_DTYPE = np.dtype([("gen", "<i4"), ("nv", "<i4"), ("pidx", "<i4"),
                       ("pad", "<i4"), ("off", "<i8"), ("half", "<f8")])
 
 
+def _circuit_params(pc, params: torch.Tensor) -> torch.Tensor:
+    """The circuit's parameters, (B, num_params): the kernels index a row by
+    that number, and read past one that is shorter."""
+    if params.dim() != 2 or params.shape[1] < pc.num_params:
+        raise ValueError(f"params must be (B, {pc.num_params}), got "
+                         f"{tuple(params.shape)}")
+    return params[:, :pc.num_params]
+
+
 def _real_params(params: torch.Tensor) -> torch.Tensor:
     """Parameters as the kernels read them: contiguous float32/float64."""
     p = _core.dense(params.detach())
@@ -480,6 +489,7 @@ def evaluate(pc: ParamCircuit, params: torch.Tensor, H: PauliSum,
              dtype=torch.complex64) -> torch.Tensor:
     """Forward only: <psi|H|psi> per batch entry (float64), no gradient."""
     _core.require_cuda(params)
+    params = _circuit_params(pc, params)
     psi_L, _ = _forward(pc, params, dtype, psi0, False)
     return pauli_expectation(H, psi_L)
 
@@ -900,8 +910,10 @@ def expectation_and_grad(pc: ParamCircuit, params: torch.Tensor,
                          dtype=torch.complex64, checkpoints: bool = True,
                          fuse: bool = True):
     """(values (B,), grads (B, num_params)), both float64.  ``fuse=False``
-    runs the forward pass one kernel per gate."""
+    runs the forward pass one kernel per gate.  Parameters beyond the
+    circuit's are not looked at."""
     _core.require_cuda(params)
+    params = _circuit_params(pc, params)
     psi_L, saved = _forward(pc, params, dtype, psi0, checkpoints, fuse)
     lam = _pauli_apply(H, psi_L, torch.empty_like(psi_L))
     values = _real_inner(psi_L, lam)
