@@ -654,6 +654,7 @@ extern "C" int gbsv_adjoint_layouts(const void* ops, int num_ops,
       regops[out++] = r;
     }
     L.count = out - L.first;
+    if (L.count == 0) --*num_layouts;  // its gates came to nothing
   }
   *num_regops = out;
   return GBSV_OK;
