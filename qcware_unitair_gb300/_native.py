@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import importlib.util
 import threading
+import warnings
 
 from . import build_lib
 
@@ -22,15 +23,17 @@ _lock = threading.Lock()
 
 def load():
     """Load the module and bind its functions here; raises if it is not
-    built."""
+    built, or not for this torch and interpreter."""
     with _lock:
-        path = build_lib.host_path()
+        path, tag = build_lib.host_path(), build_lib.host_tag_path()
+        again = ("run `python -c 'import __graft_entry__ as g; g.build()'` or "
+                 "`python -m qcware_unitair_gb300.build_lib`.")
         if not path.exists():
-            raise RuntimeError(
-                f"{path.name} is not built ({path}); run `python -c 'import "
-                "__graft_entry__ as g; g.build()'` or `python -m "
-                "qcware_unitair_gb300.build_lib`.  The engine has no CPU "
-                "fallback.")
+            raise RuntimeError(f"{path.name} is not built ({path}); {again}")
+        built = tag.read_text() if tag.exists() else "an earlier version"
+        if built != build_lib.host_tag():
+            raise RuntimeError(f"{path.name} was built for {built}, this is "
+                               f"{build_lib.host_tag()}; {again}")
         spec = importlib.util.spec_from_file_location(
             build_lib.HOST_MODULE, path)
         mod = importlib.util.module_from_spec(spec)
@@ -40,10 +43,28 @@ def load():
         return mod
 
 
+def _nothing(*args):
+    return None
+
+
+def _load_or_leave():
+    """Load the module; where that fails, leave every call to the Python
+    functions, which launch the same kernels (libgbsv.so does not depend on
+    torch), and say so once."""
+    try:
+        load()
+    except (RuntimeError, ImportError, OSError) as e:
+        warnings.warn(f"the native host path is off, calls take longer on the "
+                      f"host: {e}", RuntimeWarning, stacklevel=4)
+        for name in NAMES:
+            globals()[name] = _nothing
+
+
 def _unloaded(name):
     def call(*args):
         if any(getattr(a, "is_cuda", False) for a in args):
-            return getattr(load(), name)(*args)
+            _load_or_leave()
+            return globals()[name](*args)
         return None
     return call
 

@@ -58,24 +58,40 @@ def _stamp() -> str:
             h.update(p.read_bytes())
     h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS).encode())
     h.update(os.uname().machine.encode())
-    h.update(f"{_torch_version()} {sys.version}".encode())
+    compile_flags, link_flags = _host_flags()
+    h.update(" ".join(compile_flags + link_flags).encode())
+    h.update(f"{host_tag()} {host_headers()}".encode())
     return h.hexdigest()
 
 
-def _torch_version() -> str:
+def host_tag() -> str:
+    """What a built host module goes with: torch's C++ interface and the
+    interpreter's."""
     import torch
-    return torch.__version__
+    return f"torch {torch.__version__}, Python {sys.version}"
 
 
-def _host_flags(nvcc: str) -> tuple[list[str], list[str]]:
+def _torch_root() -> Path:
+    import torch
+    return Path(torch.__file__).resolve().parent
+
+
+def host_headers() -> bool:
+    """Whether the headers that the host module needs are installed (the
+    library of kernels needs neither Python's nor torch's)."""
+    return (Path(sysconfig.get_paths()["include"]) / "Python.h").exists() and (
+        _torch_root() / "include" / "torch" / "csrc" / "autograd" /
+        "custom_function.h").exists()
+
+
+def _host_flags() -> tuple[list[str], list[str]]:
     """(compile flags, link flags) of the host module: torch's headers and
     libraries, the C ABI's library found beside the module."""
     import torch
-    root = Path(torch.__file__).resolve().parent
-    cuda = Path(nvcc).resolve().parent.parent
+    root = _torch_root()
     inc = [root / "include",
            root / "include" / "torch" / "csrc" / "api" / "include",
-           Path(sysconfig.get_paths()["include"]), cuda / "include", INCLUDE]
+           Path(sysconfig.get_paths()["include"]), INCLUDE]
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     compile_flags = ["-O2", "-std=c++17", "-fPIC",
                      f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
@@ -94,21 +110,29 @@ def host_path() -> Path:
     return BUILD_DIR / f"{HOST_MODULE}.so"
 
 
+def host_tag_path() -> Path:
+    return BUILD_DIR / f"{HOST_MODULE}.txt"
+
+
 def build(verbose: bool = False, force: bool = False,
           extra_flags: list[str] | None = None) -> Path:
-    """Compile and link libgbsv.so; return its path."""
+    """Compile and link libgbsv.so and, where its headers are installed, the
+    host module; return the library's path."""
     BUILD_DIR.mkdir(parents=True, exist_ok=True)
     stamp_file = BUILD_DIR / "stamp.txt"
     stamp = _stamp() + (" ".join(extra_flags) if extra_flags else "")
     out = lib_path()
-    if (not force and out.exists() and host_path().exists()
+    with_host = host_headers()
+    if (not force and out.exists() and host_path().exists() == with_host
             and stamp_file.exists() and stamp_file.read_text() == stamp):
         return out
     nvcc = _nvcc()
     flags = ARCH_FLAGS + NVCC_FLAGS + (extra_flags or []) + [
         f"-I{INCLUDE}", f"-I{CSRC}"]
     objs = []
-    host_compile, host_link = _host_flags(nvcc)
+    host_compile, host_link = _host_flags()
+    host_compile.append(
+        f"-isystem{Path(nvcc).resolve().parent.parent / 'include'}")
 
     def compile_one(src: Path) -> Path:
         obj = BUILD_DIR / (src.stem + ".o")
@@ -128,7 +152,7 @@ def build(verbose: bool = False, force: bool = False,
             print(res.stderr, file=sys.stderr)
         return obj
 
-    srcs = sources() + [HOST_SOURCE]
+    srcs = sources() + ([HOST_SOURCE] if with_host else [])
     with cf.ThreadPoolExecutor(max_workers=min(len(srcs), os.cpu_count() or 4)) as ex:
         objs = list(ex.map(compile_one, srcs))
     tmp = out.with_suffix(".so.tmp")
@@ -138,13 +162,19 @@ def build(verbose: bool = False, force: bool = False,
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stderr}")
 
-    *lib_objs, host_obj = objs
+    lib_objs = objs[:len(sources())]
     link([nvcc, *ARCH_FLAGS, "-shared", "-o", str(tmp),
           f"-Xlinker=-soname={LIB_NAME}", *map(str, lib_objs), "-lcudart"])
     os.replace(tmp, out)
-    tmp = host_path().with_suffix(".so.tmp")
-    link([_cxx(), "-shared", "-o", str(tmp), str(host_obj), *host_link])
-    os.replace(tmp, host_path())
+    if with_host:
+        tmp = host_path().with_suffix(".so.tmp")
+        link([_cxx(), "-shared", "-o", str(tmp), str(objs[-1]), *host_link])
+        os.replace(tmp, host_path())
+        host_tag_path().write_text(host_tag())
+    else:
+        host_path().unlink(missing_ok=True)
+        print(f"{HOST_MODULE} not built: Python.h or torch's headers are "
+              "missing; calls take the Python route", file=sys.stderr)
     stamp_file.write_text(stamp)
     return out
 
