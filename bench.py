@@ -363,7 +363,7 @@ def bench_c2(dev, layers=100):
     import torch
     import qcware_unitair_gb300 as ug
     from qcware_unitair_gb300.adjoint import (ParamCircuit, _forward_program,
-                                              _rotation_values)
+                                              _write_rotations)
     from qcware_unitair_gb300.circuits import random_states
     n, B = 16, 4096
     pc = ParamCircuit(n, 3 * n)
@@ -380,16 +380,11 @@ def bench_c2(dev, layers=100):
     psi0 = random_states(n, (B,), torch.complex64, seed=2).to(dev)
     prog, which, _ = _forward_program(pc, 0, len(pc.ops), B,
                                       torch.complex64, dev, True)
-    idx = torch.cat([torch.arange(off, off + B * nv, device=dev)
-                     for _, _, _, off, nv in which])
-    vals = torch.stack([_rotation_values(which, angles[l], B,
-                                         torch.complex64)
-                        for l in range(layers)])
     psi = psi0.clone()
 
     def circuit():
         for l in range(layers):
-            prog.pool.index_copy_(0, idx, vals[l])
+            _write_rotations(prog, which, angles[l])
             prog.run(psi, inplace=True)
 
     circuit()  # warm-up outside capture

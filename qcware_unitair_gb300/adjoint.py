@@ -255,20 +255,16 @@ def _forward_program(pc: ParamCircuit, a: int, b: int, B: int, dtype, dev,
 
 def _rotation_values(which, params, B, dtype):
     """All rotations' pool entries, flattened in ``which`` order (rotation,
-    state, entry), from a handful of vectorised tensor ops."""
+    state, entry), from torch operations: what _write_rotations is tested
+    against."""
     dev = params.device
-    cached = _rotation_values._meta.get(id(which))
-    if cached is None or cached[0] is not which:
-        gen = torch.tensor(["XYZ".index(w[0]) for w in which], device=dev)
-        pidx = torch.tensor([w[1] for w in which], device=dev)
-        half = torch.tensor([0.5 * w[2] for w in which], dtype=torch.float64,
-                            device=dev)
-        nv = torch.tensor([w[4] for w in which], device=dev)
-        keep = (torch.arange(4, device=dev)[None, None, :] <
-                nv[:, None, None]).expand(len(which), B, 4)
-        cached = (which, gen, pidx, half, nv, keep)
-        _rotation_values._meta[id(which)] = cached
-    _, gen, pidx, half, nv, keep = cached
+    gen = torch.tensor(["XYZ".index(w[0]) for w in which], device=dev)
+    pidx = torch.tensor([w[1] for w in which], device=dev)
+    half = torch.tensor([0.5 * w[2] for w in which], dtype=torch.float64,
+                        device=dev)
+    nv = torch.tensor([w[4] for w in which], device=dev)
+    keep = (torch.arange(4, device=dev)[None, None, :] <
+            nv[:, None, None]).expand(len(which), B, 4)
     th = params[:, pidx].to(torch.float64) * half          # (B, R)
     c, s = torch.cos(th).T, torch.sin(th).T                 # (R, B)
     z = torch.zeros_like(c)
@@ -283,9 +279,6 @@ def _rotation_values(which, params, B, dtype):
     re = torch.stack([re0, re1, re2, re3], -1)
     im = torch.stack([im0, im1, im2, im3], -1)
     return torch.complex(re, im).to(dtype)[keep]
-
-
-_rotation_values._meta = {}
 
 
 ROT_DTYPE = np.dtype([("gen", "<i4"), ("nv", "<i4"), ("pidx", "<i4"),
