@@ -12,12 +12,14 @@ of a rotation is ``scale * params[b, p]`` per batch entry b.
 
 The forward pass runs the circuit as a fused program (one HBM pass per
 stage) and keeps the state at checkpoints every ~sqrt(depth) layers.  The
-backward pass starts from lambda = H psi_L (gbsv_pauli_sum_apply) and walks
-the gates in reverse with gbsv_adjoint_rotation_step (gradient Im<l|P|psi>
-accumulated in FP64, then U^dag applied to psi and lambda in the same pass);
-fixed gates are uncomputed on both states in one launch.  At each
-checkpoint the uncomputed psi is replaced by the stored forward state, so
-rounding drift never accumulates over more than one segment.
+backward pass starts from lambda = H psi_L (gbsv_pauli_sum_apply_host) and
+walks the gates in reverse, in stages as the forward pass has them
+(gbsv_adjoint_stage_regs, or gbsv_adjoint_stage where a stage has no register
+plan): for each rotation the gradient Im<l|P|psi>, summed in FP64 beyond a
+thread, then U^dag on psi and lambda.  A rotation or gate outside the stages
+is a launch of its own on both states.  At each checkpoint the uncomputed psi
+is replaced by the stored forward state, so rounding drift never accumulates
+over more than one segment.
 This replaces torch autograd through unitair's apply_operator, which keeps
 every intermediate state (one per gate) alive for the backward pass.
 """
