@@ -42,7 +42,8 @@ def test_time_grows_with_the_list(lib_built):
     seconds(lib_built, 26, 100, True)
     short = min(seconds(lib_built, 26, 1500, True) for _ in range(3))
     # eight times the gates: 64 times the work where it is quadratic
-    assert seconds(lib_built, 26, 12000, True) < 30 * short + 0.1
+    long = min(seconds(lib_built, 26, 12000, True) for _ in range(2))
+    assert long < 30 * short + 0.1
 
 
 def test_long_circuit_with_a_diagonal_qubit(lib_built):
