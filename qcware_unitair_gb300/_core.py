@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib
+from . import _lib, _native
 
 _COMPLEX = {torch.complex64: _lib.C64, torch.complex128: _lib.C128}
 _REAL = {torch.float32: _lib.F32, torch.float64: _lib.F64}
@@ -52,6 +52,9 @@ def dense(t: torch.Tensor) -> torch.Tensor:
     """``t`` as the kernels read it: contiguous memory that holds its values.
     conj(), and what autograd hands to a backward, may be lazy: a bit on the
     tensor over unchanged memory, which contiguous() keeps."""
+    out = _native.dense(t)  # a device tensor that is so already
+    if out is not None:
+        return out
     return t.resolve_conj().resolve_neg().contiguous()
 
 

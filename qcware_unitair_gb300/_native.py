@@ -16,7 +16,7 @@ from . import build_lib
 
 NAMES = ("apply_operator", "apply_layer", "apply_phase", "norm_squared",
          "abs_squared", "inner_product", "diag_expectation_value",
-         "rotation")
+         "rotation", "dense")
 
 _lock = threading.Lock()
 

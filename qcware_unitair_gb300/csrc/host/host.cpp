@@ -63,9 +63,8 @@ bool plain_context() {
          !torch::jit::tracer::isTracing();
 }
 
-// An ordinary strided CUDA tensor (not conjugated or negated lazily, no
-// forward-mode tangent).
-bool plain(const Tensor& t) {
+// An ordinary strided CUDA tensor (not conjugated or negated lazily).
+bool ordinary(const Tensor& t) {
   static const c10::DispatchKeySet allowed =
       c10::DispatchKeySet({c10::DispatchKey::CUDA,
                            c10::DispatchKey::ADInplaceOrView,
@@ -73,8 +72,11 @@ bool plain(const Tensor& t) {
                            c10::DispatchKey::AutocastCUDA});
   return t.defined() && t.is_cuda() &&
          (t.unsafeGetTensorImpl()->key_set().raw_repr() &
-          ~allowed.raw_repr()) == 0 &&
-         !t._fw_grad(/*level=*/0).defined();
+          ~allowed.raw_repr()) == 0;
+}
+// The same without a forward-mode tangent.
+bool plain(const Tensor& t) {
+  return ordinary(t) && !t._fw_grad(/*level=*/0).defined();
 }
 
 // The tensor of a Python argument, if it is exactly a Tensor or Parameter.
@@ -867,7 +869,21 @@ PyObject* py_rotation(PyObject*, PyObject* const* args, Py_ssize_t na) {
   GBSV_END_CALL
 }
 
+// (tensor): the tensor itself where its memory holds its values in order.
+PyObject* py_dense(PyObject*, PyObject* const* args, Py_ssize_t na) {
+  GBSV_CALL
+  if (na != 1 || !THPVariable_CheckExact(args[0])) return none();
+  const Tensor& t = THPVariable_Unpack(args[0]);
+  if (!ordinary(t) || !t.is_contiguous()) return none();
+  Py_INCREF(args[0]);
+  return args[0];
+  GBSV_END_CALL
+}
+
 PyMethodDef kMethods[] = {
+    {"dense",
+     reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_dense)),
+     METH_FASTCALL, "(tensor) -> the same Tensor or None"},
     {"rotation",
      reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_rotation)),
      METH_FASTCALL, "(axis, angles) -> Tensor or None"},

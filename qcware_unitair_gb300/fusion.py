@@ -783,7 +783,8 @@ class Program:
             return out
         L = _lib.load()
         stream = _core.stream_of(state.device)
-        self._uploads.use(state.device, stream)
+        if stream not in self._uploads.streams:
+            self._uploads.use(state.device, stream)
         N = 2 ** self.n
         cur = src
         if not self.ops and cur is not out:
