@@ -55,7 +55,6 @@ struct AqOp {
   int kind;
 };
 constexpr int AQ_FULL = 0, AQ_REAL = 1, AQ_RX = 2, AQ_DIAG = 3;
-constexpr int AQ_LARGE = 4;  // full, with entries beyond 2^7 or not finite
 
 // The operator of amplitude-index bit pos.
 __device__ __forceinline__ AqOp aq_load_op(const float2* ops,
@@ -70,31 +69,23 @@ __device__ __forceinline__ AqOp aq_load_op(const float2* ops,
   else if (r.m[1].x == 0 && r.m[1].y == 0 && r.m[2].x == 0 && r.m[2].y == 0)
     r.kind = AQ_DIAG;
   else r.kind = AQ_FULL;
-  float e = 0.f;  // largest |component|; NaN stays
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    asm("max.NaN.abs.f32 %0, %0, %1, %2;"
-        : "+f"(e) : "f"(r.m[j].x), "f"(r.m[j].y));
-  if (!(e <= 128.f)) r.kind = AQ_LARGE;
   return r;
 }
 
-// Whether every amplitude stays finite through a layout.  Where one is not,
+// Whether all 16 amplitudes stay finite through a layout.  Where one is not,
 // or a sum overflows, the products with zeros that the structured forms leave
-// out are NaN in a loop of gates, so the full form runs from there on.  An
-// operator with entries up to 2^7 makes at most 4 * 2^7 of the largest
-// component, four of them 2^36: below 2^91 nothing reaches 2^128.
+// out are NaN in a loop of gates, so the full form runs.  Four operators with
+// entries up to 2^26 make at most (4 * 2^26)^4 = 2^112 of the largest
+// component, so below 2^16 nothing reaches 2^128.  (A look at the entries, or
+// one before each operator, costs registers this kernel does not have: layers
+// of full matrices 81 -> 85 us on 7 states of 20 qubits, 11.3 -> 12.6 us on
+// 1000 of 10.)
 __device__ __forceinline__ bool aq_bounded(const float2* r) {
   float e = 0.f;  // largest |component|; NaN stays
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(e) : "f"(r[i].x), "f"(r[i].y));
-  return e < 0x1p91f;
-}
-// The form of the next operator; clears `bounded` after a large one.
-__device__ __forceinline__ int aq_form(const AqOp& o, bool& bounded) {
-  bounded = bounded && o.kind != AQ_LARGE;
-  return bounded ? o.kind : AQ_FULL;
+  return e < 0x1p16f;
 }
 
 // m * a, rounded as the gate kernels' products are.
@@ -159,12 +150,12 @@ template <int RB, int LO, int HI>
 __device__ __forceinline__ void aq_round(float2* r, const float2* ops,
                                          const AllqArgs& a) {
   AqOp o = aq_load_op(ops, a, aq_pos(a, HI));
-  bool bounded = aq_bounded(r);
+  const bool bounded = aq_bounded(r);
 #pragma unroll
   for (int b = HI; b >= LO; --b) {
     if (!((a.mask >> b) & 1)) continue;
     if (a.op_qstride) o = aq_load_op(ops, a, aq_pos(a, b));
-    const int kind = aq_form(o, bounded);
+    const int kind = bounded ? o.kind : AQ_FULL;
     if (b - RB == 0) aq_apply<0>(r, o, kind);
     else if (b - RB == 1) aq_apply<1>(r, o, kind);
     else if (b - RB == 2) aq_apply<2>(r, o, kind);
@@ -285,12 +276,12 @@ __global__ void __launch_bounds__(AQ_THREADS, 4)
     const int bits = w.bits[k];
     AqOp o;
     if (!staged) o = aq_load_op(ops, a, w.pos[k]);
-    bool bounded = aq_bounded(r);
+    const bool bounded = aq_bounded(r);
 #define AQ_BIT(J)                                                      \
   if ((bits >> J) & 1) {                                               \
     if (staged) o = sop[w.rb[k] + J];                                  \
     else if (a.op_qstride) o = aq_load_op(ops, a, w.pos[k] + J);       \
-    aq_apply<J>(r, o, aq_form(o, bounded));                            \
+    aq_apply<J>(r, o, bounded ? o.kind : AQ_FULL);                      \
   }
     AQ_BIT(3)
     AQ_BIT(2)
@@ -533,19 +524,18 @@ __device__ __forceinline__ void aq_grad_round(float2* g, const float2* S,
     float2 x[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) x[i] = S[aq_swz(aq_index<RB>(u, i))];
-    bool bounded = aq_bounded(x);
+    const bool bounded = aq_bounded(x);
 #pragma unroll
     for (int c = LO; c < HI; ++c) {
       if (c >= b || !((a.mask >> c) & 1)) continue;
       const AqOp o = aq_load_op(ops, a, aq_pos(a, c));
-      const int kind = aq_form(o, bounded);
+      const int kind = bounded ? o.kind : AQ_FULL;
       if (c - RB == 0) aq_apply<0>(x, o, kind);
       else if (c - RB == 1) aq_apply<1>(x, o, kind);
       else aq_apply<2>(x, o, kind);
     }
     const AqOp d = aq_dagger(aq_load_op(ops, a, aq_pos(a, b)));
-    bool gbounded = aq_bounded(g);
-    const int kind = aq_form(d, gbounded);
+    const int kind = aq_bounded(g) ? d.kind : AQ_FULL;
     Acc<float> acc[8];
     switch (b - RB) {
       case 0: aq_outer<0>(g, x, acc); aq_apply<0>(g, d, kind); break;
