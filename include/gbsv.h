@@ -359,6 +359,16 @@ int gbsv_run_stage_tc(const void* state_in, void* state_out, int dtype,
                       int num_blocks, const void* diags, const void* images,
                       const void* factors, void* stream);
 
+/* The same for a stage with blocks of flags bit 1 (column scales), which
+ * gbsv_run_stage_tc does not look at.  In it a column of the tile whose
+ * amplitudes are all below 2^-107 keeps their precision as well. */
+int gbsv_run_stage_tc_scaled(const void* state_in, void* state_out, int dtype,
+                      int num_qubits, int64_t num_states, int64_t in_stride,
+                      int tile_qubits, int contiguous_qubits,
+                      const int32_t* tile_positions, const void* blocks,
+                      int num_blocks, const void* diags, const void* images,
+                      const void* factors, void* stream);
+
 /* Nonzero bits record a bounded wait inside a tensor-core stage that ran out
  * (1: block image, 2: MMA completion, 4 / 8: draining); clear != 0 resets
  * it.  Synchronizes the device.  No counterpart in the reference. */

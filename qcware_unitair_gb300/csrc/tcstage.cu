@@ -60,7 +60,6 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <type_traits>
 
 namespace gbsv {
 
@@ -288,9 +287,10 @@ __device__ __forceinline__ void tc_scatter(float2* S, int sb, const int* rs,
 // Blocks that are not unitary: the image's entries were scaled by column into
 // its range (rows' L1 norm at most 8, largest entry near 1; without, entries
 // beyond 64 are infinite in fp16 and small ones have 11 bits), and the powers
-// of two go to the amplitudes, exactly.  The kernels have a copy of their
-// compute loop for stages with such a block: the branches alone cost 5% of the
-// others' time (26 qubits 1647 -> 1732 us).
+// of two go to the amplitudes, exactly.  Stages with such a block have
+// kernels of their own (SCALED): in one kernel the branches cost the others 5%
+// of their time (26 qubits 1647 -> 1732 us), and a second copy of the compute
+// loop 2% of a short program's (16 qubits x 10: 35.4 -> 36.1 us).
 __device__ __forceinline__ void tc_columns(const TcArgs& a, const TcBlock& B,
                                            float2* v) {
   if (!(B.flags & TC_COLS)) return;
@@ -301,12 +301,6 @@ __device__ __forceinline__ void tc_columns(const TcArgs& a, const TcBlock& B,
     v[i] = make_float2(v[i].x * w.x, v[i].y * w.x);
     v[i + 1] = make_float2(v[i + 1].x * w.y, v[i + 1].y * w.y);
   }
-}
-
-__device__ __forceinline__ bool tc_any_scaled(const TcBlock* b, int nb) {
-  int flags = 0;
-  for (int i = 0; i < nb; ++i) flags |= b[i].flags;
-  return flags & TC_COLS;
 }
 
 // Power-of-two scaling (largest |x| of the column, tree reduction): x * sc
@@ -442,6 +436,7 @@ __device__ __forceinline__ bool tc_compute_sync_or(bool x) {
   return r != 0;
 }
 
+template <bool SCALED>
 __global__ void __launch_bounds__(TC_ROLE_THREADS, 2)
     tc_stage_kernel(const float2* in, float2* out, TcArgs a) {
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
@@ -649,102 +644,97 @@ __global__ void __launch_bounds__(TC_ROLE_THREADS, 2)
     }
   } else {
     // ---------------------------------------------------------- compute
-    auto compute = [&](auto scaled) {
-      constexpr bool SCALED = decltype(scaled)::value;
-      const uint32_t lane = (uint32_t)(warp * 32) << 16;
-      const uint32_t tA = tmem, tD1 = tmem + 64, tDc = tmem + 128;
-      uint64_t s = t0 / tps, base = tc_tile_base(a, t0 % tps);
-      // A wait that runs out only sets `bad`: every compute thread runs the
-      // same tcgen05 and barrier sequence, and all leave together after the
-      // reduction barrier that ends each block.
-      uint64_t e = 0;
-      bool bad = false;
-      bool late = false;  // an MMA completion wait ran out
-      for (uint64_t k = 0; k < ntile && !bad; ++k) {
-        const int b = (int)(k & 1);
-        float2* const S = tiles + b * TC_TILE;
-        if (!tc_wait(tc_smem(&bar_full[b]), (uint32_t)((k >> 1) & 1))) {
-          fail(64);
+    const uint32_t lane = (uint32_t)(warp * 32) << 16;
+    const uint32_t tA = tmem, tD1 = tmem + 64, tDc = tmem + 128;
+    uint64_t s = t0 / tps, base = tc_tile_base(a, t0 % tps);
+    // A wait that runs out only sets `bad`: every compute thread runs the
+    // same tcgen05 and barrier sequence, and all leave together after the
+    // reduction barrier that ends each block.
+    uint64_t e = 0;
+    bool bad = false;
+    bool late = false;  // an MMA completion wait ran out
+    for (uint64_t k = 0; k < ntile && !bad; ++k) {
+      const int b = (int)(k & 1);
+      float2* const S = tiles + b * TC_TILE;
+      if (!tc_wait(tc_smem(&bar_full[b]), (uint32_t)((k >> 1) & 1))) {
+        fail(64);
+        bad = true;
+      }
+      for (int bi = 0; bi < nb; ++bi, ++e) {
+        const TcBlock& B = sblk[bi];
+        int sb = 0;
+#pragma unroll
+        for (int j = 0; j < TC_TB; ++j)
+          if ((tid >> j) & 1) sb ^= B.tspo[j];
+        int rs[TC_RB];
+#pragma unroll
+        for (int j = 0; j < TC_RB; ++j) rs[j] = B.rspo[j];
+        const bool pairs = B.flags & TC_PAIRS;
+        // loaded now and used after the MMAs
+        const float2 fv = tc_factor(a, B, base, tid);
+        float2 v[32];
+        tc_gather(S, sb, rs, pairs, v);
+        if constexpr (SCALED) tc_columns(a, B, v);
+        float sc, inv;
+        tc_scale<SCALED>(v, &sc, &inv);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t hi[16], lo[16];
+          tc_split<16>(&v[16 * h], sc, hi, lo);
+          tc_st16(tA + lane + 16 * h, hi);
+          tc_st16(tA + 32 + lane + 16 * h, lo);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
+                         tc_smem(&bar_a))
+                     : "memory");
+        // post-diagonals left in the list (a register bit, or too many
+        // outside bits), while the MMAs run
+        float2 f = make_float2(fv.x * inv, fv.y * inv);
+        const bool has_diag = B.num_diag > 0 || B.fac >= 0;
+        const bool regdiag = tc_outer_diags(B, dtab, base, tid, &f);
+        if (!tc_wait(tc_smem(&bar_mma), (uint32_t)(e & 1))) {
+          fail(2);
+          late = true;
           bad = true;
         }
-        for (int bi = 0; bi < nb; ++bi, ++e) {
-          const TcBlock& B = sblk[bi];
-          int sb = 0;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // read back D1 + Dc, undo the scaling, apply the factors
 #pragma unroll
-          for (int j = 0; j < TC_TB; ++j)
-            if ((tid >> j) & 1) sb ^= B.tspo[j];
-          int rs[TC_RB];
+        for (int h = 0; h < 2; ++h) {
+          uint32_t d1[32], dc[32];
+          tc_ld32(tD1 + lane + 32 * h, d1);
+          tc_ld32(tDc + lane + 32 * h, dc);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int j = 0; j < TC_RB; ++j) rs[j] = B.rspo[j];
-          const bool pairs = B.flags & TC_PAIRS;
-          // loaded now and used after the MMAs
-          const float2 fv = tc_factor(a, B, base, tid);
-          float2 v[32];
-          tc_gather(S, sb, rs, pairs, v);
-          if constexpr (SCALED) tc_columns(a, B, v);
-          float sc, inv;
-          tc_scale<SCALED>(v, &sc, &inv);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t hi[16], lo[16];
-            tc_split<16>(&v[16 * h], sc, hi, lo);
-            tc_st16(tA + lane + 16 * h, hi);
-            tc_st16(tA + 32 + lane + 16 * h, lo);
+          for (int j = 0; j < 16; ++j) {
+            const float re =
+                __uint_as_float(d1[2 * j]) + __uint_as_float(dc[2 * j]);
+            const float im = __uint_as_float(d1[2 * j + 1]) +
+                             __uint_as_float(dc[2 * j + 1]);
+            v[16 * h + j] = has_diag ? cmul(f, make_float2(re, im))
+                                     : make_float2(re * inv, im * inv);
           }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
-                           tc_smem(&bar_a))
-                       : "memory");
-          // post-diagonals left in the list (a register bit, or too many
-          // outside bits), while the MMAs run
-          float2 f = make_float2(fv.x * inv, fv.y * inv);
-          const bool has_diag = B.num_diag > 0 || B.fac >= 0;
-          const bool regdiag = tc_outer_diags(B, dtab, base, tid, &f);
-          if (!tc_wait(tc_smem(&bar_mma), (uint32_t)(e & 1))) {
-            fail(2);
-            late = true;
-            bad = true;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          // read back D1 + Dc, undo the scaling, apply the factors
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t d1[32], dc[32];
-            tc_ld32(tD1 + lane + 32 * h, d1);
-            tc_ld32(tDc + lane + 32 * h, dc);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float re =
-                  __uint_as_float(d1[2 * j]) + __uint_as_float(dc[2 * j]);
-              const float im = __uint_as_float(d1[2 * j + 1]) +
-                               __uint_as_float(dc[2 * j + 1]);
-              v[16 * h + j] = has_diag ? cmul(f, make_float2(re, im))
-                                       : make_float2(re * inv, im * inv);
-            }
-          }
-          if constexpr (SCALED) tc_unscale(v, inv);
-          if (regdiag) tc_register_diags(B, dtab, base, tid, v);
-          // scatter back (the same addresses the gather read)
-          tc_scatter(S, sb, rs, pairs, v);
-          // the next block reads other threads' results; errors anywhere
-          // stop every compute thread here
-          bad = tc_compute_sync_or(bad || s_abort);
-          if (bad) break;
         }
+        if constexpr (SCALED) tc_unscale(v, inv);
+        if (regdiag) tc_register_diags(B, dtab, base, tid, v);
+        // scatter back (the same addresses the gather read)
+        tc_scatter(S, sb, rs, pairs, v);
+        // the next block reads other threads' results; errors anywhere
+        // stop every compute thread here
+        bad = tc_compute_sync_or(bad || s_abort);
         if (bad) break;
-        // this thread's part of the tile is final: the storer may take it
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
-                         tc_smem(&bar_empty[b]))
-                     : "memory");
-        base = next_base(base);
-        s += base == 0;
       }
-      if (late && !tc_wait(tc_smem(&bar_mma), (uint32_t)((e & 1)))) fail(8);
-    };
-    if (tc_any_scaled(sblk, nb)) compute(std::true_type{});
-    else compute(std::false_type{});
+      if (bad) break;
+      // this thread's part of the tile is final: the storer may take it
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
+                       tc_smem(&bar_empty[b]))
+                   : "memory");
+      base = next_base(base);
+      s += base == 0;
+    }
+    if (late && !tc_wait(tc_smem(&bar_mma), (uint32_t)((e & 1)))) fail(8);
   }
   // every role is done (waits are bounded): free tensor memory
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -823,6 +813,7 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
       : "memory");
 }
 
+template <bool SCALED>
 __global__ void __launch_bounds__(TW_THREADS, 1)
     tc_wide_kernel(const float2* in, float2* out,
                    const __grid_constant__ TcArgs a) {
@@ -961,142 +952,137 @@ __global__ void __launch_bounds__(TW_THREADS, 1)
   } else {
     // ---------------------------------------------------------- compute
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TW_CALC_REGS));
-    auto compute = [&](auto scaled) {
-      constexpr bool SCALED = decltype(scaled)::value;
-      const int g = warp >> 2;
-      const int tid = threadIdx.x & (TC_THREADS - 1);
-      const uint32_t tmem = s_tmem + 128 * g;
-      const uint32_t lane = (uint32_t)((warp & 3) * 32) << 16;
-      const uint32_t tA = tmem + lane, tD = tmem + 64 + lane;
-      const uint32_t bar = tc_smem(&bar_mma[g]);
-      uint32_t par = 0;  // parity of the group's next MMA wait
-      uint64_t base = tc_tile_base(a, t0 % tps);
-      for (int j = 0; j < g; ++j) base = next_base(base);
-      bool bad = false, late = false, image = false;
-      int b = g % nbuf;
-      uint32_t ph = g >= nbuf;
-      // As in tc_stage_kernel a wait that runs out only sets `bad`, and the
-      // group leaves together after the barrier that ends each block.
-      for (uint64_t k = g; k < ntile && !bad; k += TW_GROUPS) {
-        float2* const S = tiles + b * TC_TILE;
-        if (!tc_wait(tc_smem(&bar_full[b]), ph)) {
-          fail(64);
-          bad = true;
-        }
-        for (int bi = 0; bi < nb; ++bi) {
-          const TcBlock& B = sblk[bi];
-          int sb = 0;
-#pragma unroll
-          for (int j = 0; j < TC_TB; ++j)
-            if ((tid >> j) & 1) sb ^= B.tspo[j];
-          int rs[TC_RB];
-#pragma unroll
-          for (int j = 0; j < TC_RB; ++j) rs[j] = B.rspo[j];
-          const bool pairs = B.flags & TC_PAIRS;
-          const float2 fv = tc_factor(a, B, base, tid);
-          float2 v[32];
-          tc_gather(S, sb, rs, pairs, v);
-          if constexpr (SCALED) tc_columns(a, B, v);
-          float sc, inv;
-          tc_scale<SCALED>(v, &sc, &inv);
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            uint32_t hi[8], lo[8];
-            tc_split<8>(&v[8 * h], sc, hi, lo);
-            tc_st8(tA + 8 * h, hi);
-            tc_st8(tA + 32 + 8 * h, lo);
-          }
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          tw_sync(1 + g);
-          // D1 = hi * Bh; each group's issuer sits on its own scheduler
-          const uint32_t im = tc_smem(imgs + bi * TC_IMG_BYTES);
-          if (tid == 32 * g) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (!image && !tc_wait(tc_smem(&bar_img), 0)) fail(1);
-            image = true;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              tc_mma<64>(tmem + 64, tmem + 8 * j, tc_desc(im + 1024 + 256 * j),
-                         j > 0);
-            tc_commit(bar);
-          }
-          __syncwarp();
-          float2 f = make_float2(fv.x * inv, fv.y * inv);
-          const bool has_diag = B.num_diag > 0 || B.fac >= 0;
-          const bool regdiag = tc_outer_diags(B, dtab, base, tid, &f);
-          auto finished = [&]() {
-            if (!tc_wait(bar, par)) {
-              fail(2);
-              late = true;
-              bad = true;
-            }
-            par ^= 1;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          };
-          finished();
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t d[32];
-            tc_ld32(tD + 32 * h, d);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              v[16 * h + j] = make_float2(__uint_as_float(d[2 * j]),
-                                          __uint_as_float(d[2 * j + 1]));
-          }
-          // the correction, in D1's columns
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          tw_sync(1 + g);
-          if (tid == 32 * g) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              tc_mma<64>(tmem + 64, tmem + 8 * j, tc_desc(im + 256 * j), j > 0);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              tc_mma<64>(tmem + 64, tmem + 32 + 8 * j, tc_desc(im + 256 * j),
-                         1);
-            tc_commit(bar);
-          }
-          __syncwarp();
-          finished();
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint32_t d[32];
-            tc_ld32(tD + 32 * h, d);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float re = v[16 * h + j].x + __uint_as_float(d[2 * j]);
-              const float im = v[16 * h + j].y + __uint_as_float(d[2 * j + 1]);
-              v[16 * h + j] = has_diag ? cmul(f, make_float2(re, im))
-                                      : make_float2(re * inv, im * inv);
-            }
-          }
-          if constexpr (SCALED) tc_unscale(v, inv);
-          if (regdiag) tc_register_diags(B, dtab, base, tid, v);
-          tc_scatter(S, sb, rs, pairs, v);
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          bad = tw_sync_or(1 + g, bad || s_abort);
-          if (bad) break;
-        }
-        if (bad) break;
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
-                         tc_smem(&bar_empty[b]))
-                     : "memory");
-#pragma unroll
-        for (int j = 0; j < TW_GROUPS; ++j) base = next_base(base);
-        b += TW_GROUPS;
-        if (b >= nbuf) {
-          b -= nbuf;
-          ph ^= 1;
-        }
+    const int g = warp >> 2;
+    const int tid = threadIdx.x & (TC_THREADS - 1);
+    const uint32_t tmem = s_tmem + 128 * g;
+    const uint32_t lane = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tA = tmem + lane, tD = tmem + 64 + lane;
+    const uint32_t bar = tc_smem(&bar_mma[g]);
+    uint32_t par = 0;  // parity of the group's next MMA wait
+    uint64_t base = tc_tile_base(a, t0 % tps);
+    for (int j = 0; j < g; ++j) base = next_base(base);
+    bool bad = false, late = false, image = false;
+    int b = g % nbuf;
+    uint32_t ph = g >= nbuf;
+    // As in tc_stage_kernel a wait that runs out only sets `bad`, and the
+    // group leaves together after the barrier that ends each block.
+    for (uint64_t k = g; k < ntile && !bad; k += TW_GROUPS) {
+      float2* const S = tiles + b * TC_TILE;
+      if (!tc_wait(tc_smem(&bar_full[b]), ph)) {
+        fail(64);
+        bad = true;
       }
-      if (late && !tc_wait(bar, par ^ 1)) fail(8);
-    };
-    if (tc_any_scaled(sblk, nb)) compute(std::true_type{});
-    else compute(std::false_type{});
+      for (int bi = 0; bi < nb; ++bi) {
+        const TcBlock& B = sblk[bi];
+        int sb = 0;
+#pragma unroll
+        for (int j = 0; j < TC_TB; ++j)
+          if ((tid >> j) & 1) sb ^= B.tspo[j];
+        int rs[TC_RB];
+#pragma unroll
+        for (int j = 0; j < TC_RB; ++j) rs[j] = B.rspo[j];
+        const bool pairs = B.flags & TC_PAIRS;
+        const float2 fv = tc_factor(a, B, base, tid);
+        float2 v[32];
+        tc_gather(S, sb, rs, pairs, v);
+        if constexpr (SCALED) tc_columns(a, B, v);
+        float sc, inv;
+        tc_scale<SCALED>(v, &sc, &inv);
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          uint32_t hi[8], lo[8];
+          tc_split<8>(&v[8 * h], sc, hi, lo);
+          tc_st8(tA + 8 * h, hi);
+          tc_st8(tA + 32 + 8 * h, lo);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        tw_sync(1 + g);
+        // D1 = hi * Bh; each group's issuer sits on its own scheduler
+        const uint32_t im = tc_smem(imgs + bi * TC_IMG_BYTES);
+        if (tid == 32 * g) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (!image && !tc_wait(tc_smem(&bar_img), 0)) fail(1);
+          image = true;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            tc_mma<64>(tmem + 64, tmem + 8 * j, tc_desc(im + 1024 + 256 * j),
+                       j > 0);
+          tc_commit(bar);
+        }
+        __syncwarp();
+        float2 f = make_float2(fv.x * inv, fv.y * inv);
+        const bool has_diag = B.num_diag > 0 || B.fac >= 0;
+        const bool regdiag = tc_outer_diags(B, dtab, base, tid, &f);
+        auto finished = [&]() {
+          if (!tc_wait(bar, par)) {
+            fail(2);
+            late = true;
+            bad = true;
+          }
+          par ^= 1;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        };
+        finished();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t d[32];
+          tc_ld32(tD + 32 * h, d);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            v[16 * h + j] = make_float2(__uint_as_float(d[2 * j]),
+                                        __uint_as_float(d[2 * j + 1]));
+        }
+        // the correction, in D1's columns
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        tw_sync(1 + g);
+        if (tid == 32 * g) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            tc_mma<64>(tmem + 64, tmem + 8 * j, tc_desc(im + 256 * j), j > 0);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            tc_mma<64>(tmem + 64, tmem + 32 + 8 * j, tc_desc(im + 256 * j),
+                       1);
+          tc_commit(bar);
+        }
+        __syncwarp();
+        finished();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t d[32];
+          tc_ld32(tD + 32 * h, d);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float re = v[16 * h + j].x + __uint_as_float(d[2 * j]);
+            const float im = v[16 * h + j].y + __uint_as_float(d[2 * j + 1]);
+            v[16 * h + j] = has_diag ? cmul(f, make_float2(re, im))
+                                    : make_float2(re * inv, im * inv);
+          }
+        }
+        if constexpr (SCALED) tc_unscale(v, inv);
+        if (regdiag) tc_register_diags(B, dtab, base, tid, v);
+        tc_scatter(S, sb, rs, pairs, v);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        bad = tw_sync_or(1 + g, bad || s_abort);
+        if (bad) break;
+      }
+      if (bad) break;
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(
+                       tc_smem(&bar_empty[b]))
+                   : "memory");
+#pragma unroll
+      for (int j = 0; j < TW_GROUPS; ++j) base = next_base(base);
+      b += TW_GROUPS;
+      if (b >= nbuf) {
+        b -= nbuf;
+        ph ^= 1;
+      }
+    }
+    if (late && !tc_wait(bar, par ^ 1)) fail(8);
   }
   // every role is done (waits are bounded): free tensor memory
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1113,13 +1099,12 @@ __global__ void __launch_bounds__(TW_THREADS, 1)
 
 using gbsv::set_error;
 
-extern "C" int gbsv_run_stage_tc(const void* state_in, void* state_out,
-                                 int dtype, int n, int64_t num_states,
-                                 int64_t in_stride, int m, int c,
-                                 const int32_t* positions,
-                                 const void* blocks, int num_blocks,
-                                 const void* diags, const void* images,
-                                 const void* factors, void* stream) {
+template <bool SCALED>
+static int run_stage_tc(const void* state_in, void* state_out, int dtype,
+                        int n, int64_t num_states, int64_t in_stride, int m,
+                        int c, const int32_t* positions, const void* blocks,
+                        int num_blocks, const void* diags, const void* images,
+                        const void* factors, void* stream) {
   using namespace gbsv;
   if (dtype != GBSV_C64)
     return set_error(GBSV_ERR_UNSUPPORTED,
@@ -1179,26 +1164,48 @@ extern "C" int gbsv_run_stage_tc(const void* state_in, void* state_out,
   // longer stages stream them
   if (num_blocks <= TW_BLOCKS) {
     static OncePerDevice once;
-    const int rc =
-        allow_smem(once, tc_wide_kernel, TW_SMEM_BYTES, "tc_wide_kernel");
+    const int rc = allow_smem(once, tc_wide_kernel<SCALED>, TW_SMEM_BYTES,
+                              "tc_wide_kernel");
     if (rc) return rc;
     const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)sm_count());
-    tc_wide_kernel<<<(unsigned)grid, TW_THREADS, TW_SMEM_BYTES,
-                     static_cast<cudaStream_t>(stream)>>>(
+    tc_wide_kernel<SCALED><<<(unsigned)grid, TW_THREADS, TW_SMEM_BYTES,
+                             static_cast<cudaStream_t>(stream)>>>(
         static_cast<const float2*>(state_in),
         static_cast<float2*>(state_out), a);
     return after_launch("tc_wide_kernel");
   }
   static OncePerDevice once;
-  const int rc =
-      allow_smem(once, tc_stage_kernel, TC_SMEM_BYTES, "tc_stage_kernel");
+  const int rc = allow_smem(once, tc_stage_kernel<SCALED>, TC_SMEM_BYTES,
+                            "tc_stage_kernel");
   if (rc) return rc;
   const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)sm_count() * 2);
-  tc_stage_kernel<<<(unsigned)grid, TC_ROLE_THREADS, TC_SMEM_BYTES,
-                    static_cast<cudaStream_t>(stream)>>>(
+  tc_stage_kernel<SCALED><<<(unsigned)grid, TC_ROLE_THREADS, TC_SMEM_BYTES,
+                            static_cast<cudaStream_t>(stream)>>>(
       static_cast<const float2*>(state_in), static_cast<float2*>(state_out),
       a);
   return after_launch("tc_stage_kernel");
+}
+
+extern "C" int gbsv_run_stage_tc(
+    const void* state_in, void* state_out, int dtype, int n,
+    int64_t num_states, int64_t in_stride, int m, int c,
+    const int32_t* positions, const void* blocks, int num_blocks,
+    const void* diags, const void* images, const void* factors,
+    void* stream) {
+  return run_stage_tc<false>(state_in, state_out, dtype, n, num_states,
+                       in_stride, m, c, positions, blocks, num_blocks,
+                       diags, images, factors, stream);
+}
+
+extern "C" int gbsv_run_stage_tc_scaled(
+    const void* state_in, void* state_out, int dtype, int n,
+    int64_t num_states, int64_t in_stride, int m, int c,
+    const int32_t* positions, const void* blocks, int num_blocks,
+    const void* diags, const void* images, const void* factors,
+    void* stream) {
+  return run_stage_tc<true>(state_in, state_out, dtype, n, num_states,
+                      in_stride, m, c, positions, blocks, num_blocks,
+                      diags, images, factors, stream);
 }
 
 extern "C" int gbsv_tc_status(int* status, int clear) {

@@ -623,6 +623,7 @@ class Program:
         dev = self.device
         blocks, diags, images, factors = [], [], [], []
         self.ops = []
+        self.tc_scaled = set()  # first blocks of stages with column scales
         for kind, item in raw:
             if kind == "plain":
                 self.ops.append(self._plain_op(item))
@@ -632,6 +633,8 @@ class Program:
                                            images, factors)
             positions = (ctypes.c_int32 * tcplan.TC_M)(*order)
             self.ops.append(("tc", c, positions, first, len(blocks) - first))
+            if any(int(b["flags"]) & tcplan.TC_COLS for b in blocks[first:]):
+                self.tc_scaled.add(first)
         self.tc_blocks = _to_device(
             np.stack(blocks).view(np.uint8) if blocks else None, dev)
         self.tc_diags = _to_device(
@@ -841,7 +844,9 @@ class Program:
             _lib.check(rc, "run_stage")
         elif op[0] == "tc":
             _, c, positions, first, count = op
-            rc = L.gbsv_run_stage_tc(
+            run = (L.gbsv_run_stage_tc_scaled if first in self.tc_scaled
+                   else L.gbsv_run_stage_tc)
+            rc = run(
                 cur.data_ptr(), out.data_ptr(), self.code, self.n, B, N,
                 self.m, c, positions,
                 self.tc_blocks.data_ptr() + first * 64, count,
