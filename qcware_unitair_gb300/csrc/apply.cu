@@ -620,14 +620,9 @@ __device__ __forceinline__ void c128_prologue(const C* ops,
   const uint32_t p1 = __ballot_sync(0xffffffffu, cls & 2);
   const uint32_t p2 = __ballot_sync(0xffffffffu, cls & 4);
   const uint32_t large = __ballot_sync(0xffffffffu, mag >= PAIRS_LARGE);
-  const uint32_t some = __ballot_sync(0xffffffffu, mag != 0);
-  const uint32_t tiny = __ballot_sync(0xffffffffu, small);
-  bool even = tiny == 0;
-#pragma unroll
-  for (int j = 0; j < D; ++j) {
-    const uint32_t row = ((1u << D) - 1) << (D * j);
-    even = even && ((large & row) || !(some & row));
-  }
+  const uint32_t row = ((1u << D) - 1) << (lane & ~(D - 1));
+  const bool even =
+      !__any_sync(0xffffffffu, small || (mag != 0 && !(large & row)));
   int cl[D * D];
 #pragma unroll
   for (int j = 0; j < D * D; ++j)
